@@ -22,6 +22,11 @@ NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O2",
               "--expt-relaxed-constexpr", "-I", INCLUDE, "-I", CSRC]
 
 
+# Sources compiled once more for each part (a define that selects the
+# instantiations of one object file), so that they compile in parallel.
+PARTS = {"fft_fxc.cu": ["-DGBFFT_FXC_PART=%d" % i for i in range(12)]}
+
+
 def nvcc():
     cand = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not os.path.exists(cand):
@@ -53,8 +58,9 @@ def paths(variant=""):
 VARIANT_FLAGS = {"": [], "debug": ["-DGB_DEBUG_BOUNDS"]}
 
 
-def _compile(src, extra, obj_dir=OBJ):
-    obj = os.path.join(obj_dir, os.path.basename(src) + ".o")
+def _compile(src, extra, obj_dir=OBJ, part=""):
+    obj = os.path.join(obj_dir, os.path.basename(src) + part.replace("-D", ".").replace("=", "") + ".o")
+    extra = extra + ([part] if part else [])
     cmd = [nvcc()] + ARCH + NVCC_FLAGS + extra + ["-c", src, "-o", obj]
     if src.endswith(".cpp"):
         cmd[1:1] = ["-x", "cu"]
@@ -72,10 +78,11 @@ def build(force=False, verbose=False, extra=(), variant=""):
     os.makedirs(os.path.dirname(lib_path), exist_ok=True)
     if not force and os.path.exists(lib_path) and os.path.getmtime(lib_path) >= _newest_input():
         return lib_path
-    srcs = sources()
+    # the parts are the longest compilations: first
+    jobs = [(s, p) for s in sources() for p in PARTS.get(os.path.basename(s), [])] + [(s, "") for s in sources()]
     flags = list(extra) + VARIANT_FLAGS[variant]
-    with cf.ThreadPoolExecutor(max_workers=min(len(srcs), os.cpu_count() or 4)) as ex:
-        results = list(ex.map(lambda s: _compile(s, flags, obj_dir), srcs))
+    with cf.ThreadPoolExecutor(max_workers=min(len(jobs), os.cpu_count() or 4)) as ex:
+        results = list(ex.map(lambda j: _compile(j[0], flags, obj_dir, j[1]), jobs))
     if verbose:
         for _, log in results:
             if log.strip():

@@ -92,6 +92,9 @@ struct AxisPlan {
   void* d_twf = nullptr;  // stage-major table of the power-of-two kernel
   void* d_twfb = nullptr;   // the same for the batch kernel's plan
                             // (batch_points), when the axis runs another
+  FxPlan fx{};              // FP64 lines of one tile: the fixed-point plan
+  void* d_fxtw = nullptr;   // its stage-major table
+  void* d_fxroot = nullptr; // and, with direct-sum stages, its n roots
   void* d_chirp = nullptr;  // chirp-z tables (bt points at them)
   void* d_filt = nullptr;
   void* d_twm = nullptr;
@@ -313,7 +316,190 @@ int upload_batch_table(AxisPlan& p, int prec) {
   return upload_table(&p.d_twfb, stage_twiddles(plan_radices(q)), prec);
 }
 
+// Radices of the fixed-point kernel's compile-time butterflies.
+constexpr int kFxRadices[] = {2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 13};
+// Relative cost of a point in a stage of radix r, beside its exchange and
+// twiddle (kFxStageCost).
+constexpr double kFxStageCost = 24;
+double fx_radix_cost(int r) {
+  switch (r) {
+    case 2: return 2;
+    case 3: return 6;
+    case 4: return 4;
+    case 5: return 9;
+    case 6: return 9;
+    case 7: return 22;
+    case 8: return 9;
+    case 9: return 18;
+    case 10: return 13;
+    case 11: return 38;
+    case 13: return 46;
+    default: return 26.0 * r;  // direct sum
+  }
+}
+// Cheapest split of n into radices of at most rmax (primes beyond the
+// compile-time ones excepted, which any split carries).
+void fx_split(int n, int last, int rmax, double cost, std::vector<int>& cur, double& best, std::vector<int>& out) {
+  if (cost >= best) return;
+  if (n == 1) {
+    best = cost;
+    out = cur;
+    return;
+  }
+  bool any = false;
+  for (int i = (int)(sizeof(kFxRadices) / sizeof(int)) - 1; i >= 0; --i) {
+    const int r = kFxRadices[i];
+    if (n % r || r > last || (r > rmax && r <= 10)) continue;
+    any = true;
+    cur.push_back(r);
+    fx_split(n / r, r, rmax, cost + kFxStageCost + fx_radix_cost(r), cur, best, out);
+    cur.pop_back();
+  }
+  if (any) return;
+  int q = 2;  // smallest prime factor, a direct-sum stage
+  while (n % q) ++q;
+  cur.push_back(q);
+  fx_split(n / q, last, rmax, cost + kFxStageCost + fx_radix_cost(q), cur, best, out);
+  cur.pop_back();
+}
+bool fx_special(int r) {
+  for (int v : kFxRadices)
+    if (v == r) return true;
+  return r == 16;  // the compile-time plans'
+}
+// The fixed-point plan of an axis of n points; rmax bounds the radix (small
+// grids take radix 4: twice the threads a line).  ct: a compile-time plan may
+// run (those address rows below 4 GB apart).
+FxPlan fx_plan(int n, int rmax, bool ct) {
+  std::vector<int> cur, rad;
+  double best = 1e30;
+  const FxcShape shape = ct ? fxc_shape(n) : FxcShape{0, {0, 0, 0, 0}};
+  if (shape.tpl)
+    for (int r : shape.r) {
+      if (r > 1) rad.push_back(r);
+    }
+  else
+    fx_split(n, 1 << 30, rmax, 0, cur, best, rad);
+  FxPlan p;
+  std::memset(&p, 0, sizeof p);
+  p.nst = (int)rad.size();
+  p.ct = shape.tpl > 0;
+  int ns = 1, shift = 0;
+  for (int s = 0; s < p.nst; ++s) {
+    const int r = rad[s];
+    p.radix[s] = r;
+    p.ns[s] = ns;
+    p.magic[s] = ns > 1 ? (unsigned)(((1ull << 32) + ns - 1) / ns) : 0;
+    if (ns > 1) shift += shape.tpl && p.radix[s - 1] >= 16 ? 2 : 1;
+    else if (!fx_special(r)) shift += 1;
+    ns *= r;
+    int lg = 0;
+    while ((1 << lg) < ns) ++lg;
+    p.lg[s] = lg;
+    p.shift[s] = shift;
+  }
+  if (shape.tpl) {
+    p.tpl = shape.tpl;
+    return p;
+  }
+  // threads a line: at least n / kFxPoints, the count whose stages leave the
+  // fewest threads idle
+  const int lo = (n + kFxPoints - 1) / kFxPoints, hi = std::min(kFxMaxThreads, std::max(lo, (n + rmax - 1) / rmax * 5 / 4));
+  double bestw = 1e30;
+  for (int t = lo; t <= hi; ++t) {
+    double w = 0;
+    for (int s = 0; s < p.nst; ++s) {
+      const int nb = n / p.radix[s];
+      w += (kFxStageCost + fx_radix_cost(p.radix[s])) * (double)((nb + t - 1) / t) * t / nb;
+    }
+    if (w < bestw * 0.999) {
+      bestw = w;
+      p.tpl = t;
+    }
+  }
+  return p;
+}
+
+// exp(-2 pi i m / n), m = 0..n-1 (real, imaginary), in long double: one
+// evaluation for every eighth (n a multiple of 4), quarter (even) or half
+// turn, the rest by symmetry.
+std::vector<long double> roots_ld(int n) {
+  std::vector<long double> q(2 * (size_t)n);
+  const long double two_pi = 6.283185307179586476925286766559005768L;
+  auto put = [&](long long m, long double c, long double s) {
+    m %= n;
+    q[2 * (size_t)m] = c;
+    q[2 * (size_t)m + 1] = -s;
+  };
+  const long long part = n % 4 == 0 ? 8 : n % 2 == 0 ? 4 : 2;
+  for (long long m = 0; part * m <= n; ++m) {
+    const long double a = two_pi * (long double)m / (long double)n, c = cosl(a), s = sinl(a);
+    // angles m, and by reflection n/4 - m, n/2 - m, n - m
+    put(m, c, s);
+    if (m > 0) put(n - m, c, -s);
+    if (part >= 4) {
+      put(n / 2 - m, -c, s);
+      put(n / 2 + m, -c, -s);
+    }
+    if (part == 8) {
+      put(n / 4 - m, s, c);
+      put(n / 4 + m, -s, c);
+      put(3LL * n / 4 - m, -s, -c);
+      put(3LL * n / 4 + m, s, -c);
+    }
+  }
+  return q;
+}
+// A root table in Q62 integers, as balanced 32-bit halves, rounded once (long
+// double holds 64 or more mantissa bits).
+std::vector<int> q62_table(const std::vector<long double>& t) {
+  std::vector<int> q(2 * t.size());
+  for (size_t i = 0; i < t.size(); ++i) {
+    const long long x = llrintl(ldexpl(t[i], 62));
+    const int lo = (int)(unsigned)(unsigned long long)x;
+    q[2 * i] = lo;
+    q[2 * i + 1] = (int)((x - lo) >> 32);
+  }
+  return q;
+}
+int upload_ints(void** dst, const std::vector<int>& q) {
+  cudaError_t e = dev_malloc(dst, q.size() * sizeof(int));
+  if (e != cudaSuccess) {
+    *dst = nullptr;
+    return fail(GBFFT_ERR_ALLOC, std::string("cudaMalloc(twiddles): ") + cudaGetErrorString(e));
+  }
+  e = cudaMemcpy(*dst, q.data(), q.size() * sizeof(int), cudaMemcpyHostToDevice);
+  return e == cudaSuccess ? GBFFT_OK : cuda_fail(e, "cudaMemcpy(twiddles)");
+}
+// Tables of the fixed-point plan: stage s of radix R after NS points finds
+// W_{NS R}^{k r} at (NS - 1) + (r - 1) NS + k, as stage_twiddles.
+int upload_fx(AxisPlan& p) {
+  const FxPlan& f = p.fx;
+  const std::vector<long double> ld = roots_ld(p.n);
+  const std::vector<int> root = q62_table(ld);
+  std::vector<int> t(4 * (size_t)p.n, 0);
+  bool direct = false;
+  for (int s = 0; s < f.nst; ++s) {
+    const int R = f.radix[s], ns = f.ns[s];
+    direct = direct || !fx_special(R);
+    for (int r = 1; r < R; ++r)
+      for (int k = 0; k < ns; ++k) {
+        const size_t i = (size_t)(ns - 1) + (size_t)(r - 1) * ns + k;
+        const size_t m = (size_t)k * r * (size_t)(p.n / (ns * R)) % (size_t)p.n;
+        std::memcpy(&t[4 * i], &root[4 * m], 4 * sizeof(int));
+      }
+  }
+  // the n roots in double: lines that run in FP64
+  int rc = upload_table(&p.d_tw, std::vector<double>(ld.begin(), ld.end()), GBFFT_PREC_DOUBLE);
+  if (rc == GBFFT_OK) rc = upload_ints(&p.d_fxtw, t);
+  if (rc == GBFFT_OK && direct) rc = upload_ints(&p.d_fxroot, root);
+  p.fx.tw = p.d_fxtw;
+  p.fx.root = p.d_fxroot;
+  return rc;
+}
+
 int upload_twiddles(AxisPlan& p, int prec) {
+  if (p.fx.nst) return upload_fx(p);
   int rc = upload_table(&p.d_tw, twiddles(p.n), prec);
   const std::vector<int> radices = plan_radices(p);
   if (rc == GBFFT_OK && !radices.empty()) rc = upload_table(&p.d_twf, stage_twiddles(radices), prec);
@@ -468,7 +654,7 @@ void drop_profile(gbfft_engine_t e) {
 void release(gbfft_engine_t e) {
   drop_profile(e);
   for (auto& a : e->ax) {
-    for (void** q : {&a.d_tw, &a.d_twf, &a.d_twfb, &a.d_chirp, &a.d_filt, &a.d_twm}) {
+    for (void** q : {&a.d_tw, &a.d_twf, &a.d_twfb, &a.d_fxtw, &a.d_fxroot, &a.d_chirp, &a.d_filt, &a.d_twm}) {
       if (*q) dev_free(*q);
       *q = nullptr;
     }
@@ -608,9 +794,40 @@ int gen_lines_per_cta(int n, int prec, bool contiguous, long long nlines, int fo
   return L;
 }
 
+// Lines per CTA of the fixed-point kernels: strided tiles about 256 threads
+// and at least 64-byte row segments (4 lines); contiguous lines about 128
+// threads (512 x 512 x 256 x pass 336 us, with 256 threads 349).
+int fx_lines_per_cta(const FxPlan& f, int n, bool contiguous, long long nlines, long long nv, int forced_L) {
+  const bool ct = f.ct != 0;
+  const int maxt = ct ? fxc_max_threads(f.tpl) : kFxMaxThreads;
+  auto smem = [&](int l) { return ct ? fxc_smem_bytes(n, l) : fx_smem_bytes(n, l); };
+  if (forced_L > 0 && forced_L * f.tpl <= maxt && smem(forced_L) <= kFxMaxSmem) return forced_L;
+  const int min_l = contiguous ? 1 : 4;
+  int L = (contiguous ? 128 : 256) / f.tpl;
+  if (!contiguous && L > 4) L = L / 4 * 4;
+  if (L > 32) L = 32;
+  if (L < min_l) L = min_l;
+  while (L > min_l && smem(L) > 72 * 1024) L = contiguous ? L - 1 : L - 4;
+  while (L > min_l && ((nlines + L - 1) / L) * nv < 2LL * kSmsDefault) L = std::max(min_l, L / 2);
+  while (L > 1 && (L * f.tpl > maxt || smem(L) > kFxMaxSmem)) --L;
+  if (L > 1 && nlines < L) L = (int)nlines;
+  return L;
+}
+
 void fill_plan(PassArgs& a, const AxisPlan& p, int prec, bool contiguous, int kind, int forced_L,
                bool split = false, int csize = 0, int csync = 0) {
   a.blue = p.blue ? &p.bt : nullptr;
+  if (p.fx.nst) {
+    a.n = p.n;
+    a.nst = p.nst;  // the FP64 stages of lines fixed point does not take
+    for (int i = 0; i < kMaxStages; ++i) a.radix[i] = i < p.nst ? p.radix[i] : 0;
+    a.tw = p.d_tw;
+    a.fx = &p.fx;
+    a.fast = p.fx.ct ? 7 : 6;
+    a.tpl = p.fx.tpl;
+    a.L = fx_lines_per_cta(p.fx, p.n, contiguous, a.nlines, contiguous ? 1 : a.nv, forced_L);
+    return;
+  }
   if (split && split_length(p.n)) {
     a.n = p.n;
     a.nst = 0;
@@ -1018,6 +1235,13 @@ int engine_init_host(gbfft_engine_s* e, int format, int nx, int ny, int nz, int 
     if (fast_has_alt(lens[d]) && tune.e[d] > 0 && fast_e_ok(lens[d], tune.e[d])) e->ax[d].fast_e = tune.e[d];
     if (gen_length(lens[d]) && (tune.e[d] == gen_points(lens[d]) || tune.e[d] == 2))
       e->ax[d].fast_e = tune.e[d];
+    // FP64 lines of one tile: fixed point; small grids (under about 16 warps
+    // per SM at 8 points a thread) take radix 4 and twice the threads
+    if (prec == GBFFT_PREC_DOUBLE && !e->ax[d].big && fx_length(lens[d])) {
+      const double threads = (double)nx * ny * nz / kFxPoints;
+      e->ax[d].fx = fx_plan(lens[d], threads < 512.0 * kSmsDefault ? 4 : 10,
+                           (double)(nx + 8) * ny < (double)(1 << 28));
+    }
     if (form != GBFFT_FORM_PLAIN && split_length(lens[d])) e->ax[d].fast_e = 16;  // radix-16 stages for the tensor cores
   }
   *tune_out = tune;
@@ -1566,6 +1790,11 @@ int gbfft_engine_set_plan(gbfft_engine_t e, int axis, int points) {
                                      "(8: at most 256 points, 4: at most 128)");
   }
   if (p.fast_e == points) return GBFFT_OK;
+  if (p.fx.nst) {  // FP64 passes in fixed point have one plan: only the setting is kept
+    p.fast_e = points;
+    for (int k = 0; k < GBFFT_PASS_KINDS; ++k) e->tile_L[k] = 0;
+    return GBFFT_OK;
+  }
   void* old = p.d_twf;
   const int old_e = p.fast_e;
   p.fast_e = points;

@@ -39,65 +39,16 @@ using namespace dev;
 
 std::atomic<long long> g_launches{0};
 
-// Runtime-planned pass: any length up to kMaxN, any factorisation.  The
-// lines are loaded into shared buffer 0, each stage ping-pongs between the
-// two buffers, and the result is stored from the last buffer written.
+// Runtime-planned pass: any length up to kMaxN, any factorisation (run_pp_lines,
+// fft_pp.cuh).
 template <typename T, int KIND, bool CONTIG>
 __global__ void __launch_bounds__(kMaxThreads)
     axis_pass_kernel(const __grid_constant__ PassArgs a) {
-  using C = Cx<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   chained_entry();
   LineCtx<T, KIND, CONTIG> c;
   c.init(a);
-  const size_t e = (size_t)a.n * a.L;
-  C* buf0 = reinterpret_cast<C*>(smem_raw);
-  C* buf1 = buf0 + (e + (e >> 4) + 1);
-
-#pragma unroll 1
-  for (int n = c.t; n < c.N; n += c.tpl) buf0[c.sidx(n)] = c.gload(n);
-  __syncthreads();
-
-  C* A = buf0;
-  C* B = buf1;
-  int Ns = 1;
-#pragma unroll 1
-  for (int s = 0; s < a.nst; ++s) {
-    const int R = a.radix[s];
-    if (R == 16) stage_pp<T, KIND, CONTIG, 16>(c, A, B, Ns);
-    else if (R == 8) stage_pp<T, KIND, CONTIG, 8>(c, A, B, Ns);
-    else if (R == 4) stage_pp<T, KIND, CONTIG, 4>(c, A, B, Ns);
-    else if (R == 2) stage_pp<T, KIND, CONTIG, 2>(c, A, B, Ns);
-    else if (R == 3) stage_pp<T, KIND, CONTIG, 3>(c, A, B, Ns);
-    else if (R == 5) stage_pp<T, KIND, CONTIG, 5>(c, A, B, Ns);
-    else if (R == 7) stage_pp<T, KIND, CONTIG, 7>(c, A, B, Ns);
-    else if (R == 11) stage_pp<T, KIND, CONTIG, 11>(c, A, B, Ns);
-    else if (R == 13) stage_pp<T, KIND, CONTIG, 13>(c, A, B, Ns);
-    else if (R == 17) stage_pp<T, KIND, CONTIG, 17>(c, A, B, Ns);
-    else if (R == 19) stage_pp<T, KIND, CONTIG, 19>(c, A, B, Ns);
-    else if (R == 23) stage_pp<T, KIND, CONTIG, 23>(c, A, B, Ns);
-    else if (sizeof(T) == 4 && (R == 29 || R == 31)) {
-      // in FP64 a butterfly of 29 or 31 points does not fit the registers
-      if constexpr (sizeof(T) == 4) {
-        if (R == 29) stage_pp<T, KIND, CONTIG, 29>(c, A, B, Ns);
-        else stage_pp<T, KIND, CONTIG, 31>(c, A, B, Ns);
-      }
-    } else {
-      stage_pp_generic<T, KIND, CONTIG>(c, A, B, R, Ns);
-    }
-    __syncthreads();
-    C* tmp = A;
-    A = B;
-    B = tmp;
-    Ns *= R;
-  }
-
-  if (KIND == K_R2C) {
-    c.store_r2c(A);
-  } else {
-#pragma unroll 1
-    for (int n = c.t; n < c.N; n += c.tpl) c.gstore(n, A[c.sidx(n)]);
-  }
+  run_pp_lines<T, KIND, CONTIG>(c, a, reinterpret_cast<Cx<T>*>(smem_raw), (size_t)a.n * a.L);
 }
 
 template <typename T, int KIND, bool CONTIG>
@@ -166,21 +117,15 @@ cudaError_t launch_axis_one(int prec_bytes, int kind, bool contiguous, const Pas
     if (!tc_pass_supported(prec_bytes, kind, contiguous, a)) return cudaErrorInvalidValue;
     return launch_tc_pass(a, stream);
   }
-  if (a.fast == 4) return prec_bytes == 4 ? launch_gen_f32(kind, contiguous, a, stream)
-                                          : launch_gen_f64(kind, contiguous, a, stream);
-  if (a.fast == 3) {
-    if (prec_bytes != 4) return cudaErrorInvalidValue;
-    return launch_split_f32(kind, contiguous, a, stream);
-  }
-  if (a.fast == 2) return prec_bytes == 4 ? launch_mixed_f32(kind, contiguous, a, stream)
-                                          : launch_mixed_f64(kind, contiguous, a, stream);
-  if (a.fast) {
-    if (prec_bytes == 4)
-      return kind == K_C2C ? launch_fast_f32_c2c(kind, contiguous, a, stream)
-                           : launch_fast_f32_real(kind, contiguous, a, stream);
-    return kind == K_C2C ? launch_fast_f64_c2c(kind, contiguous, a, stream)
-                         : launch_fast_f64_real(kind, contiguous, a, stream);
-  }
+  if (a.fast == 7) return prec_bytes == 8 ? launch_fxc(kind, contiguous, a, stream) : cudaErrorInvalidValue;
+  if (a.fast == 6) return prec_bytes == 8 ? launch_fx(kind, contiguous, a, stream) : cudaErrorInvalidValue;
+  if (a.fast && prec_bytes != 4) return cudaErrorInvalidValue;  // the other compile-time kernels are FP32's
+  if (a.fast == 4) return launch_gen_f32(kind, contiguous, a, stream);
+  if (a.fast == 3) return launch_split_f32(kind, contiguous, a, stream);
+  if (a.fast == 2) return launch_mixed_f32(kind, contiguous, a, stream);
+  if (a.fast)
+    return kind == K_C2C ? launch_fast_f32_c2c(kind, contiguous, a, stream)
+                         : launch_fast_f32_real(kind, contiguous, a, stream);
 #define GB_DISPATCH(T)                                                              \
   switch (kind) {                                                                   \
     case K_C2C: return contiguous ? launch_typed<T, K_C2C, true>(a, stream)         \

@@ -570,6 +570,32 @@ struct LineCtx {
     }
   }
 
+  // Point n of a c2c or r2c line as it lies in memory (no conjugation), and
+  // of a c2c or c2r line the way back (c2r: x into the first real line, y
+  // into the second).
+  __device__ __forceinline__ C gload_raw(int n) const {
+    if constexpr (KIND == K_C2C) {
+      if ((PRED && !valid) || !GB_SRC(sb0 + n * ssn, 1)) return cmk<C>(T(0), T(0));
+      return ld(reinterpret_cast<const C*>(src) + sb0 + n * ssn);
+    } else {
+      return gload(n);
+    }
+  }
+  __device__ __forceinline__ void gstore_raw(int n, C v) const {
+    if (!valid) return;
+    if constexpr (KIND == K_C2C) {
+      if (GB_DST(db0 + n * dsn, 1)) reinterpret_cast<C*>(dst)[db0 + n * dsn] = v;
+    } else {
+      T* d = reinterpret_cast<T*>(dst);
+      if (!CONTIG && pvec && has1) {
+        if (GB_DST(db0 + n * dsn, 2)) *reinterpret_cast<C*>(d + db0 + n * dsn) = v;
+        return;
+      }
+      if (GB_DST(db0 + n * dsn, 1)) d[db0 + n * dsn] = v.x;
+      if (has1 && GB_DST(db1 + n * dsn, 1)) d[db1 + n * dsn] = v.y;
+    }
+  }
+
   // Point n of this line from a tile that a copy engine filled in natural
   // order (slot sidx(n)), as the forward transform must see it.
   __device__ __forceinline__ C sload(const C* S, int n) const {
@@ -651,6 +677,18 @@ struct LineCtx {
       x2.y = T(0);
     }
     return cmk<C>(x1.x - x2.y, -(x1.y + x2.x));
+  }
+
+  // Point j of half spectrum `which` (0, 1) of this c2r line pair.
+  __device__ __forceinline__ C half(int which, int j) const {
+    const long long at = (which ? sb1 : sb0) + j * ssn;
+    if ((PRED && !valid) || (which && !has1) || !GB_SRC(at, 1)) return cmk<C>(T(0), T(0));
+    return ld(reinterpret_cast<const C*>(src) + at);
+  }
+  // Point k of half spectrum `which` of this r2c line pair.
+  __device__ __forceinline__ void put_half(int which, int k, C x) const {
+    const long long at = (which ? db1 : db0) + k * dsn;
+    if (valid && (!which || has1) && GB_DST(at, 1)) reinterpret_cast<C*>(dst)[at] = x;
   }
 
   // r2c output in pair slots (the c2r staging layout): slot k holds

@@ -1,0 +1,248 @@
+// Axis passes of FP64 lines in 64-bit fixed point (fft_fx.cuh), any length a
+// tile holds.
+//
+// What bounds an FP64 pass on GB300 is the FP64 pipe (two multiply-adds an SM
+// and clock): a 512-point line costs about 17 SM clocks a point there, four
+// times what its DRAM traffic takes and more.  In integers the same line
+// costs two to three.
+//
+// A CTA owns L lines, `tpl` threads each:
+//   1. every thread loads its points (at most kE, in registers) and the line's
+//      largest high word goes to shared memory;
+//   2. the line's sum of moduli, in units of 2^-20 of that, follows; the two
+//      give the scale at which no stage's output leaves the word;
+//   3. the points become integers in shared buffer 0 (c2r: the Hermitian
+//      combination of the two half spectra);
+//   4. Stockham stages ping-pong between the two buffers, twiddles from a
+//      stage-major Q62 table;
+//   5. the result goes back to doubles (r2c: the two half spectra apart),
+//      rounded once, to nearest.
+// A CTA that meets a NaN, an infinity or a line outside the exponents of
+// fx::kMinExp..kMaxExp runs its lines in FP64 instead (fx::fallback), with the
+// result those had before.
+#include "fft_fx.cuh"
+
+namespace gbfft {
+
+namespace {
+
+using namespace dev;
+using fx::I2;
+using fx::ll;
+using fx::W4;
+
+constexpr int kE = kFxPoints;
+
+template <int R, class Ctx>
+__device__ __forceinline__ void fx_stage(const Ctx& c, const I2* A, I2* B, const W4* __restrict__ tw, int Ns,
+                                         unsigned magic) {
+  const int nb = c.N / R;
+#pragma unroll 1
+  for (int b = c.t; b < nb; b += c.tpl) {
+    I2 v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = A[c.sidx(b + r * nb)];
+    int k = 0;
+    if (Ns > 1) {
+      k = b - (int)__umulhi((unsigned)b, magic) * Ns;
+      const W4* w = tw + (Ns - 1) + k;
+      v[0] = fx::mk(fx::scale_down(v[0].x), fx::scale_down(v[0].y));
+#pragma unroll
+      for (int r = 1; r < R; ++r) v[r] = fx::mul_tw(v[r], fx::ldw(w + (r - 1) * Ns), r);
+    }
+    const int base = (b - k) * R + k;
+    if constexpr (R > 5 && R % 2 == 1 && R % 3 != 0) {
+      fx::dft_odd<R>(v, [&](int m, I2 x) { B[c.sidx(base + m * Ns)] = x; });
+    } else {
+      fx::dft<R>(v);
+#pragma unroll
+      for (int r = 0; r < R; ++r) B[c.sidx(base + r * Ns)] = v[r];
+    }
+  }
+}
+
+// Any other prime: every output a direct sum over R inputs, half of each.
+template <class Ctx>
+__device__ void fx_stage_generic(const Ctx& c, const I2* A, I2* B, const W4* __restrict__ root, int R, int Ns) {
+  const int N = c.N, nb = N / R, tstride = N / (Ns * R);
+#pragma unroll 1
+  for (int o = c.t; o < N; o += c.tpl) {
+    const int k = o % Ns, r = (o / Ns) % R, b = o / (Ns * R) * Ns + k;
+    const int step = (k * tstride + r * nb) % N;
+    I2 acc = fx::mk(0, 0);
+    int e = 0;
+#pragma unroll 1
+    for (int j = 0; j < R; ++j) {
+      acc = fx::add(acc, fx::mul_tw(A[c.sidx(b + j * nb)], fx::ldw(root + e), j));
+      e += step;
+      if (e >= N) e -= N;
+    }
+    B[c.sidx(o)] = acc;
+  }
+}
+
+template <int KIND, bool CONTIG>
+__global__ void __launch_bounds__(kFxMaxThreads) fx_pass_kernel(const __grid_constant__ PassArgs a,
+                                                                const __grid_constant__ FxPlan p) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  chained_entry();
+  LineCtx<double, KIND, CONTIG> c;
+  c.init(a);
+  const int N = c.N, tpl = c.tpl, t = c.t;
+  const int e = N * a.L;
+  I2* buf0 = reinterpret_cast<I2*>(smem_raw);
+  I2* buf1 = buf0 + (e + (e >> 4) + 1);
+  int* smax = reinterpret_cast<int*>(buf1 + (e + (e >> 4) + 1));
+  unsigned* ssum = reinterpret_cast<unsigned*>(smax + a.L);
+  {
+    const int threads = blockDim.x * blockDim.y;
+    for (int i = threadIdx.x + threadIdx.y * blockDim.x; i < 2 * a.L; i += threads) smax[i] = 0;
+  }
+  __syncthreads();
+
+  // c2r: two half spectra of N / 2 + 1 points, point j of both in v[2 i], v[2 i + 1]
+  constexpr int J = KIND == K_C2R ? kE / 2 + 1 : kE;
+  constexpr int W = KIND == K_C2R ? 2 : 1;
+  const int cnt = KIND == K_C2R ? N / 2 + 1 : N;
+  double2 v[J * W];
+  int m = 0;
+#pragma unroll
+  for (int i = 0; i < J; ++i) {
+    const int n = t + i * tpl;
+    if constexpr (KIND == K_C2R) {
+      v[2 * i] = n < cnt ? c.half(0, n) : make_double2(0, 0);
+      v[2 * i + 1] = n < cnt ? c.half(1, n) : make_double2(0, 0);
+      if (n == 0 || 2 * n == N) v[2 * i].y = v[2 * i + 1].y = 0;  // Im of the DC and Nyquist bins is ignored
+    } else {
+      v[i] = n < cnt ? c.gload_raw(n) : make_double2(0, 0);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < J * W; ++i) m = max(m, fx::max_hi(v[i]));
+  atomicMax(&smax[c.line], m);
+  __syncthreads();
+  m = smax[c.line];
+  const int em = m >> 20;
+  float sum = 0;
+#pragma unroll
+  for (int i = 0; i < J * W; ++i) sum += fx::share(fx::max_hi(v[i]), fx::share_base(em));
+  atomicAdd(&ssum[c.line], fx::share_units(sum, J * W));
+  int bad = m != 0 && (em < fx::kMinExp || em > fx::kMaxExp);
+  if (m == 0) {  // all zero, or subnormals below 2^-1042
+#pragma unroll
+    for (int i = 0; i < J * W; ++i) bad |= fx::any_lo(v[i]);
+  }
+  if (__syncthreads_or(bad)) {
+    fx::fallback<KIND, CONTIG>(a, reinterpret_cast<double2*>(smem_raw));
+    return;
+  }
+  // exponents (less em) of what bounds the moduli: the sum of all, and n
+  // times the largest; after each stage the smaller of the two holds
+  const unsigned S = ssum[c.line];
+  constexpr int X = KIND == K_C2R ? 1 : 0;  // a point combines two values
+  const int es = 32 - __clz((int)(S + (S >> 1))) - 1040 + X;
+  int top = -1021 + X;
+#pragma unroll 1
+  for (int s = 0; s < p.nst; ++s) top = max(top, min(es, p.lg[s] - 1021 + X) - p.shift[s]);
+  // the moduli may reach 2^62 (2^61 where r2c adds two values that no
+  // twiddle has halved)
+  if (KIND == K_R2C && p.shift[p.nst - 1] == 0) ++top;
+  // right shift of a mantissa, less its exponent; a zero line shifts all out
+  const int sh = m == 0 ? 4096 : 1021 + top + em;
+  int adj = (em - 62 + top + p.shift[p.nst - 1]) << 20;  // exponent of a result's unit, in a high word
+
+  // backward: conjugated on the way in (c2r: by its combination) and out
+  const int flip = c.inverse ? (int)0x80000000 : 0;
+  if constexpr (KIND == K_C2R) {
+#pragma unroll
+    for (int i = 0; i < J; ++i) {
+      const int j = t + i * tpl;
+      if (j < cnt) {
+        const ll ax = fx::to_fixed(v[2 * i].x, sh), ay = fx::to_fixed(v[2 * i].y, sh);
+        const ll bx = fx::to_fixed(v[2 * i + 1].x, sh), by = fx::to_fixed(v[2 * i + 1].y, sh);
+        // z = x1 + i x2, conjugated for the inverse-by-conjugation
+        buf0[c.sidx(j)] = fx::mk(ax - by, -(ay + bx));
+        if (j > 0 && 2 * j < N) buf0[c.sidx(N - j)] = fx::mk(ax + by, ay - bx);
+      }
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < J; ++i) {
+      const int n = t + i * tpl;
+      if (n < N) buf0[c.sidx(n)] = fx::mk(fx::to_fixed(v[i].x, sh), fx::to_fixed(v[i].y, sh, flip));
+    }
+  }
+  __syncthreads();
+
+  const I2* A = buf0;
+  I2* B = buf1;
+  const W4* tw = reinterpret_cast<const W4*>(p.tw);
+#pragma unroll 1
+  for (int s = 0; s < p.nst; ++s) {
+    const int R = p.radix[s], Ns = p.ns[s];
+    const unsigned mg = p.magic[s];
+    switch (R) {
+      case 2: fx_stage<2>(c, A, B, tw, Ns, mg); break;
+      case 3: fx_stage<3>(c, A, B, tw, Ns, mg); break;
+      case 4: fx_stage<4>(c, A, B, tw, Ns, mg); break;
+      case 5: fx_stage<5>(c, A, B, tw, Ns, mg); break;
+      case 6: fx_stage<6>(c, A, B, tw, Ns, mg); break;
+      case 7: fx_stage<7>(c, A, B, tw, Ns, mg); break;
+      case 8: fx_stage<8>(c, A, B, tw, Ns, mg); break;
+      case 9: fx_stage<9>(c, A, B, tw, Ns, mg); break;
+      case 10: fx_stage<10>(c, A, B, tw, Ns, mg); break;
+      case 11: fx_stage<11>(c, A, B, tw, Ns, mg); break;
+      case 13: fx_stage<13>(c, A, B, tw, Ns, mg); break;
+      default: fx_stage_generic(c, A, B, reinterpret_cast<const W4*>(p.root), R, Ns); break;
+    }
+    __syncthreads();
+    I2* const done = B;
+    B = const_cast<I2*>(A);
+    A = done;
+  }
+
+  if constexpr (KIND == K_R2C) {
+    adj -= 1 << 20;  // the halves of X1 = (Z_k + conj Z_{n-k}) / 2, X2 = (Z_k - conj Z_{n-k}) / 2i
+#pragma unroll 1
+    for (int k = t; 2 * k <= N; k += tpl) {
+      const I2 zk = A[c.sidx(k)], zm = A[c.sidx(k == 0 ? 0 : N - k)];
+      c.put_half(0, k, make_double2(fx::to_double(zk.x + zm.x, adj), fx::to_double(zk.y - zm.y, adj)));
+      c.put_half(1, k, make_double2(fx::to_double(zk.y + zm.y, adj), fx::to_double(zm.x - zk.x, adj)));
+    }
+  } else {
+#pragma unroll 1
+    for (int n = t; n < N; n += tpl) {
+      const I2 z = A[c.sidx(n)];
+      c.gstore_raw(n, make_double2(fx::to_double(z.x, adj), fx::to_double(z.y, adj, flip)));
+    }
+  }
+}
+
+template <int KIND, bool CONTIG>
+cudaError_t launch_k(const PassArgs& a, cudaStream_t stream) {
+  const FxPlan& p = *a.fx;
+  const size_t smem = fx_smem_bytes(a.n, a.L);
+  if (a.L < 1 || a.tpl < 1 || a.L * a.tpl > kFxMaxThreads || a.tpl * kE < a.n || smem > kFxMaxSmem)
+    return cudaErrorInvalidValue;
+  auto kern = fx_pass_kernel<KIND, CONTIG>;
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  const dim3 block = CONTIG ? dim3(a.tpl, a.L) : dim3(a.L, a.tpl);
+  const dim3 grid((unsigned)((a.nlines + a.L - 1) / a.L), CONTIG ? 1u : (unsigned)a.nv);
+  const cudaError_t err = launch_chained(kern, grid, block, smem, stream, a, p);
+  add_launches(1);
+  return err != cudaSuccess ? err : cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t launch_fx(int kind, bool contiguous, const PassArgs& a, cudaStream_t s) {
+  if (kind == K_C2C) return contiguous ? launch_k<K_C2C, true>(a, s) : launch_k<K_C2C, false>(a, s);
+  if (kind == K_R2C) return contiguous ? launch_k<K_R2C, true>(a, s) : launch_k<K_R2C, false>(a, s);
+  if (kind == K_C2R) return contiguous ? launch_k<K_C2R, true>(a, s) : launch_k<K_C2R, false>(a, s);
+  return cudaErrorInvalidValue;
+}
+
+}  // namespace gbfft

@@ -1,0 +1,410 @@
+// 64-bit fixed-point complex arithmetic for FP64 lines.
+//
+// An SM issues two FP64 multiply-adds a clock but 64 64-bit integer adds and
+// 32 32 x 32 -> 64-bit multiply-adds (measured on GB300).  An FFT is adds
+// and multiplications by constants of modulus one, and no value of a line's
+// transform exceeds the sum of the moduli of its inputs, so a line can be
+// transformed in integers that share one power-of-two scale, chosen from
+// that sum: 64 bits for numbers that hold 53, of which at most a few go to
+// headroom.  The scale is the line's own (never a neighbour's), so a small
+// line next to a large one keeps all its digits.
+//
+// Formats: a value is a signed 64-bit integer v, |v| < 2^62.  Table twiddles
+// are Q62 (w 2^62) and multiplying by one divides by 2, after a stage of
+// radix 16 by 4 (a value grows by sqrt(R) in a stage of radix R on noise and
+// by nothing on a line with one large point; a division by more loses bits);
+// constants of the butterflies are Q64 and keep the scale.  Every product is rounded to
+// nearest at 2^-64 of its factors' range; the low 32 x 32 product (below
+// half a unit) is left out.
+#pragma once
+
+#include "fft_common.cuh"
+#include "fft_pp.cuh"
+
+namespace gbfft {
+namespace fx {
+
+using ll = long long;
+
+struct alignas(16) I2 {
+  ll x, y;
+};
+// Q62 root: real and imaginary parts as balanced 32-bit halves (both signed,
+// value = hi 2^32 + lo)
+struct alignas(16) W4 {
+  int xl, xh, yl, yh;
+};
+
+__device__ __forceinline__ I2 mk(ll a, ll b) {
+  I2 r;
+  r.x = a;
+  r.y = b;
+  return r;
+}
+__device__ __forceinline__ I2 add(I2 a, I2 b) { return mk(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ I2 sub(I2 a, I2 b) { return mk(a.x - b.x, a.y - b.y); }
+// a * b + c and a * b, 32 x 32 -> 64 bits.  Spelt out: from (ll)a * b the
+// compiler made unsigned products and sign corrections (76 of 313
+// instructions a point of a 256-point pass).
+__device__ __forceinline__ ll madw(int a, int b, ll c) {
+  ll d;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ ll mulw(int a, int b) {
+  ll d;
+  asm("mul.wide.s32 %0, %1, %2;" : "=l"(d) : "r"(a), "r"(b));
+  return d;
+}
+// balanced halves: v = hi(v) 2^32 + lo(v), both signed
+__host__ __device__ __forceinline__ constexpr int hi(ll v) {
+  return (int)(v >> 32) + (int)((unsigned)(unsigned long long)v >> 31);  // one shift-add
+}
+__host__ __device__ __forceinline__ constexpr int lo(ll v) { return (int)(unsigned)(unsigned long long)v; }
+constexpr ll kHalf = 0x80000000ll;  // rounds a sum of middle products
+
+// ---- compile-time roots in Q62 --------------------------------------------
+// cos and sin of 2 pi m / d: the angle reduced exactly to [0, pi/4] on the
+// rational, then Taylor series in 128-bit integer arithmetic.
+constexpr unsigned long long kTwoPiQ61 = 14488038916154245685ull;  // 2 pi 2^61
+constexpr ll mulq62(ll a, ll b) { return (ll)(((__int128)a * b + ((__int128)1 << 61)) >> 62); }
+struct SC {
+  ll s, c;
+};
+constexpr SC sincos_q62(long long m, long long d) {
+  m %= d;
+  if (m < 0) m += d;
+  bool ns = false, nc = false, swap = false;
+  if (2 * m > d) {
+    m = d - m;
+    ns = true;
+  }
+  if (4 * m > d) {
+    m = d - 2 * m;
+    d = 2 * d;
+    nc = !nc;
+  }
+  if (8 * m > d) {
+    m = d - 4 * m;
+    d = 4 * d;
+    swap = true;
+  }
+  const ll one = 1ll << 62;
+  const ll x = (ll)(((unsigned __int128)kTwoPiQ61 * 2 * (unsigned __int128)m + (unsigned __int128)(d / 2)) /
+                    (unsigned __int128)d);
+  const ll x2 = mulq62(x, x);
+  ll ts = x, s = x, tc = one, c = one;
+  for (int k = 1; k < 14; ++k) {
+    tc = -mulq62(tc, x2) / ((2 * k - 1) * (2 * k));
+    c += tc;
+    ts = -mulq62(ts, x2) / ((2 * k) * (2 * k + 1));
+    s += ts;
+  }
+  if (swap) {
+    const ll t = s;
+    s = c;
+    c = t;
+  }
+  return {ns ? -s : s, nc ? -c : c};
+}
+// A constant of [-1, 1] in Q62 as base + frac: base in {-1, 0, 1}, |frac| at
+// most one half, as Q64.
+constexpr int k_base(ll q) { return q >= (1ll << 61) ? 1 : q < -(1ll << 61) ? -1 : 0; }
+constexpr ll k_frac(ll q) { return (q - k_base(q) * (1ll << 62)) * 4; }
+
+// x times a constant (Q62 template argument), at x's scale.
+template <ll Q>
+__device__ __forceinline__ ll mulk(ll x) {
+  constexpr ll F = k_frac(Q);
+  constexpr int B = k_base(Q);
+  const ll m = madw(lo(x), hi(F), madw(hi(x), lo(F), kHalf));
+  const ll h = madw(hi(x), hi(F), m >> 32);
+  return B > 0 ? h + x : B < 0 ? h - x : h;
+}
+// x * KX + y * KY.  The middle products of two terms fit 64 bits: with moduli
+// that sum to at most 2^62 the high halves give at most sqrt(2) 2^61 there,
+// the low ones |frac x| + |frac y| (at most 0.634 for the two parts of a
+// root) times 2^63.
+template <ll QX, ll QY>
+__device__ __forceinline__ ll lin2(ll x, ll y) {
+  constexpr ll FX = k_frac(QX), FY = k_frac(QY);
+  constexpr int BX = k_base(QX), BY = k_base(QY);
+  ll m = madw(lo(x), hi(FX), madw(hi(x), lo(FX), kHalf));
+  m = madw(lo(y), hi(FY), madw(hi(y), lo(FY), m));
+  ll h = madw(hi(y), hi(FY), madw(hi(x), hi(FX), m >> 32));
+  h = BX > 0 ? h + x : BX < 0 ? h - x : h;
+  return BY > 0 ? h + y : BY < 0 ? h - y : h;
+}
+// a * exp(-2 pi i M / R)
+template <int R, int M>
+__device__ __forceinline__ I2 mul_root(I2 a) {
+  constexpr int m = ((M % R) + R) % R;
+  if constexpr (m == 0) {
+    return a;
+  } else if constexpr (4 * m == R) {
+    return mk(a.y, -a.x);
+  } else if constexpr (2 * m == R) {
+    return mk(-a.x, -a.y);
+  } else if constexpr (4 * m == 3 * R) {
+    return mk(-a.y, a.x);
+  } else if constexpr ((8 * m) % R == 0) {
+    // (+-1 +- i) / sqrt 2: one real constant for each component
+    constexpr ll q = sincos_q62(1, 8).c;
+    constexpr int o = 8 * m / R;  // 1, 3, 5, 7 eighths of a turn
+    if constexpr (o == 1) return mk(mulk<q>(a.x + a.y), mulk<q>(a.y - a.x));
+    else if constexpr (o == 3) return mk(mulk<q>(a.y - a.x), mulk<-q>(a.x + a.y));
+    else if constexpr (o == 5) return mk(mulk<-q>(a.x + a.y), mulk<q>(a.x - a.y));
+    else return mk(mulk<q>(a.x - a.y), mulk<q>(a.x + a.y));
+  } else {
+    constexpr SC w = sincos_q62(m, R);
+    return mk(lin2<w.c, w.s>(a.x, a.y), lin2<-w.s, w.c>(a.x, a.y));
+  }
+}
+__device__ __forceinline__ W4 ldw(const W4* p) {
+  const int4 q = __ldg(reinterpret_cast<const int4*>(p));
+  W4 w;
+  w.xl = q.x;
+  w.xh = q.y;
+  w.yl = q.z;
+  w.yh = q.w;
+  return w;
+}
+// a * w / 2^SH (SH 1 or 2) for a table root: the middle products shifted by
+// 30 + SH, the high ones doubled for SH = 1.  Exact ties (the
+// twiddle 1 makes them) round up or down by the parity of r's bits, the
+// imaginary part the other way: one direction for all would add up in bin 0,
+// alternating ones in another.
+template <int SH = 1>
+__device__ __forceinline__ I2 mul_tw(I2 a, W4 w, int r) {
+  static_assert(SH == 1 || SH == 2, "scale");
+  const int xh = hi(a.x), xl = lo(a.x), yh = hi(a.y), yl = lo(a.y);
+  const int xd = xh * (3 - SH), yd = yh * (3 - SH);
+  const int odd = (0x6996 >> (r & 15)) & 1;
+  const ll ur = kHalf / (3 - SH) - odd, ui = kHalf / (3 - SH) - 1 + odd;
+  const ll mr = madw(xl, w.xh, madw(xh, w.xl, ur)) - madw(yl, w.yh, mulw(yh, w.yl));
+  const ll mi = madw(yl, w.xh, madw(yh, w.xl, madw(xl, w.yh, madw(xh, w.yl, ui))));
+  return mk(madw(xd, w.xh, mr >> (30 + SH)) - mulw(yd, w.yh), madw(yd, w.xh, madw(xd, w.yh, mi >> (30 + SH))));
+}
+// v / 2^SH, rounded to nearest even: the scale of a value that meets the
+// twiddle 1 (a bias common to all of them would add up in one bin)
+template <int SH = 1>
+__device__ __forceinline__ ll scale_down(ll v) {
+  return (v + (SH - 1) + ((v >> SH) & 1)) >> SH;
+}
+
+// ---- butterflies (forward, natural order in and out) -----------------------
+__device__ __forceinline__ void dft4v(I2& a0, I2& a1, I2& a2, I2& a3) {
+  const I2 t0 = add(a0, a2), t1 = sub(a0, a2), t2 = add(a1, a3), d = sub(a1, a3);
+  a0 = add(t0, t2);
+  a2 = sub(t0, t2);
+  a1 = mk(t1.x + d.y, t1.y - d.x);
+  a3 = mk(t1.x - d.y, t1.y + d.x);
+}
+__device__ __forceinline__ void dft3p(I2* v) {
+  constexpr ll q = sincos_q62(1, 3).s;
+  const I2 t = add(v[1], v[2]), d = sub(v[1], v[2]);
+  const I2 m = mk(v[0].x - ((t.x + 1) >> 1), v[0].y - (t.y >> 1));
+  const ll sx = mulk<q>(d.x), sy = mulk<q>(d.y);
+  v[0] = add(v[0], t);
+  v[1] = mk(m.x + sy, m.y - sx);
+  v[2] = mk(m.x - sy, m.y + sx);
+}
+// DFT5 on two constants a component: m1, m2 = (a0 - (t1 + t2) / 4) +- sqrt5/4
+// (t1 - t2), and the sine pair.
+__device__ __forceinline__ void dft5p(I2* v) {
+  constexpr ll s1 = sincos_q62(1, 5).s, s2 = sincos_q62(2, 5).s;
+  constexpr ll c5 = (sincos_q62(1, 5).c - sincos_q62(2, 5).c) / 2;  // sqrt 5 / 4
+  const I2 t1 = add(v[1], v[4]), t2 = add(v[2], v[3]), t3 = sub(v[1], v[4]), t4 = sub(v[2], v[3]);
+  const I2 a0 = v[0], ts = add(t1, t2), td = sub(t1, t2);
+  const I2 b = mk(a0.x - ((ts.x + 2) >> 2), a0.y - ((ts.y + 2) >> 2));
+  const I2 e = mk(mulk<c5>(td.x), mulk<c5>(td.y));
+  const I2 m1 = add(b, e), m2 = sub(b, e);
+  const I2 n1 = mk(lin2<s1, s2>(t3.x, t4.x), lin2<s1, s2>(t3.y, t4.y));
+  const I2 n2 = mk(lin2<s2, -s1>(t3.x, t4.x), lin2<s2, -s1>(t3.y, t4.y));
+  v[0] = add(a0, ts);
+  v[1] = mk(m1.x + n1.y, m1.y - n1.x);
+  v[4] = mk(m1.x - n1.y, m1.y + n1.x);
+  v[2] = mk(m2.x + n2.y, m2.y - n2.x);
+  v[3] = mk(m2.x - n2.y, m2.y + n2.x);
+}
+// A sum of constant multiples.  Its middle products are carried before they
+// could leave 64 bits: two terms fit while their fracs sum to at most 0.7.
+struct Acc {
+  ll h, m;
+  __device__ __forceinline__ Acc(ll start) : h(start), m(kHalf) {}
+  template <ll Q>
+  __device__ __forceinline__ void term(ll x) {
+    constexpr ll F = k_frac(Q);
+    constexpr int B = k_base(Q);
+    m = madw(lo(x), hi(F), madw(hi(x), lo(F), m));
+    h = madw(hi(x), hi(F), h);
+    if (B > 0) h += x;
+    if (B < 0) h -= x;
+  }
+  __device__ __forceinline__ void carry() {
+    h += m >> 32;
+    m &= 0xffffffffll;
+  }
+  __device__ __forceinline__ ll value() const { return h + (m >> 32); }
+};
+constexpr double k_abs(ll f) { return (f < 0 ? -(double)f : (double)f) / 18446744073709551616.0; }
+// Whether output m's sum over j is carried after term j: always after every
+// second one, and after the first of a pair whose fracs are too large.
+template <int R, int M>
+constexpr bool carry_after(int j) {
+  if (j % 2 == 0) return true;
+  const SC a = sincos_q62((j * M) % R, R), b = sincos_q62(((j + 1) * M) % R, R);
+  return k_abs(k_frac(a.c)) + k_abs(k_frac(b.c)) > 0.7 || k_abs(k_frac(a.s)) + k_abs(k_frac(b.s)) > 0.7;
+}
+// Odd prime R from the symmetric pairs (as dev::dft_odd).  Outputs go to
+// out(m, value) as they come, so that no second array of R values is live.
+template <int R, class Out>
+__device__ __forceinline__ void dft_odd(const I2* v, Out&& out) {
+  constexpr int H = (R - 1) / 2;
+  I2 t[H], u[H];
+  const I2 a0 = v[0];
+  I2 s0 = a0;
+  dev::static_for<0, H>([&](auto J) {
+    constexpr int j = decltype(J)::value + 1;
+    t[j - 1] = add(v[j], v[R - j]);
+    u[j - 1] = sub(v[j], v[R - j]);
+    s0 = add(s0, t[j - 1]);
+  });
+  out(0, s0);
+  dev::static_for<1, H + 1>([&](auto Mi) {
+    constexpr int m = decltype(Mi)::value;
+    Acc rx(a0.x), ry(a0.y), ix(0), iy(0);
+    dev::static_for<1, H + 1>([&](auto J) {
+      constexpr int j = decltype(J)::value;
+      constexpr SC w = sincos_q62((j * m) % R, R);
+      rx.template term<w.c>(t[j - 1].x);
+      ry.template term<w.c>(t[j - 1].y);
+      ix.template term<w.s>(u[j - 1].x);
+      iy.template term<w.s>(u[j - 1].y);
+      if (carry_after<R, m>(j) && j < H) {
+        rx.carry();
+        ry.carry();
+        ix.carry();
+        iy.carry();
+      }
+    });
+    const ll a = rx.value(), b = ry.value(), c = ix.value(), d = iy.value();
+    out(m, mk(a + d, b - c));
+    out(R - m, mk(a - d, b + c));
+  });
+}
+template <int R>
+__device__ __forceinline__ void dft(I2* v);
+// R = P Q: DFT_P over n1 of n = Q n1 + n2, W_R^(n2 k1), DFT_Q over n2
+template <int R, int P>
+__device__ __forceinline__ void dft_pq(I2* v) {
+  constexpr int Q = R / P;
+  I2 a[R];
+  dev::static_for<0, Q>([&](auto I) {
+    constexpr int n2 = decltype(I)::value;
+    I2 t[P];
+    dev::static_for<0, P>([&](auto J) { t[decltype(J)::value] = v[Q * decltype(J)::value + n2]; });
+    dft<P>(t);
+    dev::static_for<0, P>([&](auto K) {
+      constexpr int k1 = decltype(K)::value;
+      a[n2 * P + k1] = mul_root<R, n2 * k1>(t[k1]);
+    });
+  });
+  dev::static_for<0, P>([&](auto K) {
+    constexpr int k1 = decltype(K)::value;
+    I2 u[Q];
+    dev::static_for<0, Q>([&](auto I) { u[decltype(I)::value] = a[decltype(I)::value * P + k1]; });
+    dft<Q>(u);
+    dev::static_for<0, Q>([&](auto I) { v[k1 + P * decltype(I)::value] = u[decltype(I)::value]; });
+  });
+}
+template <int R>
+__device__ __forceinline__ void dft(I2* v) {
+  if constexpr (R == 1) {
+  } else if constexpr (R == 2) {
+    const I2 a = v[0];
+    v[0] = add(a, v[1]);
+    v[1] = sub(a, v[1]);
+  } else if constexpr (R == 3) {
+    dft3p(v);
+  } else if constexpr (R == 4) {
+    dft4v(v[0], v[1], v[2], v[3]);
+  } else if constexpr (R == 5) {
+    dft5p(v);
+  } else if constexpr (R % 4 == 0) {
+    dft_pq<R, 4>(v);
+  } else if constexpr (R % 5 == 0) {
+    dft_pq<R, 5>(v);
+  } else if constexpr (R % 3 == 0) {
+    dft_pq<R, 3>(v);
+  } else if constexpr (R % 2 == 0) {
+    dft_pq<R, 2>(v);
+  } else {
+    dft_odd<R>(v, [&](int m, I2 x) { v[m] = x; });
+  }
+}
+
+// ---- between doubles and a line's integers ---------------------------------
+// m: the largest magnitude's high word of a line; em = m >> 20 its biased
+// exponent.  A finite line whose exponent lies in [kMinExp, kMaxExp] runs in
+// integers: its results then neither overflow nor leave the normal range.
+constexpr int kMinExp = 200, kMaxExp = 1990;
+
+__device__ __forceinline__ int abs_hi(double v) { return __double2hiint(v) & 0x7fffffff; }
+__device__ __forceinline__ int max_hi(double2 v) { return max(fx::abs_hi(v.x), fx::abs_hi(v.y)); }
+__device__ __forceinline__ int any_lo(double2 v) { return __double2loint(v.x) | __double2loint(v.y); }
+// A value's share of the line's sum of moduli, over 2^(em - 1023), from the
+// larger component's high word h: 20 mantissa bits as a float (an upward
+// margin of 2^-17 a value covers the rest).
+__device__ __forceinline__ float share(int h, int base) { return __int_as_float(max(h - base, 0) << 3); }
+__device__ __forceinline__ int share_base(int em) { return (em - 127) << 20; }
+__device__ __forceinline__ unsigned share_units(float sum, int count) {
+  return (unsigned)(sum * 131072.0f) + (unsigned)count + 1;  // units of 2^(em - 1040)
+}
+// x as an integer, rounded: 61 mantissa bits shifted right by sh - e (not
+// negative); `flip` = 0x80000000 negates.
+__device__ __forceinline__ ll to_fixed(double x, int sh, int flip = 0) {
+  const int h = __double2hiint(x);
+  const unsigned l = (unsigned)__double2loint(x);
+  int s = sh - ((h >> 20) & 0x7ff);
+  s = s < 63 ? s : 63;
+  const unsigned mh = (unsigned)(h & 0xfffff) | 0x100000u;
+  const unsigned long long m = (((unsigned long long)mh << 32) | l) << 9;
+  const ll v = (ll)(((m >> s) + 1) >> 1);
+  return (h ^ flip) < 0 ? -v : v;
+}
+// an integer as a double times 2^(adj >> 20) (the result is normal or zero);
+// `flip` = 0x80000000 negates
+__device__ __forceinline__ double to_double(ll v, int adj, int flip = 0) {
+  const double d = __ll2double_rn(v);
+  const int h = __double2hiint(d);
+  return __hiloint2double((h != 0 ? h + adj : 0) ^ flip, __double2loint(d));
+}
+
+// The lines of a CTA that fixed point does not take, in FP64: as many lines
+// at a time as two buffers of the CTA's shared memory hold.
+template <int KIND, bool CONTIG>
+__device__ __noinline__ void fallback(const PassArgs& a, double2* buf) {
+  const int threads = blockDim.x * blockDim.y, tid = threadIdx.x + threadIdx.y * blockDim.x;
+  const int G = a.L > 1 ? a.L / 2 : 1, tpl = threads / G;
+  const int t = CONTIG ? tid % tpl : tid / G, line = CONTIG ? tid / tpl : tid % G;
+  for (int g = 0; g < a.L; g += G) {
+    dev::LineCtx<double, KIND, CONTIG> c;
+    const long long cl = (long long)blockIdx.x * a.L + g + line;
+    c.init_at(a, t, line, cl, CONTIG ? 0 : (long long)blockIdx.y, a.nlines);
+    c.L = G;
+    c.tpl = tpl;
+    if (g + line >= a.L) c.valid = false;
+    // threads left over by the division take no point
+    if (t >= tpl || line >= G) {
+      c.t = a.n;
+      c.line = 0;
+      c.valid = false;
+    }
+    dev::run_pp_lines<double, KIND, CONTIG>(c, a, buf, (size_t)a.n * G);
+    __syncthreads();
+  }
+}
+
+}  // namespace fx
+}  // namespace gbfft

@@ -1,0 +1,300 @@
+// Fixed-point axis passes of FP64 lines (fft_fx.cuh) with compile-time plans:
+// the arithmetic and the scale of fft_fx.cu for the common lengths, with the
+// points in registers and one exchange buffer.
+//
+// What bounds the runtime-planned kernel is the integer and address
+// instructions it issues (390 a point at 512 points, 2.1 a clock and SM with
+// 16 warps).  With the length known the slots and strides fold into the
+// instructions, the first stage starts from the loaded registers, the last
+// one stores from them, and half the shared memory and registers a thread
+// leave room for more warps.
+#pragma once
+
+#include "fft_fx.cuh"
+
+namespace gbfft {
+namespace fx {
+
+using namespace dev;
+
+// n = R0 R1 R2 R3 in that order; TPL threads a line, each with butterflies
+// t, t + TPL, ... of a stage.
+template <int N_, int TPL_, int R0, int R1 = 1, int R2 = 1, int R3 = 1>
+struct Plan {
+  static constexpr int N = N_, TPL = TPL_;
+  static constexpr int NST = R3 > 1 ? 4 : R2 > 1 ? 3 : R1 > 1 ? 2 : 1;
+  __host__ __device__ static constexpr int radix(int s) { return s == 0 ? R0 : s == 1 ? R1 : s == 2 ? R2 : R3; }
+  __host__ __device__ static constexpr int ns(int s) {
+    int v = 1;
+    for (int i = 0; i < s; ++i) v *= radix(i);
+    return v;
+  }
+  __host__ __device__ static constexpr int mb(int s) { return (N / radix(s) + TPL - 1) / TPL; }
+  __host__ __device__ static constexpr int points() {
+    int e = 0;
+    for (int s = 0; s < NST; ++s)
+      if (mb(s) * radix(s) > e) e = mb(s) * radix(s);
+    return e;
+  }
+  // powers of two that stage s divides its inputs by (its twiddles do)
+  __host__ __device__ static constexpr int sh(int s) { return s == 0 ? 0 : radix(s - 1) >= 16 ? 2 : 1; }
+  __host__ __device__ static constexpr int shift(int s) {
+    int v = 0;
+    for (int i = 0; i <= s; ++i) v += sh(i);
+    return v;
+  }
+  __host__ __device__ static constexpr int lg(int s) {
+    int l = 0;
+    while ((1 << l) < ns(s + 1)) ++l;
+    return l;
+  }
+  static_assert(R0 * R1 * R2 * R3 == N_, "radices");
+};
+
+// Exchange slots: contiguous lines padded by one entry in eight (a quarter
+// warp's 16-byte accesses cover the banks once), strided tiles dense (the
+// lanes walk the lines).
+template <class P, bool CONTIG>
+struct Slots {
+  static constexpr int kLine = P::N + P::N / 8 + 1;
+  int base, L;
+  __device__ __forceinline__ int operator()(int n) const { return CONTIG ? base + n + (n >> 3) : n * L + base; }
+};
+
+// Global accesses of a thread's points t + n, n known at compile time: one
+// multiply-add an address (the row strides are below 2^32 bytes).
+template <int KIND, bool CONTIG>
+struct Io {
+  const LineCtx<double, KIND, CONTIG>& c;
+  const char *s0, *s1;
+  char *d0, *d1;
+  unsigned ss, ds;
+  __device__ __forceinline__ explicit Io(const LineCtx<double, KIND, CONTIG>& ctx) : c(ctx) {
+    constexpr int SB = KIND == K_R2C ? 8 : 16, DB = KIND == K_C2R ? 8 : 16;
+    ss = (unsigned)c.ssn * SB;
+    ds = (unsigned)c.dsn * DB;
+    s0 = reinterpret_cast<const char*>(c.src) + c.sb0 * SB + (unsigned long long)ss * (unsigned)c.t;
+    s1 = reinterpret_cast<const char*>(c.src) + c.sb1 * SB + (unsigned long long)ss * (unsigned)c.t;
+    d0 = reinterpret_cast<char*>(c.dst) + c.db0 * DB + (unsigned long long)ds * (unsigned)c.t;
+    d1 = reinterpret_cast<char*>(c.dst) + c.db1 * DB + (unsigned long long)ds * (unsigned)c.t;
+  }
+#ifdef GB_DEBUG_BOUNDS
+  __device__ __forceinline__ double2 load(int n) const { return c.gload_raw(c.t + n); }
+  __device__ __forceinline__ double2 half(int which, int n) const { return c.half(which, c.t + n); }
+  __device__ __forceinline__ void store(int n, double2 v) const { c.gstore_raw(c.t + n, v); }
+  __device__ __forceinline__ void put_half(int which, int n, double2 v) const { c.put_half(which, c.t + n, v); }
+#else
+  __device__ __forceinline__ unsigned long long so(int n) const { return (unsigned long long)(unsigned)n * ss; }
+  __device__ __forceinline__ unsigned long long dof(int n) const { return (unsigned long long)(unsigned)n * ds; }
+  __device__ __forceinline__ double2 load(int n) const {
+    if (!c.valid) return make_double2(0, 0);
+    if (KIND == K_C2C || (!CONTIG && c.pvec && c.has1)) return *reinterpret_cast<const double2*>(s0 + so(n));
+    return make_double2(*reinterpret_cast<const double*>(s0 + so(n)),
+                        c.has1 ? *reinterpret_cast<const double*>(s1 + so(n)) : 0.0);
+  }
+  __device__ __forceinline__ double2 half(int which, int n) const {
+    if (!c.valid || (which && !c.has1)) return make_double2(0, 0);
+    return *reinterpret_cast<const double2*>((which ? s1 : s0) + so(n));
+  }
+  __device__ __forceinline__ void store(int n, double2 v) const {
+    if (!c.valid) return;
+    if (KIND == K_C2C || (!CONTIG && c.pvec && c.has1)) {
+      *reinterpret_cast<double2*>(d0 + dof(n)) = v;
+      return;
+    }
+    *reinterpret_cast<double*>(d0 + dof(n)) = v.x;
+    if (c.has1) *reinterpret_cast<double*>(d1 + dof(n)) = v.y;
+  }
+  __device__ __forceinline__ void put_half(int which, int n, double2 v) const {
+    if (c.valid && (!which || c.has1)) *reinterpret_cast<double2*>((which ? d1 : d0) + dof(n)) = v;
+  }
+#endif
+};
+
+template <class P, int S, bool FROM_SMEM, int KIND, bool CONTIG>
+__device__ __forceinline__ void run(const Io<KIND, CONTIG>& io, I2* Sm, const Slots<P, CONTIG>& slot, const W4* __restrict__ tw,
+                                    I2 (&v)[P::points()], int adj, int flip) {
+  constexpr int R = P::radix(S), NS = P::ns(S), NB = P::N / R, MB = P::mb(S), TPL = P::TPL;
+  constexpr bool LAST = S == P::NST - 1;
+  const int t = io.c.t;
+  if constexpr (FROM_SMEM) {
+#pragma unroll
+    for (int m = 0; m < MB; ++m) {
+      const int b = t + m * TPL;
+      if ((NB % TPL != 0 && b >= NB)) break;
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[m * R + r] = Sm[slot(b + r * NB)];
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < MB; ++m) {
+    const int b = t + m * TPL;
+    if ((NB % TPL != 0 && b >= NB)) break;
+    if constexpr (NS > 1) {
+      const W4* w = tw + (NS - 1) + b % NS;
+      constexpr int SH = P::sh(S);
+      v[m * R] = mk(scale_down<SH>(v[m * R].x), scale_down<SH>(v[m * R].y));
+#pragma unroll
+      for (int r = 1; r < R; ++r) v[m * R + r] = mul_tw<SH>(v[m * R + r], ldw(w + (r - 1) * NS), r);
+    }
+    dft<R>(&v[m * R]);
+  }
+  if constexpr (LAST && KIND != K_R2C) {
+#pragma unroll
+    for (int m = 0; m < MB; ++m) {
+      const int b = t + m * TPL;
+      if ((NB % TPL != 0 && b >= NB)) break;
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        io.store(m * TPL + r * NS, make_double2(to_double(v[m * R + r].x, adj), to_double(v[m * R + r].y, adj, flip)));
+    }
+  } else {
+    if constexpr (FROM_SMEM) __syncthreads();  // every point read before the outputs overwrite them
+#pragma unroll
+    for (int m = 0; m < MB; ++m) {
+      const int b = t + m * TPL;
+      if ((NB % TPL != 0 && b >= NB)) break;
+      const int k = b % NS, base = (b - k) * R + k;
+#pragma unroll
+      for (int r = 0; r < R; ++r) Sm[slot(base + r * NS)] = v[m * R + r];
+    }
+    __syncthreads();
+    if constexpr (!LAST) run<P, S + 1, true, KIND, CONTIG>(io, Sm, slot, tw, v, adj, flip);
+  }
+}
+
+// CTAs an SM the register budget aims at: 64 registers a thread for at most
+// ten points a thread (32 warps; 80 registers and 24 measured 15 % slower),
+// 128 for more.
+template <class P>
+__host__ __device__ constexpr int min_ctas() {
+  return 65536 / fxc_max_threads(P::TPL) / (P::points() > 10 ? 128 : 64);
+}
+template <class P, int KIND, bool CONTIG>
+__global__ void __launch_bounds__(fxc_max_threads(P::TPL), min_ctas<P>())
+    fxc_pass_kernel(const __grid_constant__ PassArgs a, const W4* __restrict__ tw) {
+  constexpr int N = P::N, TPL = P::TPL, E = P::points();
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  chained_entry();
+  LineCtx<double, KIND, CONTIG> c;
+  c.init(a);
+  const Io<KIND, CONTIG> io(c);
+  const int t = c.t, L = a.L;
+  I2* Sm = reinterpret_cast<I2*>(smem_raw);
+  Slots<P, CONTIG> slot;
+  slot.base = CONTIG ? c.line * Slots<P, CONTIG>::kLine : c.line;
+  slot.L = L;
+  // the lines' scale words, behind the exchange buffer
+  int* smax = reinterpret_cast<int*>(smem_raw + fxc_smem_bytes(N, L) - (size_t)L * 8);
+  unsigned* ssum = reinterpret_cast<unsigned*>(smax + L);
+  for (int i = threadIdx.x + threadIdx.y * blockDim.x; i < 2 * L; i += blockDim.x * blockDim.y) smax[i] = 0;
+  __syncthreads();
+
+  // 1. load: c2r both half spectra (point j in x[2 i], x[2 i + 1]), else the
+  // points of the first stage's butterflies
+  constexpr int H = N / 2 + 1, J = KIND == K_C2R ? (H + TPL - 1) / TPL : 1;
+  constexpr int R0 = P::radix(0), NB0 = N / R0, MB0 = P::mb(0);
+  constexpr int Q = KIND == K_C2R ? 2 * J : MB0 * R0;
+  double2 x[Q];
+  if constexpr (KIND == K_C2R) {
+#pragma unroll
+    for (int i = 0; i < J; ++i) {
+      const int j = t + i * TPL;
+      x[2 * i] = j < H ? io.half(0, i * TPL) : make_double2(0, 0);
+      x[2 * i + 1] = j < H ? io.half(1, i * TPL) : make_double2(0, 0);
+      if (j == 0 || 2 * j == N) x[2 * i].y = x[2 * i + 1].y = 0;  // Im of the DC and Nyquist bins is ignored
+    }
+  } else {
+#pragma unroll
+    for (int m = 0; m < MB0; ++m) {
+      const int b = t + m * TPL;
+      const bool in = NB0 % TPL == 0 || b < NB0;
+#pragma unroll
+      for (int r = 0; r < R0; ++r) x[m * R0 + r] = in ? io.load(m * TPL + r * NB0) : make_double2(0, 0);
+    }
+  }
+  // 2. the line's scale
+  int m = 0;
+#pragma unroll
+  for (int i = 0; i < Q; ++i) m = max(m, max_hi(x[i]));
+  atomicMax(&smax[c.line], m);
+  __syncthreads();
+  m = smax[c.line];
+  const int em = m >> 20;
+  float sum = 0;
+#pragma unroll
+  for (int i = 0; i < Q; ++i) sum += share(max_hi(x[i]), share_base(em));
+  atomicAdd(&ssum[c.line], share_units(sum, Q));
+  int bad = m != 0 && (em < kMinExp || em > kMaxExp);
+  if (m == 0) {  // all zero, or subnormals below 2^-1042
+#pragma unroll
+    for (int i = 0; i < Q; ++i) bad |= any_lo(x[i]);
+  }
+  if (__syncthreads_or(bad)) {
+    fallback<KIND, CONTIG>(a, reinterpret_cast<double2*>(smem_raw));
+    return;
+  }
+  const unsigned s15 = ssum[c.line];
+  constexpr int X = KIND == K_C2R ? 1 : 0;  // a point combines two values
+  const int es = 32 - __clz((int)(s15 + (s15 >> 1))) - 1040 + X;
+  int top = -1021 + X;
+#pragma unroll
+  for (int s = 0; s < P::NST; ++s) top = max(top, min(es, P::lg(s) - 1021 + X) - P::shift(s));
+  if (KIND == K_R2C && P::NST == 1) ++top;
+  const int sh = m == 0 ? 4096 : 1021 + top + em;  // a zero line shifts all out
+  int adj = (em - 62 + top + P::shift(P::NST - 1)) << 20;
+  // backward c2c: conjugated on the way in and out (c2r: out)
+  const int flip_in = KIND == K_C2C && c.inverse ? (int)0x80000000 : 0;
+  // 3. integers, and the stages
+  I2 v[E];
+  if constexpr (KIND == K_C2R) {
+#pragma unroll
+    for (int i = 0; i < J; ++i) {
+      const int j = t + i * TPL;
+      if (j < H) {
+        const ll ax = to_fixed(x[2 * i].x, sh), ay = to_fixed(x[2 * i].y, sh);
+        const ll bx = to_fixed(x[2 * i + 1].x, sh), by = to_fixed(x[2 * i + 1].y, sh);
+        // z = x1 + i x2, conjugated for the inverse-by-conjugation
+        Sm[slot(j)] = mk(ax - by, -(ay + bx));
+        if (j > 0 && 2 * j < N) Sm[slot(N - j)] = mk(ax + by, ay - bx);
+      }
+    }
+    __syncthreads();
+  } else {
+#pragma unroll
+    for (int i = 0; i < Q; ++i) v[i] = mk(to_fixed(x[i].x, sh), to_fixed(x[i].y, sh, flip_in));
+  }
+  run<P, 0, KIND == K_C2R, KIND, CONTIG>(io, Sm, slot, tw, v, adj, KIND == K_C2R ? (int)0x80000000 : flip_in);
+  if constexpr (KIND == K_R2C) {
+    adj -= 1 << 20;  // the halves of X1 = (Z_k + conj Z_{n-k}) / 2, X2 = (Z_k - conj Z_{n-k}) / 2i
+    constexpr int K = (H + TPL - 1) / TPL;
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+      const int k = t + i * TPL;
+      if (k < H) {
+        const I2 zk = Sm[slot(k)], zm = Sm[slot(k == 0 ? 0 : N - k)];
+        io.put_half(0, i * TPL, make_double2(to_double(zk.x + zm.x, adj), to_double(zk.y - zm.y, adj)));
+        io.put_half(1, i * TPL, make_double2(to_double(zk.y + zm.y, adj), to_double(zm.x - zk.x, adj)));
+      }
+    }
+  }
+}
+
+template <class P, int KIND, bool CONTIG>
+cudaError_t launch_p(const PassArgs& a, cudaStream_t stream) {
+  const size_t smem = fxc_smem_bytes(P::N, a.L);
+  if (a.tpl != P::TPL || a.L < 1 || a.L * a.tpl > fxc_max_threads(P::TPL) || smem > kFxMaxSmem) return cudaErrorInvalidValue;
+  auto kern = fxc_pass_kernel<P, KIND, CONTIG>;
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  const dim3 block = CONTIG ? dim3(a.tpl, a.L) : dim3(a.L, a.tpl);
+  const dim3 grid((unsigned)((a.nlines + a.L - 1) / a.L), CONTIG ? 1u : (unsigned)a.nv);
+  const cudaError_t err = launch_chained(kern, grid, block, smem, stream, a, reinterpret_cast<const W4*>(a.fx->tw));
+  add_launches(1);
+  return err != cudaSuccess ? err : cudaGetLastError();
+}
+
+}  // namespace fx
+}  // namespace gbfft

@@ -63,5 +63,60 @@ __device__ void stage_pp_generic(const Ctx& c, const Cx<T>* A, Cx<T>* B, int R, 
   }
 }
 
+// The runtime-planned pass of a CTA's lines (e points in all): loaded into
+// shared buffer 0, each stage ping-pongs between the two buffers, the result
+// is stored from the last buffer written.
+template <typename T, int KIND, bool CONTIG>
+__device__ __forceinline__ void run_pp_lines(const LineCtx<T, KIND, CONTIG>& c, const PassArgs& a, Cx<T>* buf0,
+                                             size_t e) {
+  using C = Cx<T>;
+  C* buf1 = buf0 + (e + (e >> 4) + 1);
+
+#pragma unroll 1
+  for (int n = c.t; n < c.N; n += c.tpl) buf0[c.sidx(n)] = c.gload(n);
+  __syncthreads();
+
+  C* A = buf0;
+  C* B = buf1;
+  int Ns = 1;
+#pragma unroll 1
+  for (int s = 0; s < a.nst; ++s) {
+    const int R = a.radix[s];
+    if (R == 16) stage_pp<T, KIND, CONTIG, 16>(c, A, B, Ns);
+    else if (R == 8) stage_pp<T, KIND, CONTIG, 8>(c, A, B, Ns);
+    else if (R == 4) stage_pp<T, KIND, CONTIG, 4>(c, A, B, Ns);
+    else if (R == 2) stage_pp<T, KIND, CONTIG, 2>(c, A, B, Ns);
+    else if (R == 3) stage_pp<T, KIND, CONTIG, 3>(c, A, B, Ns);
+    else if (R == 5) stage_pp<T, KIND, CONTIG, 5>(c, A, B, Ns);
+    else if (R == 7) stage_pp<T, KIND, CONTIG, 7>(c, A, B, Ns);
+    else if (R == 11) stage_pp<T, KIND, CONTIG, 11>(c, A, B, Ns);
+    else if (R == 13) stage_pp<T, KIND, CONTIG, 13>(c, A, B, Ns);
+    else if (R == 17) stage_pp<T, KIND, CONTIG, 17>(c, A, B, Ns);
+    else if (R == 19) stage_pp<T, KIND, CONTIG, 19>(c, A, B, Ns);
+    else if (R == 23) stage_pp<T, KIND, CONTIG, 23>(c, A, B, Ns);
+    else if (sizeof(T) == 4 && (R == 29 || R == 31)) {
+      // in FP64 a butterfly of 29 or 31 points does not fit the registers
+      if constexpr (sizeof(T) == 4) {
+        if (R == 29) stage_pp<T, KIND, CONTIG, 29>(c, A, B, Ns);
+        else stage_pp<T, KIND, CONTIG, 31>(c, A, B, Ns);
+      }
+    } else {
+      stage_pp_generic<T, KIND, CONTIG>(c, A, B, R, Ns);
+    }
+    __syncthreads();
+    C* tmp = A;
+    A = B;
+    B = tmp;
+    Ns *= R;
+  }
+
+  if (KIND == K_R2C) {
+    c.store_r2c(A);
+  } else {
+#pragma unroll 1
+    for (int n = c.t; n < c.N; n += c.tpl) c.gstore(n, A[c.sidx(n)]);
+  }
+}
+
 }  // namespace dev
 }  // namespace gbfft

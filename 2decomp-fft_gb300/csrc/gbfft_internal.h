@@ -61,6 +61,77 @@ struct BlueTables {
 // direct-sum stage costs that many multiply-adds a point.
 constexpr int kBluePrime = 256;
 
+// Fixed-point plan of one FP64 axis (fft_fx.cu): radix stages after ns
+// points, and for the line's scale, per stage, the exponent that bounds how
+// many inputs a value then sums (lg) and the powers of two it was divided
+// by (shift).  Built by the engine for one length; the struct lives on the
+// host and travels as a kernel argument.
+struct FxPlan {
+  int nst;
+  int radix[kMaxStages];
+  int ns[kMaxStages];
+  unsigned magic[kMaxStages];  // ceil(2^32 / ns)
+  int lg[kMaxStages];
+  int shift[kMaxStages];
+  const void* tw;    // stage-major Q62 roots (stage_twiddles order)
+  const void* root;  // the n roots in Q62, for direct-sum stages
+  int tpl;           // threads a line (runtime plans: at least n / kFxPoints)
+  int ct;            // 1: a compile-time plan (fft_fxc.cuh)
+};
+constexpr int kFxPoints = 8;        // points a thread loads at most
+constexpr int kFxMaxThreads = 512;  // threads of a CTA
+constexpr size_t kFxMaxSmem = 200 * 1024;
+// Shared memory of L lines of n points: two padded buffers and the lines'
+// scale words.
+__host__ __device__ constexpr size_t fx_smem_bytes(int n, int L) {
+  const size_t e = (size_t)n * (size_t)L;
+  return 2 * (e + (e >> 4) + 1) * 16 + (size_t)L * 8;
+}
+// ... and of the compile-time plans (fft_fxc.cuh): one buffer, padded by an
+// entry in eight; a single line keeps room for the two of its FP64 fallback.
+__host__ __device__ constexpr size_t fxc_smem_bytes(int n, int L) {
+  const size_t one = ((size_t)n + n / 8 + 2) * (size_t)L;
+  return (L == 1 ? 2 * one : one) * 16 + 32 + (size_t)L * 8;
+}
+// Lengths with a compile-time plan (fft_fxc.cuh): X(group, n, threads a line,
+// radices).  The radices stay at most 10 (64 registers a thread, four CTAs
+// of 256 threads an SM) but for 1024, 2048 and 4096 points, and the threads a line
+// are those that leave the fewest idle over the stages.  `group` splits the
+// instantiations over translation units.
+#define GBFFT_FXC_PLANS(X) \
+  X(0, 16, 4, 4, 4, 1, 1)     \
+  X(0, 32, 4, 8, 4, 1, 1)     \
+  X(0, 48, 8, 8, 6, 1, 1)     \
+  X(0, 64, 8, 8, 8, 1, 1)     \
+  X(0, 96, 12, 8, 4, 3, 1)    \
+  X(0, 126, 14, 9, 7, 2, 1)   \
+  X(0, 128, 16, 8, 4, 4, 1)   \
+  X(0, 160, 20, 10, 4, 4, 1)  \
+  X(0, 180, 20, 10, 9, 2, 1)  \
+  X(0, 192, 24, 8, 8, 3, 1)   \
+  X(1, 243, 27, 9, 9, 3, 1)   \
+  X(1, 256, 32, 8, 8, 4, 1)   \
+  X(1, 320, 40, 10, 8, 4, 1)  \
+  X(1, 384, 48, 8, 8, 6, 1)   \
+  X(1, 400, 50, 10, 8, 5, 1)  \
+  X(1, 512, 64, 8, 8, 8, 1)   \
+  X(1, 1024, 64, 16, 8, 8, 1) \
+  X(1, 2048, 128, 16, 16, 8, 1) \
+  X(1, 4096, 256, 16, 16, 16, 1)
+// threads of a CTA: 256, or what four lines (64-byte rows of a strided tile)
+// take
+__host__ __device__ constexpr int fxc_max_threads(int tpl) { return tpl <= 64 ? 256 : tpl <= 128 ? 4 * tpl : 512; }
+struct FxcShape {
+  int tpl, r[4];  // tpl 0: no compile-time plan
+};
+__host__ __device__ constexpr FxcShape fxc_shape(int n) {
+#define GBFFT_FXC_SHAPE(g, N, T, a, b, c, d) \
+  if (n == N) return FxcShape{T, {a, b, c, d}};
+  GBFFT_FXC_PLANS(GBFFT_FXC_SHAPE)
+#undef GBFFT_FXC_SHAPE
+  return FxcShape{0, {0, 0, 0, 0}};
+}
+
 struct PassArgs {
   const void* src;
   void* dst;
@@ -80,7 +151,8 @@ struct PassArgs {
   int fast;        // 1: compile-time power-of-two kernel, 2: mixed-radix kernel,
                    // 3: split-precision tensor-core kernel (mma.sync), 4:
                    // balanced non-power-of-two plan, 5: split-precision
-                   // tcgen05 kernel (fft_tc.cu)
+                   // tcgen05 kernel (fft_tc.cu), 6: fixed-point FP64 kernel
+                   // (fft_fx.cu), 7: its compile-time plans (fft_fxc.cuh)
   int pair_vec;    // r2c/c2r on strided lines, bit 0: the two real lines of a
                    // pair are adjacent and aligned (read/write as one pair);
                    // bit 1 (FP32): so are their two complex lines, 16-byte
@@ -104,6 +176,8 @@ struct PassArgs {
                    // caught an access outside an array (null: not recorded)
   long long src_elems, dst_elems;  // extents of the two arrays in elements of
                                    // each side's type (bounds-checked build)
+  const FxPlan* fx;  // fast == 6: host-side plan of the fixed-point FP64 pass
+                     // (fft_fx.cu); never read on the device
   const BlueTables* blue;  // host-side tables of the chirp-z path (fft_long.cu),
                            // null unless the axis runs it; never read on the device
   int radix[kMaxStages];
@@ -181,13 +255,16 @@ __host__ __device__ constexpr int gen_max_threads(int e, int prec_bytes) {
   return prec_bytes == 8 ? 256 : (e <= 16 ? 1024 : 512);
 }
 cudaError_t launch_gen_f32(int kind, bool contiguous, const PassArgs& a, cudaStream_t s);
-cudaError_t launch_gen_f64(int kind, bool contiguous, const PassArgs& a, cudaStream_t s);
 // Split-precision tensor-core passes (fft_split.cuh): FP32 lines of 256,
 // 512, 1024 points, 256-thread CTAs of split_lines_per_cta lines.
 bool split_length(int n);
 int split_lines_per_cta(int n, bool contiguous);
 cudaError_t launch_split_f32(int kind, bool contiguous, const PassArgs& a, cudaStream_t s);
-cudaError_t launch_mixed_f64(int kind, bool contiguous, const PassArgs& a, cudaStream_t s);
+// Lengths whose FP64 lines run in fixed point: up to 2048 points, and 4096,
+// whose plan divides by enough on the way.  On longer lines the headroom
+// costs more bits than a double's rounding (rel-L2 0.9 of the FP64 kernels'
+// at 4096 with radix-8 stages; 0.25 to 0.6 at 64 to 2048 points).
+__host__ __device__ constexpr bool fx_length(int n) { return (n >= 2 && n <= 2048) || n == 4096; }
 
 // Thread limit of the power-of-two kernel for E points a thread.
 __host__ __device__ constexpr int fast_max_threads(int e, int prec_bytes) {
@@ -203,8 +280,10 @@ __host__ __device__ constexpr long long fast_smem_entries(int n, int L) {
 
 cudaError_t launch_fast_f32_c2c(int kind, bool contiguous, const PassArgs& a, cudaStream_t s);
 cudaError_t launch_fast_f32_real(int kind, bool contiguous, const PassArgs& a, cudaStream_t s);
-cudaError_t launch_fast_f64_c2c(int kind, bool contiguous, const PassArgs& a, cudaStream_t s);
-cudaError_t launch_fast_f64_real(int kind, bool contiguous, const PassArgs& a, cudaStream_t s);
+
+// Compile-time plans, one function a kind and layout and group of lengths.
+cudaError_t launch_fxc(int kind, bool contiguous, const PassArgs& a, cudaStream_t s);
+cudaError_t launch_fx(int kind, bool contiguous, const PassArgs& a, cudaStream_t s);
 
 // The x and y passes of one z-plane run by one fused kernel
 // (fft_fused.cuh): ax holds the x pass with ax.nlines = complex x lines per
