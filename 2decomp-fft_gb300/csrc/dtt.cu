@@ -13,6 +13,12 @@
 //   DST-II(x)_k  = DCT-II((-1)^j x_j)_{n-1-k}
 //   DST-III(x)_k = (-1)^k DCT-III(x_{n-1-j})_k
 //   DST-IV(x)_k  = (-1)^k DCT-IV(x_{n-1-j})_k
+// FP64 windows whose FFT fits the fixed-point kernels run there, two real
+// lines a complex one and without the extensions (fft_r2r.cuh).  In FP32 that
+// form measured 1.9 to 2.4 times as fast as the one here, but its rel-L2
+// against 64 bits is up to 1.6 times as large (the second line's rounding
+// errors join the first's), so FP32 stays with one extended line a transform.
+//
 // A CTA owns L lines.  Each line's extension is built in shared memory
 // straight from the real window, transformed by the runtime-planned Stockham
 // stages (fft_pp.cuh) and reduced to the n real outputs, which go back to the
@@ -411,15 +417,17 @@ size_t dtt_smem_bytes(int prec_bytes, int M, int L) {
 namespace {
 cudaError_t launch_dtt_one(int prec_bytes, bool contiguous, const DttArgs& a, cudaStream_t stream) {
   if (a.n < 1 || a.M < 2 || a.L < 1 || a.tpl < 1) return cudaErrorInvalidValue;
-  if (a.twf && dtt_mixed_length(a.M)) {
-    // FP32 only: the engine keeps FP64 on the runtime plan
-    if (prec_bytes != 4) return cudaErrorInvalidValue;
-    return contiguous ? launch_mixed<float, true>(a, stream) : launch_mixed<float, false>(a, stream);
+  if (a.fx) {
+    if (prec_bytes != 8) return cudaErrorInvalidValue;
+    return a.fx->ct ? launch_fxc_r2r(contiguous, a, stream) : launch_fx_r2r(contiguous, a, stream);
   }
   if (a.twf) {
+    // compile-time plans: FP32 only (FP64 runs in fixed point or on the runtime plan)
+    if (prec_bytes != 4) return cudaErrorInvalidValue;
+    if (dtt_mixed_length(a.M))
+      return contiguous ? launch_mixed<float, true>(a, stream) : launch_mixed<float, false>(a, stream);
     if (!dtt_fast_length(a.M)) return cudaErrorInvalidValue;
-    if (prec_bytes == 4) return contiguous ? launch_fast<float, true>(a, stream) : launch_fast<float, false>(a, stream);
-    return contiguous ? launch_fast<double, true>(a, stream) : launch_fast<double, false>(a, stream);
+    return contiguous ? launch_fast<float, true>(a, stream) : launch_fast<float, false>(a, stream);
   }
   if (a.L * a.tpl > kMaxThreads) return cudaErrorInvalidValue;
   if (prec_bytes == 4) return contiguous ? launch_t<float, true>(a, stream) : launch_t<float, false>(a, stream);

@@ -317,7 +317,7 @@ int upload_batch_table(AxisPlan& p, int prec) {
 }
 
 // Radices of the fixed-point kernel's compile-time butterflies.
-constexpr int kFxRadices[] = {2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 13};
+constexpr int kFxRadices[] = {2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 13, 17};
 // Relative cost of a point in a stage of radix r, beside its exchange and
 // twiddle (kFxStageCost).
 constexpr double kFxStageCost = 24;
@@ -334,6 +334,7 @@ double fx_radix_cost(int r) {
     case 10: return 13;
     case 11: return 38;
     case 13: return 46;
+    case 17: return 64;
     default: return 26.0 * r;  // direct sum
   }
 }
@@ -651,14 +652,16 @@ void drop_profile(gbfft_engine_t e) {
   e->prof.clear();
 }
 
+void free_tables(AxisPlan& a) {
+  for (void** q : {&a.d_tw, &a.d_twf, &a.d_twfb, &a.d_fxtw, &a.d_fxroot, &a.d_chirp, &a.d_filt, &a.d_twm}) {
+    if (*q) dev_free(*q);
+    *q = nullptr;
+  }
+}
+
 void release(gbfft_engine_t e) {
   drop_profile(e);
-  for (auto& a : e->ax) {
-    for (void** q : {&a.d_tw, &a.d_twf, &a.d_twfb, &a.d_fxtw, &a.d_fxroot, &a.d_chirp, &a.d_filt, &a.d_twm}) {
-      if (*q) dev_free(*q);
-      *q = nullptr;
-    }
-  }
+  for (auto& a : e->ax) free_tables(a);
   if (e->work) dev_free(e->work);
   e->work = nullptr;
   if (e->d_sync) dev_free(e->d_sync);
@@ -1927,11 +1930,11 @@ constexpr unsigned kDttMagic = 0x47424454u;  // "GBDT"
 
 struct DttAxis {
   int kind = 0, off = 0, n = 0, M = 0;
-  AxisPlan plan;        // radix stages of M
-  void* tw = nullptr;   // exp(-2 pi i m / M)
-  void* twf = nullptr;  // power-of-two M: stage-major table of the 16-point plan
-  void* w4 = nullptr;   // exp(-2 pi i m / (4 n)), m < n
+  AxisPlan plan;         // of the M-point FFT, with its tables
+  void* w4 = nullptr;    // exp(-2 pi i m / (4 n)), m < n
   double c0x = 1, c0y = 0;
+  void* w = nullptr;     // fixed point: roots of the maps around the FFT
+  void* w_fx = nullptr;  // the same in Q62
 };
 
 }  // namespace
@@ -1952,10 +1955,11 @@ bool valid_dtt(gbfft_dtt_t d) { return d != nullptr && d->magic == kDttMagic; }
 void release_dtt(gbfft_dtt_t d) {
   for (auto& dir : d->ax)
     for (DttAxis& a : dir) {
-      if (a.tw) dev_free(a.tw);
-      if (a.twf) dev_free(a.twf);
-      if (a.w4) dev_free(a.w4);
-      a.tw = a.twf = a.w4 = nullptr;
+      free_tables(a.plan);
+      for (void** q : {&a.w4, &a.w, &a.w_fx}) {
+        if (*q) dev_free(*q);
+        *q = nullptr;
+      }
     }
 }
 
@@ -1992,31 +1996,50 @@ int dtt_config(const int* in, int nin, int* c) {
   return GBFFT_OK;
 }
 
-int setup_dtt_axis(DttAxis& a, int kind, int first, int ndismiss, int naxis, int prec) {
+int setup_dtt_axis(DttAxis& a, int kind, int first, int ndismiss, int naxis, int prec, double cells) {
   a.kind = kind;
   a.off = first - 1;
   a.n = naxis - ndismiss;
   if (a.off < 0 || a.n < 1 || a.off + a.n > naxis || (kind == 1 && a.n < 2))
     return fail(GBFFT_ERR_INVALID, "r2r window outside the axis");
-  a.M = kind == 1 ? 2 * (a.n - 1) : kind == 5 ? 2 * (a.n + 1) : 2 * a.n;
-  std::string why;
-  if (!factorize(a.M, a.plan, why)) return fail(GBFFT_ERR_UNSUPPORTED, "r2r extension: " + why);
-  if (a.M > kMaxN || dtt_smem_bytes(prec, a.M, 1) > 200 * 1024)
+  // windows up to the length whose extension fits one tile
+  const int ext = kind == 1 ? 2 * (a.n - 1) : kind == 5 ? 2 * (a.n + 1) : 2 * a.n;
+  if (ext > kMaxN || dtt_smem_bytes(prec, ext, 1) > 200 * 1024)
     return fail(GBFFT_ERR_UNSUPPORTED, "r2r extension does not fit one shared-memory tile");
-  int rc = upload_table(&a.tw, twiddles(a.M), prec);
+  std::string why;
+  if (prec == GBFFT_PREC_DOUBLE && fx_length(dtt_fft_length(kind, a.n))) {
+    a.M = dtt_fft_length(kind, a.n);
+    if (!factorize(a.M, a.plan, why)) return fail(GBFFT_ERR_UNSUPPORTED, "r2r transform: " + why);
+    // roots of the maps: exp(-2 pi i k / (4 n)), or of the even DCT-IV
+    // exp(-2 pi i (8 k + 1) / (16 n))
+    const bool even4 = kind % 4 == 0 && a.n % 2 == 0;
+    std::vector<long double> w(kind == 1 || kind == 5 ? 2 : 2 * (size_t)a.n);
+    const long double two_pi = 6.283185307179586476925286766559005768L;
+    for (size_t k = 0; 2 * k < w.size(); ++k) {
+      const long double t =
+          even4 ? two_pi * (long double)(8 * k + 1) / (16.0L * a.n) : two_pi * (long double)k / (4.0L * a.n);
+      w[2 * k] = cosl(t);
+      w[2 * k + 1] = -sinl(t);
+    }
+    int rc = upload_table(&a.w, std::vector<double>(w.begin(), w.end()), prec);
+    if (rc == GBFFT_OK) rc = upload_ints(&a.w_fx, q62_table(w));
+    if (rc != GBFFT_OK) return rc;
+    // small grids (two real lines a complex one): radix 4, as the axis passes
+    a.plan.fx = fx_plan(a.M, cells / 2 / kFxPoints < 512.0 * kSmsDefault ? 4 : 10, true);
+    return upload_fx(a.plan);
+  }
+  a.M = ext;
+  if (!factorize(a.M, a.plan, why)) return fail(GBFFT_ERR_UNSUPPORTED, "r2r extension: " + why);
+  int rc = upload_table(&a.plan.d_tw, twiddles(a.M), prec);
   if (rc != GBFFT_OK) return rc;
-  // the two-stage plan in FP32 only: in FP64 its 30-point butterflies take
-  // 210 registers a thread and the 510-point pass ran slower than the
-  // runtime-planned one
-  const bool mixed = dtt_mixed_length(a.M) && prec == GBFFT_PREC_SINGLE;
-  if (dtt_fast_length(a.M) || mixed) {
+  if (prec == GBFFT_PREC_SINGLE && (dtt_fast_length(a.M) || dtt_mixed_length(a.M))) {
     std::vector<int> radices;
-    if (mixed) {
+    if (dtt_mixed_length(a.M)) {
       radices = {mixed_r0(a.M), a.M / mixed_r0(a.M)};
     } else {
       for (int s = 0; s < fast_nst(a.M, 16); ++s) radices.push_back(fast_radix(a.M, 16, s));
     }
-    rc = upload_table(&a.twf, stage_twiddles(radices), prec);
+    rc = upload_table(&a.plan.d_twf, stage_twiddles(radices), prec);
     if (rc != GBFFT_OK) return rc;
   }
   std::vector<double> w = twiddles(4 * a.n);
@@ -2057,7 +2080,7 @@ int gbfft_dtt_create(int format, int nx, int ny, int nz, const int* skip, int pr
       if (d->skip[k]) continue;
       const int kind = d->cfg[dir == 0 ? k : 12 + k];
       const int first = d->cfg[dir == 0 ? 3 + k : 9 + k];
-      rc = setup_dtt_axis(d->ax[dir][k], kind, first, d->cfg[6 + k], lens[k], prec);
+      rc = setup_dtt_axis(d->ax[dir][k], kind, first, d->cfg[6 + k], lens[k], prec, (double)nx * ny * nz);
     }
   if (rc != GBFFT_OK) {
     const std::string msg = g_err;
@@ -2125,11 +2148,14 @@ int gbfft_exec_r2r(gbfft_dtt_t d, void* d_in, void* d_out, int isign, void* stre
     a.M = ax.M;
     a.nst = ax.plan.nst;
     for (int s = 0; s < kMaxStages; ++s) a.radix[s] = s < ax.plan.nst ? ax.plan.radix[s] : 0;
-    a.tw = ax.tw;
-    a.twf = ax.twf;
+    a.tw = ax.plan.d_tw;
+    a.twf = ax.plan.d_twf;
     a.w4 = ax.w4;
     a.c0x = ax.c0x;
     a.c0y = ax.c0y;
+    a.w = ax.w;
+    a.w_fx = ax.w_fx;
+    a.fx = ax.plan.fx.nst ? &ax.plan.fx : nullptr;
     const bool contiguous = k == 0;
     if (k == 0) {
       a.sn = 1;
@@ -2150,7 +2176,21 @@ int gbfft_exec_r2r(gbfft_dtt_t d, void* d_in, void* d_out, int isign, void* stre
       a.nv = (int)ny;
       a.naxis = (int)nz;
     }
-    if (ax.twf && dtt_mixed_length(ax.M)) {
+    if (a.fx) {
+      // strided pairs are neighbouring x positions
+      a.pair_vec = !contiguous && nx % 2 == 0 && ((uintptr_t)src | (uintptr_t)dst) % (2 * (size_t)d->prec) == 0;
+      const long long lines = dtt_complex_lines(a);
+      a.tpl = a.fx->tpl;
+      a.L = fx_lines_per_cta(*a.fx, a.M, contiguous, lines, a.nv, 0);
+      // one real line each: twice as many for the same row segments
+      const int maxt = a.fx->ct ? fxc_max_threads(a.tpl) : kFxMaxThreads;
+      if (a.kind % 4 == 0 && a.n % 2 == 0 && !contiguous)
+        while (2 * a.L <= 16 && 2 * a.L * a.tpl <= maxt && 2 * a.L <= lines) a.L *= 2;
+      cudaError_t err = launch_dtt_pass(d->prec, contiguous, a, st);
+      if (err != cudaSuccess) return cuda_fail(err, "r2r pass launch");
+      continue;
+    }
+    if (ax.plan.d_twf && dtt_mixed_length(ax.M)) {
       // compile-time two-stage plan: R1 threads a line, at most 256 a CTA;
       // contiguous about 128, strided up to 16 neighbouring lines
       const int tplm = ax.M / mixed_r0(ax.M);
@@ -2164,7 +2204,7 @@ int gbfft_exec_r2r(gbfft_dtt_t d, void* d_in, void* d_out, int isign, void* stre
       if (err != cudaSuccess) return cuda_fail(err, "r2r pass launch");
       continue;
     }
-    if (ax.twf) {
+    if (ax.plan.d_twf) {
       // compile-time 16-point plan: M / 16 threads a line; contiguous
       // 128-thread CTAs, strided up to 16 neighbouring lines
       const int tplf = ax.M / 16, maxt = fast_max_threads(16, d->prec);

@@ -21,6 +21,7 @@
 // fx::kMinExp..kMaxExp runs its lines in FP64 instead (fx::fallback), with the
 // result those had before.
 #include "fft_fx.cuh"
+#include "fft_r2r.cuh"
 
 namespace gbfft {
 
@@ -81,6 +82,40 @@ __device__ void fx_stage_generic(const Ctx& c, const I2* A, I2* B, const W4* __r
   }
 }
 
+// The stages of a plan on the lines in A, ping-ponging with B; returns the
+// buffer that holds the result.
+template <class Ctx>
+__device__ __forceinline__ const I2* fx_stages(const Ctx& c, const FxPlan& p, I2* first, I2* second) {
+  const I2* A = first;
+  I2* B = second;
+  const W4* tw = reinterpret_cast<const W4*>(p.tw);
+#pragma unroll 1
+  for (int s = 0; s < p.nst; ++s) {
+    const int R = p.radix[s], Ns = p.ns[s];
+    const unsigned mg = p.magic[s];
+    switch (R) {
+      case 2: fx_stage<2>(c, A, B, tw, Ns, mg); break;
+      case 3: fx_stage<3>(c, A, B, tw, Ns, mg); break;
+      case 4: fx_stage<4>(c, A, B, tw, Ns, mg); break;
+      case 5: fx_stage<5>(c, A, B, tw, Ns, mg); break;
+      case 6: fx_stage<6>(c, A, B, tw, Ns, mg); break;
+      case 7: fx_stage<7>(c, A, B, tw, Ns, mg); break;
+      case 8: fx_stage<8>(c, A, B, tw, Ns, mg); break;
+      case 9: fx_stage<9>(c, A, B, tw, Ns, mg); break;
+      case 10: fx_stage<10>(c, A, B, tw, Ns, mg); break;
+      case 11: fx_stage<11>(c, A, B, tw, Ns, mg); break;
+      case 13: fx_stage<13>(c, A, B, tw, Ns, mg); break;
+      case 17: fx_stage<17>(c, A, B, tw, Ns, mg); break;
+      default: fx_stage_generic(c, A, B, reinterpret_cast<const W4*>(p.root), R, Ns); break;
+    }
+    __syncthreads();
+    I2* const done = B;
+    B = const_cast<I2*>(A);
+    A = done;
+  }
+  return A;
+}
+
 template <int KIND, bool CONTIG>
 __global__ void __launch_bounds__(kFxMaxThreads) fx_pass_kernel(const __grid_constant__ PassArgs a,
                                                                 const __grid_constant__ FxPlan p) {
@@ -105,7 +140,6 @@ __global__ void __launch_bounds__(kFxMaxThreads) fx_pass_kernel(const __grid_con
   constexpr int W = KIND == K_C2R ? 2 : 1;
   const int cnt = KIND == K_C2R ? N / 2 + 1 : N;
   double2 v[J * W];
-  int m = 0;
 #pragma unroll
   for (int i = 0; i < J; ++i) {
     const int n = t + i * tpl;
@@ -117,39 +151,19 @@ __global__ void __launch_bounds__(kFxMaxThreads) fx_pass_kernel(const __grid_con
       v[i] = n < cnt ? c.gload_raw(n) : make_double2(0, 0);
     }
   }
-#pragma unroll
-  for (int i = 0; i < J * W; ++i) m = max(m, fx::max_hi(v[i]));
-  atomicMax(&smax[c.line], m);
-  __syncthreads();
-  m = smax[c.line];
-  const int em = m >> 20;
-  float sum = 0;
-#pragma unroll
-  for (int i = 0; i < J * W; ++i) sum += fx::share(fx::max_hi(v[i]), fx::share_base(em));
-  atomicAdd(&ssum[c.line], fx::share_units(sum, J * W));
-  int bad = m != 0 && (em < fx::kMinExp || em > fx::kMaxExp);
-  if (m == 0) {  // all zero, or subnormals below 2^-1042
-#pragma unroll
-    for (int i = 0; i < J * W; ++i) bad |= fx::any_lo(v[i]);
-  }
-  if (__syncthreads_or(bad)) {
+  fx::Scale sc;
+  if (!sc.find<J * W>(v, &smax[c.line], &ssum[c.line])) {
     fx::fallback<KIND, CONTIG>(a, reinterpret_cast<double2*>(smem_raw));
     return;
   }
-  // exponents (less em) of what bounds the moduli: the sum of all, and n
-  // times the largest; after each stage the smaller of the two holds
-  const unsigned S = ssum[c.line];
   constexpr int X = KIND == K_C2R ? 1 : 0;  // a point combines two values
-  const int es = 32 - __clz((int)(S + (S >> 1))) - 1040 + X;
   int top = -1021 + X;
 #pragma unroll 1
-  for (int s = 0; s < p.nst; ++s) top = max(top, min(es, p.lg[s] - 1021 + X) - p.shift[s]);
-  // the moduli may reach 2^62 (2^61 where r2c adds two values that no
-  // twiddle has halved)
+  for (int s = 0; s < p.nst; ++s) top = max(top, sc.bound(p.lg[s], X) - p.shift[s]);
+  // r2c adds two values that no twiddle has halved
   if (KIND == K_R2C && p.shift[p.nst - 1] == 0) ++top;
-  // right shift of a mantissa, less its exponent; a zero line shifts all out
-  const int sh = m == 0 ? 4096 : 1021 + top + em;
-  int adj = (em - 62 + top + p.shift[p.nst - 1]) << 20;  // exponent of a result's unit, in a high word
+  const int sh = sc.shift(top);
+  int adj = (sc.em - 62 + top + p.shift[p.nst - 1]) << 20;  // exponent of a result's unit, in a high word
 
   // backward: conjugated on the way in (c2r: by its combination) and out
   const int flip = c.inverse ? (int)0x80000000 : 0;
@@ -174,32 +188,7 @@ __global__ void __launch_bounds__(kFxMaxThreads) fx_pass_kernel(const __grid_con
   }
   __syncthreads();
 
-  const I2* A = buf0;
-  I2* B = buf1;
-  const W4* tw = reinterpret_cast<const W4*>(p.tw);
-#pragma unroll 1
-  for (int s = 0; s < p.nst; ++s) {
-    const int R = p.radix[s], Ns = p.ns[s];
-    const unsigned mg = p.magic[s];
-    switch (R) {
-      case 2: fx_stage<2>(c, A, B, tw, Ns, mg); break;
-      case 3: fx_stage<3>(c, A, B, tw, Ns, mg); break;
-      case 4: fx_stage<4>(c, A, B, tw, Ns, mg); break;
-      case 5: fx_stage<5>(c, A, B, tw, Ns, mg); break;
-      case 6: fx_stage<6>(c, A, B, tw, Ns, mg); break;
-      case 7: fx_stage<7>(c, A, B, tw, Ns, mg); break;
-      case 8: fx_stage<8>(c, A, B, tw, Ns, mg); break;
-      case 9: fx_stage<9>(c, A, B, tw, Ns, mg); break;
-      case 10: fx_stage<10>(c, A, B, tw, Ns, mg); break;
-      case 11: fx_stage<11>(c, A, B, tw, Ns, mg); break;
-      case 13: fx_stage<13>(c, A, B, tw, Ns, mg); break;
-      default: fx_stage_generic(c, A, B, reinterpret_cast<const W4*>(p.root), R, Ns); break;
-    }
-    __syncthreads();
-    I2* const done = B;
-    B = const_cast<I2*>(A);
-    A = done;
-  }
+  const I2* A = fx_stages(c, p, buf0, buf1);
 
   if constexpr (KIND == K_R2C) {
     adj -= 1 << 20;  // the halves of X1 = (Z_k + conj Z_{n-k}) / 2, X2 = (Z_k - conj Z_{n-k}) / 2i
@@ -236,7 +225,94 @@ cudaError_t launch_k(const PassArgs& a, cudaStream_t stream) {
   return err != cudaSuccess ? err : cudaGetLastError();
 }
 
+// A real-to-real pass (fft_r2r.cuh) in the same arithmetic.
+template <bool CONTIG>
+__global__ void __launch_bounds__(kFxMaxThreads) fx_r2r_kernel(const __grid_constant__ DttArgs a,
+                                                              const __grid_constant__ FxPlan p) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  chained_entry();
+  LineCtx<double, K_C2C, CONTIG> c;
+  c.N = a.M;
+  c.L = a.L;
+  c.tpl = a.tpl;
+  c.t = CONTIG ? threadIdx.x : threadIdx.y;
+  c.line = CONTIG ? threadIdx.y : threadIdx.x;
+  const r2r::Lines<double, CONTIG> ln(a, (long long)blockIdx.x * a.L + c.line, CONTIG ? 0 : (long long)blockIdx.y);
+  const int e = a.M * a.L, t = c.t, tpl = c.tpl, cnt = r2r::elements(a.kind, a.n);
+  I2* buf0 = reinterpret_cast<I2*>(smem_raw);
+  I2* buf1 = buf0 + (e + (e >> 4) + 1);
+  int* smax = reinterpret_cast<int*>(buf1 + (e + (e >> 4) + 1));
+  unsigned* ssum = reinterpret_cast<unsigned*>(smax + 2 * a.L);
+  const int threads = blockDim.x * blockDim.y;
+  for (int i = threadIdx.x + threadIdx.y * blockDim.x; i < 4 * a.L; i += threads) smax[i] = 0;
+  __syncthreads();
+  double2 x[kE];
+#pragma unroll
+  for (int i = 0; i < kE; ++i) {
+    const int j = t + i * tpl;
+    x[i] = j < cnt ? ln.element(j) : make_double2(0, 0);
+  }
+  r2r::PairScale sc;
+  if (!sc.find<kE>(x, &smax[2 * c.line], &ssum[2 * c.line], ln.single)) {
+    r2r::fallback<CONTIG>(a, reinterpret_cast<double2*>(smem_raw));
+    return;
+  }
+  using Map = r2r::Maps<r2r::Fixed, r2r::CtxSlot<LineCtx<double, K_C2C, CONTIG>>>;
+  const Map mp{a.kind, a.n, a.M, reinterpret_cast<const W4*>(a.w_fx), {&c}};
+  const int g = mp.grow(), pre = mp.pre(), last = p.nst - 1;
+  int ta = -1021 + g, tb = ta;
+#pragma unroll 1
+  for (int s = 0; s <= last; ++s) {
+    const int down = pre + p.shift[s] - (s == last ? mp.post() : 0);
+    ta = max(ta, sc.a.bound(p.lg[s], g) - down);
+    tb = max(tb, sc.b.bound(p.lg[s], g) - down);
+  }
+  const int sa = sc.a.shift(ta), sb = sc.b.shift(tb);
+  const int down = pre + p.shift[last] + mp.tail() + Map::doubled(a.kind, a.n) - 62;
+  const int adj_a = (sc.a.em + ta + down) << 20, adj_b = (sc.b.em + tb + down) << 20;
+#pragma unroll
+  for (int i = 0; i < kE; ++i) {
+    const int j = t + i * tpl;
+    if (j < cnt) mp.place(buf0, j, fx::mk(fx::to_fixed(x[i].x, sa), fx::to_fixed(x[i].y, sb)));
+  }
+  __syncthreads();
+  if (mp.combines()) {
+#pragma unroll 1
+    for (int k = t; 2 * k <= a.n; k += tpl) mp.combine(buf0, k);
+    __syncthreads();
+  }
+  const I2* A = fx_stages(c, p, buf0, buf1);
+#pragma unroll 1
+  for (int k = t; k < mp.steps(); k += tpl)
+    mp.finish(
+        A, k, [&](int i, ll ya, ll yb) { ln.store(i, sc.a.out(ya, adj_a), sc.b.out(yb, adj_b)); },
+        [&](int i, ll y) { ln.store1(i, sc.a.out(y, adj_a)); });
+  ln.pass_through(a.naxis, t, tpl);
+}
+
+template <bool CONTIG>
+cudaError_t launch_r2r_k(const DttArgs& a, cudaStream_t stream) {
+  const size_t smem = fx_smem_bytes(a.M, a.L);
+  if (a.L < 1 || a.tpl < 1 || a.L * a.tpl > kFxMaxThreads || a.tpl * kE < a.M || smem > kFxMaxSmem)
+    return cudaErrorInvalidValue;
+  auto kern = fx_r2r_kernel<CONTIG>;
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  const long long lines = dtt_complex_lines(a);
+  const dim3 block = CONTIG ? dim3(a.tpl, a.L) : dim3(a.L, a.tpl);
+  const dim3 grid((unsigned)((lines + a.L - 1) / a.L), CONTIG ? 1u : (unsigned)a.nv);
+  const cudaError_t err = launch_chained(kern, grid, block, smem, stream, a, *a.fx);
+  add_launches(1);
+  return err != cudaSuccess ? err : cudaGetLastError();
+}
+
 }  // namespace
+
+cudaError_t launch_fx_r2r(bool contiguous, const DttArgs& a, cudaStream_t s) {
+  return contiguous ? launch_r2r_k<true>(a, s) : launch_r2r_k<false>(a, s);
+}
 
 cudaError_t launch_fx(int kind, bool contiguous, const PassArgs& a, cudaStream_t s) {
   if (kind == K_C2C) return contiguous ? launch_k<K_C2C, true>(a, s) : launch_k<K_C2C, false>(a, s);

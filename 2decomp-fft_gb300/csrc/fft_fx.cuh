@@ -361,6 +361,54 @@ __device__ __forceinline__ int share_base(int em) { return (em - 127) << 20; }
 __device__ __forceinline__ unsigned share_units(float sum, int count) {
   return (unsigned)(sum * 131072.0f) + (unsigned)count + 1;  // units of 2^(em - 1040)
 }
+// an integer as a double times 2^(adj >> 20) (the result is normal or zero);
+// `flip` = 0x80000000 negates
+__device__ __forceinline__ double to_double(ll v, int adj, int flip = 0) {
+  const double d = __ll2double_rn(v);
+  const int h = __double2hiint(d);
+  return __hiloint2double((h != 0 ? h + adj : 0) ^ flip, __double2loint(d));
+}
+
+// The scale of a line, from the values its threads hold.
+struct Scale {
+  int m, em, es;  // largest high word, its exponent, exponent of the sum of moduli (over 2^em)
+  // The line's scale words start at zero.  False (for the whole CTA): a line
+  // of the CTA must run in FP64.
+  template <int Q>
+  __device__ __forceinline__ bool find(const double2 (&x)[Q], int* smax, unsigned* ssum) {
+    m = 0;
+#pragma unroll
+    for (int i = 0; i < Q; ++i) m = max(m, max_hi(x[i]));
+    atomicMax(smax, m);
+    __syncthreads();
+    m = *smax;
+    em = m >> 20;
+    float sum = 0;
+#pragma unroll
+    for (int i = 0; i < Q; ++i) sum += share(max_hi(x[i]), share_base(em));
+    atomicAdd(ssum, share_units(sum, Q));
+    int bad = m != 0 && (em < kMinExp || em > kMaxExp);
+    if (m == 0) {  // all zero, or subnormals below 2^-1042
+#pragma unroll
+      for (int i = 0; i < Q; ++i) bad |= any_lo(x[i]);
+    }
+    if (__syncthreads_or(bad)) return false;
+    const unsigned s = *ssum;
+    es = 32 - __clz((int)(s + (s >> 1))) - 1040;  // a modulus is at most sqrt 2 times the larger component
+    return true;
+  }
+  // Exponent (less em) that bounds the modulus of a sum of at most 2^lg
+  // values, each raised by at most 2^grow: the sum of all, or 2^lg times the
+  // largest.
+  __device__ __forceinline__ int bound(int lg, int grow) const { return min(es, lg - 1021) + grow; }
+  // The moduli may reach 2^62 where exponent `top` bounds them: the right
+  // shift of a mantissa, less its exponent.  A zero line shifts all out.
+  __device__ __forceinline__ int shift(int top) const { return m == 0 ? 4096 : 1021 + top + em; }
+  // A result of a line that shares its transform: a zero line's is zero
+  // whatever the other's rounding left there.
+  __device__ __forceinline__ double out(ll v, int adj) const { return m == 0 ? 0.0 : to_double(v, adj); }
+};
+
 // x as an integer, rounded: 61 mantissa bits shifted right by sh - e (not
 // negative); `flip` = 0x80000000 negates.
 __device__ __forceinline__ ll to_fixed(double x, int sh, int flip = 0) {
@@ -373,14 +421,6 @@ __device__ __forceinline__ ll to_fixed(double x, int sh, int flip = 0) {
   const ll v = (ll)(((m >> s) + 1) >> 1);
   return (h ^ flip) < 0 ? -v : v;
 }
-// an integer as a double times 2^(adj >> 20) (the result is normal or zero);
-// `flip` = 0x80000000 negates
-__device__ __forceinline__ double to_double(ll v, int adj, int flip = 0) {
-  const double d = __ll2double_rn(v);
-  const int h = __double2hiint(d);
-  return __hiloint2double((h != 0 ? h + adj : 0) ^ flip, __double2loint(d));
-}
-
 // The lines of a CTA that fixed point does not take, in FP64: as many lines
 // at a time as two buffers of the CTA's shared memory hold.
 template <int KIND, bool CONTIG>

@@ -1,6 +1,7 @@
 // Instantiations of the compile-time fixed-point passes (fft_fxc.cuh).  The
 // build compiles this file once for every part: a line kind, a layout and a
-// group of lengths (GBFFT_FXC_PART = group * 6 + kind * 2 + contiguous), and
+// group of lengths (GBFFT_FXC_PART = group * 8 + kind * 2 + contiguous, kind
+// 3 the real-to-real passes), and
 // once without, for the dispatch.
 #ifdef GBFFT_FXC_PART
 #include "fft_fxc.cuh"
@@ -10,12 +11,26 @@
 
 namespace gbfft {
 
-cudaError_t GBFFT_CAT(launch_fxc_part, GBFFT_FXC_PART)(const PassArgs& a, cudaStream_t s) {
-  constexpr int kGroup = GBFFT_FXC_PART / 6, kKind = GBFFT_FXC_PART % 6 / 2;
-  constexpr bool kContig = GBFFT_FXC_PART % 2 == 1;
-#define GBFFT_FXC_CASE(g, N, T, r0, r1, r2, r3)                                              \
-  if constexpr (g == kGroup)                                                                 \
-    if (a.n == N) return fx::launch_p<fx::Plan<N, T, r0, r1, r2, r3>, kKind, kContig>(a, s);
+namespace {
+constexpr int kGroup = GBFFT_FXC_PART / 8, kKind = GBFFT_FXC_PART % 8 / 2;
+constexpr bool kContig = GBFFT_FXC_PART % 2 == 1;
+#if GBFFT_FXC_PART % 8 / 2 == 3
+using Args = DttArgs;
+int length(const Args& a) { return a.M; }
+template <class P>
+cudaError_t launch(const Args& a, cudaStream_t s) { return fx::launch_r2r_p<P, kContig>(a, s); }
+#else
+using Args = PassArgs;
+int length(const Args& a) { return a.n; }
+template <class P>
+cudaError_t launch(const Args& a, cudaStream_t s) { return fx::launch_p<P, kKind, kContig>(a, s); }
+#endif
+}  // namespace
+
+cudaError_t GBFFT_CAT(launch_fxc_part, GBFFT_FXC_PART)(const Args& a, cudaStream_t s) {
+#define GBFFT_FXC_CASE(g, N, T, r0, r1, r2, r3)                                  \
+  if constexpr (g == kGroup)                                                     \
+    if (length(a) == N) return launch<fx::Plan<N, T, r0, r1, r2, r3>>(a, s);
   GBFFT_FXC_PLANS(GBFFT_FXC_CASE)
 #undef GBFFT_FXC_CASE
   return cudaErrorNotSupported;
@@ -27,22 +42,36 @@ cudaError_t GBFFT_CAT(launch_fxc_part, GBFFT_FXC_PART)(const PassArgs& a, cudaSt
 
 namespace gbfft {
 
+#define GBFFT_FXC_PARTS(X) X(0) X(1) X(2) X(3) X(4) X(5) X(8) X(9) X(10) X(11) X(12) X(13)
+#define GBFFT_FXC_R2R_PARTS(X) X(6) X(7) X(14) X(15)
 #define GBFFT_FXC_DECL(p) cudaError_t launch_fxc_part##p(const PassArgs& a, cudaStream_t s);
-#define GBFFT_FXC_PARTS(X) X(0) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11)
+#define GBFFT_FXC_R2R_DECL(p) cudaError_t launch_fxc_part##p(const DttArgs& a, cudaStream_t s);
 GBFFT_FXC_PARTS(GBFFT_FXC_DECL)
-
-cudaError_t launch_fxc(int kind, bool contiguous, const PassArgs& a, cudaStream_t s) {
-  int group = -1;
-#define GBFFT_FXC_GROUP(g, N, T, r0, r1, r2, r3) \
-  if (a.n == N) group = g;
-  GBFFT_FXC_PLANS(GBFFT_FXC_GROUP)
-#undef GBFFT_FXC_GROUP
-  if (group < 0) return cudaErrorNotSupported;
-  switch (group * 6 + kind * 2 + (contiguous ? 1 : 0)) {
+GBFFT_FXC_R2R_PARTS(GBFFT_FXC_R2R_DECL)
 #define GBFFT_FXC_CALL(p) \
   case p: return launch_fxc_part##p(a, s);
+
+namespace {
+int group_of(int n) {
+  int group = -1;
+#define GBFFT_FXC_GROUP(g, N, T, r0, r1, r2, r3) \
+  if (n == N) group = g;
+  GBFFT_FXC_PLANS(GBFFT_FXC_GROUP)
+#undef GBFFT_FXC_GROUP
+  return group;
+}
+}  // namespace
+
+cudaError_t launch_fxc(int kind, bool contiguous, const PassArgs& a, cudaStream_t s) {
+  switch (group_of(a.n) * 8 + kind * 2 + (contiguous ? 1 : 0)) {
     GBFFT_FXC_PARTS(GBFFT_FXC_CALL)
-#undef GBFFT_FXC_CALL
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+cudaError_t launch_fxc_r2r(bool contiguous, const DttArgs& a, cudaStream_t s) {
+  switch (group_of(a.M) * 8 + 6 + (contiguous ? 1 : 0)) {
+    GBFFT_FXC_R2R_PARTS(GBFFT_FXC_CALL)
     default: return cudaErrorInvalidValue;
   }
 }

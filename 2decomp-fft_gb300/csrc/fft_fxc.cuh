@@ -11,6 +11,7 @@
 #pragma once
 
 #include "fft_fx.cuh"
+#include "fft_r2r.cuh"
 
 namespace gbfft {
 namespace fx {
@@ -111,12 +112,12 @@ struct Io {
 #endif
 };
 
-template <class P, int S, bool FROM_SMEM, int KIND, bool CONTIG>
-__device__ __forceinline__ void run(const Io<KIND, CONTIG>& io, I2* Sm, const Slots<P, CONTIG>& slot, const W4* __restrict__ tw,
+// The stages from S on.  KIND K_R2C: the last one leaves its outputs in Sm.
+template <class P, int S, bool FROM_SMEM, int KIND, bool CONTIG, class Out>
+__device__ __forceinline__ void run(const Out& io, int t, I2* Sm, const Slots<P, CONTIG>& slot, const W4* __restrict__ tw,
                                     I2 (&v)[P::points()], int adj, int flip) {
   constexpr int R = P::radix(S), NS = P::ns(S), NB = P::N / R, MB = P::mb(S), TPL = P::TPL;
   constexpr bool LAST = S == P::NST - 1;
-  const int t = io.c.t;
   if constexpr (FROM_SMEM) {
 #pragma unroll
     for (int m = 0; m < MB; ++m) {
@@ -159,7 +160,7 @@ __device__ __forceinline__ void run(const Io<KIND, CONTIG>& io, I2* Sm, const Sl
       for (int r = 0; r < R; ++r) Sm[slot(base + r * NS)] = v[m * R + r];
     }
     __syncthreads();
-    if constexpr (!LAST) run<P, S + 1, true, KIND, CONTIG>(io, Sm, slot, tw, v, adj, flip);
+    if constexpr (!LAST) run<P, S + 1, true, KIND, CONTIG>(io, t, Sm, slot, tw, v, adj, flip);
   }
 }
 
@@ -214,35 +215,19 @@ __global__ void __launch_bounds__(fxc_max_threads(P::TPL), min_ctas<P>())
     }
   }
   // 2. the line's scale
-  int m = 0;
-#pragma unroll
-  for (int i = 0; i < Q; ++i) m = max(m, max_hi(x[i]));
-  atomicMax(&smax[c.line], m);
-  __syncthreads();
-  m = smax[c.line];
-  const int em = m >> 20;
-  float sum = 0;
-#pragma unroll
-  for (int i = 0; i < Q; ++i) sum += share(max_hi(x[i]), share_base(em));
-  atomicAdd(&ssum[c.line], share_units(sum, Q));
-  int bad = m != 0 && (em < kMinExp || em > kMaxExp);
-  if (m == 0) {  // all zero, or subnormals below 2^-1042
-#pragma unroll
-    for (int i = 0; i < Q; ++i) bad |= any_lo(x[i]);
-  }
-  if (__syncthreads_or(bad)) {
+  Scale sc;
+  if (!sc.find<Q>(x, &smax[c.line], &ssum[c.line])) {
     fallback<KIND, CONTIG>(a, reinterpret_cast<double2*>(smem_raw));
     return;
   }
-  const unsigned s15 = ssum[c.line];
   constexpr int X = KIND == K_C2R ? 1 : 0;  // a point combines two values
-  const int es = 32 - __clz((int)(s15 + (s15 >> 1))) - 1040 + X;
   int top = -1021 + X;
 #pragma unroll
-  for (int s = 0; s < P::NST; ++s) top = max(top, min(es, P::lg(s) - 1021 + X) - P::shift(s));
+  for (int s = 0; s < P::NST; ++s) top = max(top, sc.bound(P::lg(s), X) - P::shift(s));
+  // r2c adds two values that no twiddle has halved
   if (KIND == K_R2C && P::NST == 1) ++top;
-  const int sh = m == 0 ? 4096 : 1021 + top + em;  // a zero line shifts all out
-  int adj = (em - 62 + top + P::shift(P::NST - 1)) << 20;
+  const int sh = sc.shift(top);
+  int adj = (sc.em - 62 + top + P::shift(P::NST - 1)) << 20;
   // backward c2c: conjugated on the way in and out (c2r: out)
   const int flip_in = KIND == K_C2C && c.inverse ? (int)0x80000000 : 0;
   // 3. integers, and the stages
@@ -264,7 +249,7 @@ __global__ void __launch_bounds__(fxc_max_threads(P::TPL), min_ctas<P>())
 #pragma unroll
     for (int i = 0; i < Q; ++i) v[i] = mk(to_fixed(x[i].x, sh), to_fixed(x[i].y, sh, flip_in));
   }
-  run<P, 0, KIND == K_C2R, KIND, CONTIG>(io, Sm, slot, tw, v, adj, KIND == K_C2R ? (int)0x80000000 : flip_in);
+  run<P, 0, KIND == K_C2R, KIND, CONTIG>(io, t, Sm, slot, tw, v, adj, KIND == K_C2R ? (int)0x80000000 : flip_in);
   if constexpr (KIND == K_R2C) {
     adj -= 1 << 20;  // the halves of X1 = (Z_k + conj Z_{n-k}) / 2, X2 = (Z_k - conj Z_{n-k}) / 2i
     constexpr int K = (H + TPL - 1) / TPL;
@@ -278,6 +263,87 @@ __global__ void __launch_bounds__(fxc_max_threads(P::TPL), min_ctas<P>())
       }
     }
   }
+}
+
+// A real-to-real pass (fft_r2r.cuh) around a compile-time plan of its FFT.
+template <class P, bool CONTIG>
+__global__ void __launch_bounds__(fxc_max_threads(P::TPL), min_ctas<P>())
+    fxc_r2r_kernel(const __grid_constant__ DttArgs a, const W4* __restrict__ tw) {
+  constexpr int N = P::N, TPL = P::TPL, Q = (N + TPL - 1) / TPL;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  chained_entry();
+  const int t = CONTIG ? threadIdx.x : threadIdx.y, line = CONTIG ? threadIdx.y : threadIdx.x, L = a.L;
+  const r2r::Lines<double, CONTIG> ln(a, (long long)blockIdx.x * L + line, CONTIG ? 0 : (long long)blockIdx.y);
+  I2* Sm = reinterpret_cast<I2*>(smem_raw);
+  Slots<P, CONTIG> slot;
+  slot.base = CONTIG ? line * Slots<P, CONTIG>::kLine : line;
+  slot.L = L;
+  int* smax = reinterpret_cast<int*>(smem_raw + fxc_smem_bytes(N, L) - (size_t)L * 16);
+  unsigned* ssum = reinterpret_cast<unsigned*>(smax + 2 * L);
+  for (int i = threadIdx.x + threadIdx.y * blockDim.x; i < 4 * L; i += blockDim.x * blockDim.y) smax[i] = 0;
+  __syncthreads();
+  const int cnt = r2r::elements(a.kind, a.n);
+  double2 x[Q];
+#pragma unroll
+  for (int i = 0; i < Q; ++i) {
+    const int j = t + i * TPL;
+    x[i] = j < cnt ? ln.element(j) : make_double2(0, 0);
+  }
+  r2r::PairScale sc;
+  if (!sc.find<Q>(x, &smax[2 * line], &ssum[2 * line], ln.single)) {
+    r2r::fallback<CONTIG>(a, reinterpret_cast<double2*>(smem_raw));
+    return;
+  }
+  using Map = r2r::Maps<r2r::Fixed, Slots<P, CONTIG>>;
+  const Map mp{a.kind, a.n, N, reinterpret_cast<const W4*>(a.w_fx), slot};
+  const int g = mp.grow(), pre = mp.pre();
+  int ta = -1021 + g, tb = ta;
+#pragma unroll
+  for (int s = 0; s < P::NST; ++s) {
+    const int down = pre + P::shift(s) - (s == P::NST - 1 ? mp.post() : 0);
+    ta = max(ta, sc.a.bound(P::lg(s), g) - down);
+    tb = max(tb, sc.b.bound(P::lg(s), g) - down);
+  }
+  const int sa = sc.a.shift(ta), sb = sc.b.shift(tb);
+  const int down = pre + P::shift(P::NST - 1) + mp.tail() + Map::doubled(a.kind, a.n) - 62;
+  const int adj_a = (sc.a.em + ta + down) << 20, adj_b = (sc.b.em + tb + down) << 20;
+#pragma unroll
+  for (int i = 0; i < Q; ++i) {
+    const int j = t + i * TPL;
+    if (j < cnt) mp.place(Sm, j, mk(to_fixed(x[i].x, sa), to_fixed(x[i].y, sb)));
+  }
+  __syncthreads();
+  if (mp.combines()) {
+#pragma unroll 1
+    for (int k = t; 2 * k <= a.n; k += TPL) mp.combine(Sm, k);
+    __syncthreads();
+  }
+  I2 v[P::points()];
+  run<P, 0, true, K_R2C, CONTIG>(ln, t, Sm, slot, tw, v, 0, 0);
+#pragma unroll 1
+  for (int k = t; k < mp.steps(); k += TPL)
+    mp.finish(
+        Sm, k, [&](int i, ll ya, ll yb) { ln.store(i, sc.a.out(ya, adj_a), sc.b.out(yb, adj_b)); },
+        [&](int i, ll y) { ln.store1(i, sc.a.out(y, adj_a)); });
+  ln.pass_through(a.naxis, t, TPL);
+}
+
+template <class P, bool CONTIG>
+cudaError_t launch_r2r_p(const DttArgs& a, cudaStream_t stream) {
+  const size_t smem = fxc_smem_bytes(P::N, a.L);
+  if (a.tpl != P::TPL || a.L < 1 || a.L * a.tpl > fxc_max_threads(P::TPL) || smem > kFxMaxSmem)
+    return cudaErrorInvalidValue;
+  auto kern = fxc_r2r_kernel<P, CONTIG>;
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  const long long lines = dtt_complex_lines(a);
+  const dim3 block = CONTIG ? dim3(a.tpl, a.L) : dim3(a.L, a.tpl);
+  const dim3 grid((unsigned)((lines + a.L - 1) / a.L), CONTIG ? 1u : (unsigned)a.nv);
+  const cudaError_t err = launch_chained(kern, grid, block, smem, stream, a, reinterpret_cast<const W4*>(a.fx->tw));
+  add_launches(1);
+  return err != cudaSuccess ? err : cudaGetLastError();
 }
 
 template <class P, int KIND, bool CONTIG>

@@ -63,25 +63,15 @@ __device__ void stage_pp_generic(const Ctx& c, const Cx<T>* A, Cx<T>* B, int R, 
   }
 }
 
-// The runtime-planned pass of a CTA's lines (e points in all): loaded into
-// shared buffer 0, each stage ping-pongs between the two buffers, the result
-// is stored from the last buffer written.
-template <typename T, int KIND, bool CONTIG>
-__device__ __forceinline__ void run_pp_lines(const LineCtx<T, KIND, CONTIG>& c, const PassArgs& a, Cx<T>* buf0,
-                                             size_t e) {
+// The radix stages of the lines in shared buffer A, ping-ponging with B; A is
+// the last buffer written when it returns.
+template <typename T, int KIND, bool CONTIG, class Ctx>
+__device__ __forceinline__ void run_stages_pp(const Ctx& c, int nst, const int* radix, Cx<T>*& A, Cx<T>*& B) {
   using C = Cx<T>;
-  C* buf1 = buf0 + (e + (e >> 4) + 1);
-
-#pragma unroll 1
-  for (int n = c.t; n < c.N; n += c.tpl) buf0[c.sidx(n)] = c.gload(n);
-  __syncthreads();
-
-  C* A = buf0;
-  C* B = buf1;
   int Ns = 1;
 #pragma unroll 1
-  for (int s = 0; s < a.nst; ++s) {
-    const int R = a.radix[s];
+  for (int s = 0; s < nst; ++s) {
+    const int R = radix[s];
     if (R == 16) stage_pp<T, KIND, CONTIG, 16>(c, A, B, Ns);
     else if (R == 8) stage_pp<T, KIND, CONTIG, 8>(c, A, B, Ns);
     else if (R == 4) stage_pp<T, KIND, CONTIG, 4>(c, A, B, Ns);
@@ -109,6 +99,24 @@ __device__ __forceinline__ void run_pp_lines(const LineCtx<T, KIND, CONTIG>& c, 
     B = tmp;
     Ns *= R;
   }
+}
+
+// The runtime-planned pass of a CTA's lines (e points in all): loaded into
+// shared buffer 0, each stage ping-pongs between the two buffers, the result
+// is stored from the last buffer written.
+template <typename T, int KIND, bool CONTIG>
+__device__ __forceinline__ void run_pp_lines(const LineCtx<T, KIND, CONTIG>& c, const PassArgs& a, Cx<T>* buf0,
+                                             size_t e) {
+  using C = Cx<T>;
+  C* buf1 = buf0 + (e + (e >> 4) + 1);
+
+#pragma unroll 1
+  for (int n = c.t; n < c.N; n += c.tpl) buf0[c.sidx(n)] = c.gload(n);
+  __syncthreads();
+
+  C* A = buf0;
+  C* B = buf1;
+  run_stages_pp<T, KIND, CONTIG>(c, a.nst, a.radix, A, B);
 
   if (KIND == K_R2C) {
     c.store_r2c(A);

@@ -82,16 +82,16 @@ constexpr int kFxPoints = 8;        // points a thread loads at most
 constexpr int kFxMaxThreads = 512;  // threads of a CTA
 constexpr size_t kFxMaxSmem = 200 * 1024;
 // Shared memory of L lines of n points: two padded buffers and the lines'
-// scale words.
+// scale words (two a line, four for two real lines).
 __host__ __device__ constexpr size_t fx_smem_bytes(int n, int L) {
   const size_t e = (size_t)n * (size_t)L;
-  return 2 * (e + (e >> 4) + 1) * 16 + (size_t)L * 8;
+  return 2 * (e + (e >> 4) + 1) * 16 + (size_t)L * 16;
 }
 // ... and of the compile-time plans (fft_fxc.cuh): one buffer, padded by an
 // entry in eight; a single line keeps room for the two of its FP64 fallback.
 __host__ __device__ constexpr size_t fxc_smem_bytes(int n, int L) {
   const size_t one = ((size_t)n + n / 8 + 2) * (size_t)L;
-  return (L == 1 ? 2 * one : one) * 16 + 32 + (size_t)L * 8;
+  return (L == 1 ? 2 * one : one) * 16 + 32 + (size_t)L * 16;
 }
 // Lengths with a compile-time plan (fft_fxc.cuh): X(group, n, threads a line,
 // radices).  The radices stay at most 10 (64 registers a thread, four CTAs
@@ -345,38 +345,56 @@ int engine_passes(struct ::gbfft_engine_s* e, int which, const void* in, void* o
 // (two padded buffers); the power-of-two pass needs half of it.
 size_t pass_smem_bytes(int prec_bytes, int n, int L);
 
-// One real-to-real pass along an axis (dtt.cu): the window of n points
-// starting at point `off` of every line is transformed by kind 1..8
-// (DCT-I..IV, DST-I..IV) through a complex FFT of length M.
+// One real-to-real pass along an axis: the window of n points starting at
+// point `off` of every line is transformed by kind 1..8 (DCT-I..IV,
+// DST-I..IV) through a complex FFT of length M -- of one line's extension
+// (dtt.cu), or in fixed point of dtt_fft_length points that carry two real
+// lines (one for DCT-IV / DST-IV of an even n; fft_r2r.cuh).
 struct DttArgs {
   const void* src;   // real array the window is read from
   void* dst;         // real array it is written to (may be src)
   long long sn;      // element stride between points of a line
   long long sl;      // contiguous: line stride; strided: stride of v
-  long long nlines;  // contiguous: lines; strided: extent of u (x positions)
+  long long nlines;  // real lines: contiguous all, strided along u (x positions)
   int nv;            // strided: extent of v (grid.y)
   int naxis;         // points on the axis (copied through outside the window)
   int off, n;        // window: first point, length
   int kind;          // 1..8
-  int M;             // FFT length of the extension
+  int M;             // FFT length
   int nst;           // radix stages of M
   int radix[kMaxStages];
   const void* tw;    // exp(-2 pi i m / M), m < M
-  const void* twf;   // power-of-two M: stage-major table of the 16-point plan,
-                     // which runs instead of the runtime plan (null: runtime plan)
+  const void* twf;   // FP32, power-of-two or two-stage M: stage-major table of the
+                     // compile-time plan, which runs instead of the runtime plan
+                     // (null: runtime plan)
   const void* w4;    // exp(-2 pi i m / (4 n)), m < n
   double c0x, c0y;   // exp(-i pi / (4 n))
-  int L, tpl;        // lines a CTA, threads a line
+  const FxPlan* fx;  // FP64: host-side plan of the fixed-point pass, or null; then
+  const void* w;     //   the roots of the maps around the FFT, in double
+  const void* w_fx;  //   and in Q62
+  int pair_vec;      //   strided: the two real lines of a pair are adjacent and
+                     //   aligned in both arrays (one access for both)
+  int L, tpl;        // transforms a CTA (lines; fixed point: complex lines), threads each
 };
+// FFT length behind kind 1..8 of an n-point window in fixed point.
+__host__ __device__ constexpr int dtt_fft_length(int kind, int n) {
+  return kind == 1 ? 2 * (n - 1) : kind == 5 ? 2 * (n + 1) : kind % 4 == 0 && n % 2 == 0 ? n / 2 : n;
+}
+// Complex lines of a pass: pairs of its real lines, or each alone.
+inline long long dtt_complex_lines(const DttArgs& a) {
+  return a.kind % 4 == 0 && a.n % 2 == 0 ? a.nlines : (a.nlines + 1) / 2;
+}
 size_t dtt_smem_bytes(int prec_bytes, int M, int L);
-// power-of-two extension lengths with a compile-time plan for the r2r pass
+// power-of-two extension lengths with a compile-time plan for the FP32 r2r pass
 __host__ __device__ constexpr bool dtt_fast_length(int M) { return M >= 32 && M <= 2048 && (M & (M - 1)) == 0; }
 // Extension lengths with the compile-time two-stage plan M = R0 * R1
 // (mixed_r0): 126 = 9 * 14 and 510 = 17 * 30, the default windows of every
-// kind on axes of 64 and 256 points (FP32; the engine keeps FP64 on the
-// runtime plan).
+// kind on axes of 64 and 256 points (FP32).
 __host__ __device__ constexpr bool dtt_mixed_length(int M) { return M == 126 || M == 510; }
 cudaError_t launch_dtt_pass(int prec_bytes, bool contiguous, const DttArgs& a, cudaStream_t stream);
+// ... its fixed-point forms (a.fx), runtime and compile-time plans
+cudaError_t launch_fx_r2r(bool contiguous, const DttArgs& a, cudaStream_t stream);
+cudaError_t launch_fxc_r2r(bool contiguous, const DttArgs& a, cudaStream_t stream);
 
 // TMA-staged strided c2c passes (fft_tma.cu): FP32 lines of 1024 points
 // whose source and destination rows and planes lie multiples of 16 bytes

@@ -141,3 +141,72 @@ def test_scaling_by_a_power_of_two_is_exact():
         e.c2c(x, y, -1)
         out.append(y * 2.0 ** -k)
     assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])
+
+
+# ---- real-to-real passes ---------------------------------------------------
+def r2r_matrix(kind, n):
+    """FFTW's definition of kind 1..8 at n points, in long double."""
+    j, k = np.arange(n, dtype=np.int64)[None], np.arange(n, dtype=np.int64)[:, None]
+    num, den = {1: (j * k, n - 1), 2: ((2 * j + 1) * k, 2 * n), 3: (j * (2 * k + 1), 2 * n),
+                4: ((2 * j + 1) * (2 * k + 1), 4 * n), 5: ((j + 1) * (k + 1), n + 1), 6: ((2 * j + 1) * (k + 1), 2 * n),
+                7: ((j + 1) * (2 * k + 1), 2 * n), 8: ((2 * j + 1) * (2 * k + 1), 4 * n)}[kind]
+    pi = np.longdouble("3.14159265358979323846264338327950288")
+    a = pi * (num % (2 * den)).astype(np.longdouble) / np.longdouble(den)
+    m = 2 * (np.cos(a) if kind <= 4 else np.sin(a))
+    if kind in (1, 3):
+        m[:, 0] /= 2
+    if kind in (1, 7):
+        m[:, -1] /= 2
+    return m
+
+
+def r2r(lines, kind, axis, pad=0):
+    """`lines` (rows) through a pass of `kind` along x or y; the window starts
+    `pad` points in."""
+    import gbfft
+    a = np.pad(lines, ((0, 0), (pad, pad)), constant_values=7.0)
+    x = torch.from_numpy(np.ascontiguousarray(a[None] if axis == 0 else a.T[None])).cuda()
+    y = torch.empty_like(x)
+    cfg = [kind if axis == 0 else 2, kind if axis == 1 else 2, 2]
+    first, gone = [1, 1, 1], [0, 0, 0]
+    first[axis], gone[axis] = pad + 1, 2 * pad
+    d = gbfft.Dtt(1, x.shape[2], x.shape[1], 1, cfg + first + gone + first, skip=(axis != 0, axis != 1, True))
+    d.r2r(x, y, -1)
+    got = y.cpu().numpy()[0]
+    got = got if axis == 0 else got.T
+    assert (got[:, :pad] == 7).all() and (got[:, got.shape[1] - pad:] == 7).all()
+    return got[:, pad:got.shape[1] - pad]
+
+
+@pytest.mark.parametrize("axis", [0, 1])
+@pytest.mark.parametrize("kind", range(1, 9))
+@pytest.mark.parametrize("n", [2, 3, 4, 5, 9, 16, 17, 32, 33, 96, 127, 129, 255, 256, 400, 512])
+def test_r2r_lengths_against_long_double(n, kind, axis):
+    rng = np.random.default_rng(n + kind)
+    m = r2r_matrix(kind, n)
+    for lines, pad in ((7, 0), (8, 2)):  # an odd and an even number of real lines
+        a = rng.standard_normal((lines, n))
+        assert rel(r2r(a, kind, axis, pad), a.astype(np.longdouble) @ m.T) <= TOL
+
+
+@pytest.mark.parametrize("axis", [0, 1])
+@pytest.mark.parametrize("kind", range(1, 9))
+@pytest.mark.parametrize("n", [12, 16, 17])
+def test_r2r_lines_are_independent(n, kind, axis):
+    """The two real lines of a pair share a complex transform: their scales
+    and their non-finite values stay apart."""
+    rng = np.random.default_rng(n + kind)
+    m = r2r_matrix(kind, n)
+    a = rng.standard_normal((8, n)) * 2.0 ** np.array([0, -200, 0, 300, -300, 0, 0, 50])[:, None]
+    a[5] = 0
+    got, ref = r2r(a, kind, axis), a.astype(np.longdouble) @ m.T
+    for i in range(8):
+        assert not got[i].any() if i == 5 else rel(got[i], ref[i]) <= 2 * TOL, i
+    a[2, n // 2] = np.nan
+    a[7, 0] = np.inf
+    got = r2r(a, kind, axis)
+    for i in range(8):
+        if i in (2, 7):
+            assert not np.isfinite(got[i]).all()
+        elif i != 5:
+            assert rel(got[i], ref[i]) <= 5e-15, i
