@@ -316,108 +316,129 @@ int upload_batch_table(AxisPlan& p, int prec) {
   return upload_table(&p.d_twfb, stage_twiddles(plan_radices(q)), prec);
 }
 
-// Radices of the fixed-point kernel's compile-time butterflies.
-constexpr int kFxRadices[] = {2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 13, 17};
-// Relative cost of a point in a stage of radix r, beside its exchange and
-// twiddle (kFxStageCost).
-constexpr double kFxStageCost = 24;
-double fx_radix_cost(int r) {
-  switch (r) {
-    case 2: return 2;
-    case 3: return 6;
-    case 4: return 4;
-    case 5: return 9;
-    case 6: return 9;
-    case 7: return 22;
-    case 8: return 9;
-    case 9: return 18;
-    case 10: return 13;
-    case 11: return 38;
-    case 13: return 46;
-    case 17: return 64;
-    default: return 26.0 * r;  // direct sum
-  }
+// ---- plans of the fixed-point and the smooth-length kernels --------------
+// Relative cost of a point in a stage of radix r beside its exchange and
+// twiddle (kStageCost), on the integer and the FP32 pipes; 0: no compile-time
+// butterfly.
+constexpr double kStageCost[2] = {24, 14};
+double radix_cost(bool fixed, int r) {
+  static const double x[] = {2, 6, 4, 9, 8, 22, 9, 18, 11, 38, 0, 46, 0, 0, 0, 64};  // 2..17
+  static const double f[] = {2, 4, 4, 7, 6, 12, 8, 12, 9, 24, 8, 28, 14, 11, 13, 0};
+  return r < 2 || r > 17 ? 0 : (fixed ? x : f)[r - 2];
 }
-// Cheapest split of n into radices of at most rmax (primes beyond the
-// compile-time ones excepted, which any split carries).
-void fx_split(int n, int last, int rmax, double cost, std::vector<int>& cur, double& best, std::vector<int>& out) {
-  if (cost >= best) return;
-  if (n == 1) {
-    best = cost;
-    out = cur;
-    return;
-  }
-  bool any = false;
-  for (int i = (int)(sizeof(kFxRadices) / sizeof(int)) - 1; i >= 0; --i) {
-    const int r = kFxRadices[i];
-    if (n % r || r > last || (r > rmax && r <= 10)) continue;
-    any = true;
-    cur.push_back(r);
-    fx_split(n / r, r, rmax, cost + kFxStageCost + fx_radix_cost(r), cur, best, out);
+// Cheapest split of n into radices of at most `last`, composite ones of at
+// most rmax; false when a prime factor has no butterfly and `direct` (a
+// direct-sum stage for it) is not allowed.
+struct Splitter {
+  bool fixed, direct;
+  int rmax;
+  std::vector<int> cur, out;
+  double best = 1e30;
+  void go(int n, int last, double cost) {
+    if (cost >= best) return;
+    if (n == 1) {
+      best = cost;
+      out = cur;
+      return;
+    }
+    bool any = false;
+    for (int r = std::min(last, 17); r >= 2; --r) {
+      const double c = radix_cost(fixed, r);
+      const bool prime = r == 2 || r == 3 || r == 5 || r == 7 || r == 11 || r == 13 || r == 17;
+      if (n % r || c == 0 || (r > rmax && !prime)) continue;
+      any = true;
+      cur.push_back(r);
+      go(n / r, r, cost + kStageCost[fixed ? 0 : 1] + c);
+      cur.pop_back();
+    }
+    if (any || !direct) return;
+    int q = 2;  // smallest prime factor
+    while (n % q) ++q;
+    cur.push_back(q);
+    go(n / q, last, cost + kStageCost[fixed ? 0 : 1] + 26.0 * q);
     cur.pop_back();
   }
-  if (any) return;
-  int q = 2;  // smallest prime factor, a direct-sum stage
-  while (n % q) ++q;
-  cur.push_back(q);
-  fx_split(n / q, last, rmax, cost + kFxStageCost + fx_radix_cost(q), cur, best, out);
-  cur.pop_back();
-}
-bool fx_special(int r) {
-  for (int v : kFxRadices)
-    if (v == r) return true;
-  return r == 16;  // the compile-time plans'
-}
-// The fixed-point plan of an axis of n points; rmax bounds the radix (small
-// grids take radix 4: twice the threads a line).  ct: a compile-time plan may
-// run (those address rows below 4 GB apart).
-FxPlan fx_plan(int n, int rmax, bool ct) {
-  std::vector<int> cur, rad;
-  double best = 1e30;
-  const FxcShape shape = ct ? fxc_shape(n) : FxcShape{0, {0, 0, 0, 0}};
-  if (shape.tpl)
-    for (int r : shape.r) {
-      if (r > 1) rad.push_back(r);
-    }
-  else
-    fx_split(n, 1 << 30, rmax, 0, cur, best, rad);
-  FxPlan p;
+};
+bool fx_special(int r) { return radix_cost(true, r) > 0 || r == 16; }  // 16: compile-time plans
+// Fill a plan's stages from its radices.
+void set_stages(FxPlan& p, const std::vector<int>& rad, bool fixed) {
   std::memset(&p, 0, sizeof p);
   p.nst = (int)rad.size();
-  p.ct = shape.tpl > 0;
   int ns = 1, shift = 0;
   for (int s = 0; s < p.nst; ++s) {
     const int r = rad[s];
     p.radix[s] = r;
     p.ns[s] = ns;
     p.magic[s] = ns > 1 ? (unsigned)(((1ull << 32) + ns - 1) / ns) : 0;
-    if (ns > 1) shift += shape.tpl && p.radix[s - 1] >= 16 ? 2 : 1;
-    else if (!fx_special(r)) shift += 1;
+    if (fixed && (ns > 1 || !fx_special(r))) shift += 1;
     ns *= r;
     int lg = 0;
     while ((1 << lg) < ns) ++lg;
     p.lg[s] = lg;
     p.shift[s] = shift;
   }
-  if (shape.tpl) {
-    p.tpl = shape.tpl;
-    return p;
-  }
-  // threads a line: at least n / kFxPoints, the count whose stages leave the
-  // fewest threads idle
-  const int lo = (n + kFxPoints - 1) / kFxPoints, hi = std::min(kFxMaxThreads, std::max(lo, (n + rmax - 1) / rmax * 5 / 4));
+}
+// Threads a line, from lo to hi, whose stages leave the fewest threads idle.
+int best_threads(const FxPlan& p, int n, bool fixed, int lo, int hi) {
+  int best = lo;
   double bestw = 1e30;
   for (int t = lo; t <= hi; ++t) {
     double w = 0;
     for (int s = 0; s < p.nst; ++s) {
       const int nb = n / p.radix[s];
-      w += (kFxStageCost + fx_radix_cost(p.radix[s])) * (double)((nb + t - 1) / t) * t / nb;
+      const double c = radix_cost(fixed, p.radix[s]);
+      w += (kStageCost[fixed ? 0 : 1] + (c > 0 ? c : 26.0 * p.radix[s])) * (double)((nb + t - 1) / t) * t / nb;
     }
     if (w < bestw * 0.999) {
       bestw = w;
-      p.tpl = t;
+      best = t;
     }
   }
+  return best;
+}
+// The smooth-length plan of n points (fft_rt.cuh): at least two stages, all
+// of them with a butterfly, the first one butterfly a thread; nst 0: none.
+FxPlan rt_plan(int n, int rmax, bool fixed) {
+  FxPlan p;
+  std::memset(&p, 0, sizeof p);
+  const int cap = rt_max_radix(fixed ? 8 : 4);
+  Splitter sp{fixed, false, std::min(rmax, cap), {}, {}};
+  sp.go(n, cap, 0);
+  if (sp.out.size() < 2) return p;
+  set_stages(p, sp.out, fixed);
+  const int lo = n / p.radix[0], maxt = rt_threads(fixed ? 8 : 4);
+  if (lo > maxt) {
+    p.nst = 0;
+    return p;
+  }
+  p.tpl = best_threads(p, n, fixed, lo, std::min(maxt, lo * 3 / 2));
+  p.rt = 1;
+  return p;
+}
+// The fixed-point plan of an axis of n points; rmax bounds the radix (small
+// grids take radix 4: twice the threads a line).  near: rows lie below 2^28
+// elements apart, as the compile-time and smooth-length kernels address them.
+FxPlan fx_plan(int n, int rmax, bool near) {
+  FxPlan p;
+  const FxcShape shape = near ? fxc_shape(n) : FxcShape{0, {0, 0, 0, 0}};
+  if (shape.tpl) {
+    std::vector<int> rad;
+    for (int r : shape.r)
+      if (r > 1) rad.push_back(r);
+    set_stages(p, rad, true);
+    p.ct = 1;
+    p.tpl = shape.tpl;
+    return p;
+  }
+  if (near) {
+    p = rt_plan(n, rmax, true);
+    if (p.nst) return p;
+  }
+  Splitter sp{true, true, rmax, {}, {}};
+  sp.go(n, 1 << 30, 0);
+  set_stages(p, sp.out, true);
+  const int lo = (n + kFxPoints - 1) / kFxPoints;
+  p.tpl = best_threads(p, n, true, lo, std::min(kFxMaxThreads, std::max(lo, (n + rmax - 1) / rmax * 5 / 4)));
   return p;
 }
 
@@ -500,7 +521,19 @@ int upload_fx(AxisPlan& p) {
 }
 
 int upload_twiddles(AxisPlan& p, int prec) {
-  if (p.fx.nst) return upload_fx(p);
+  if (p.fx.nst && prec == GBFFT_PREC_DOUBLE) return upload_fx(p);
+  if (p.fx.nst) {  // FP32, smooth length: its kernel reads the stage-major table alone
+    const std::vector<double> t = stage_twiddles(std::vector<int>(p.fx.radix, p.fx.radix + p.fx.nst));
+    std::vector<double> parts(2 * t.size());  // high parts (rounded to FP32), then what they leave
+    for (size_t i = 0; i < t.size(); ++i) {
+      const double high = (double)(float)t[i];
+      parts[i / 2 * 4 + i % 2] = high;
+      parts[i / 2 * 4 + 2 + i % 2] = t[i] - high;
+    }
+    const int rc = upload_table(&p.d_fxtw, parts, prec);
+    p.fx.tw = p.d_fxtw;
+    return rc;
+  }
   int rc = upload_table(&p.d_tw, twiddles(p.n), prec);
   const std::vector<int> radices = plan_radices(p);
   if (rc == GBFFT_OK && !radices.empty()) rc = upload_table(&p.d_twf, stage_twiddles(radices), prec);
@@ -716,7 +749,7 @@ int lines_per_cta(const AxisPlan& p, int prec, bool contiguous, long long nlines
   if (L > 1 && nlines < L) {
     int l2 = 1;
     while (l2 < nlines) l2 *= 2;
-    L = l2;
+    L = std::min(L, l2);
   }
   return L < 1 ? 1 : L;
 }
@@ -797,20 +830,21 @@ int gen_lines_per_cta(int n, int prec, bool contiguous, long long nlines, int fo
   return L;
 }
 
-// Lines per CTA of the fixed-point kernels: strided tiles about 256 threads
-// and at least 64-byte row segments (4 lines); contiguous lines about 128
-// threads (512 x 512 x 256 x pass 336 us, with 256 threads 349).
-int fx_lines_per_cta(const FxPlan& f, int n, bool contiguous, long long nlines, long long nv, int forced_L) {
-  const bool ct = f.ct != 0;
-  const int maxt = ct ? fxc_max_threads(f.tpl) : kFxMaxThreads;
-  auto smem = [&](int l) { return ct ? fxc_smem_bytes(n, l) : fx_smem_bytes(n, l); };
+// Lines per CTA of the fixed-point and smooth-length kernels: strided tiles
+// about 256 threads and at least 64-byte row segments; contiguous lines about
+// 128 threads (512 x 512 x 256 FP64 x pass 336 us, with 256 threads 349).
+int fx_lines_per_cta(const FxPlan& f, int n, int prec, bool contiguous, long long nlines, long long nv, int forced_L) {
+  const int maxt = f.ct ? fxc_max_threads(f.tpl) : f.rt ? rt_threads(prec) : kFxMaxThreads;
+  auto smem = [&](int l) {
+    return f.ct ? fxc_smem_bytes(n, l) : f.rt ? rt_smem_bytes(prec, n, l, f.nst) : fx_smem_bytes(n, l);
+  };
   if (forced_L > 0 && forced_L * f.tpl <= maxt && smem(forced_L) <= kFxMaxSmem) return forced_L;
-  const int min_l = contiguous ? 1 : 4;
+  const int seg = 64 / (2 * prec), min_l = contiguous ? 1 : seg;
   int L = (contiguous ? 128 : 256) / f.tpl;
-  if (!contiguous && L > 4) L = L / 4 * 4;
+  if (!contiguous && L > seg) L = L / seg * seg;
   if (L > 32) L = 32;
   if (L < min_l) L = min_l;
-  while (L > min_l && smem(L) > 72 * 1024) L = contiguous ? L - 1 : L - 4;
+  while (L > min_l && smem(L) > 72 * 1024) L = contiguous ? L - 1 : L - seg;
   while (L > min_l && ((nlines + L - 1) / L) * nv < 2LL * kSmsDefault) L = std::max(min_l, L / 2);
   while (L > 1 && (L * f.tpl > maxt || smem(L) > kFxMaxSmem)) --L;
   if (L > 1 && nlines < L) L = (int)nlines;
@@ -826,9 +860,9 @@ void fill_plan(PassArgs& a, const AxisPlan& p, int prec, bool contiguous, int ki
     for (int i = 0; i < kMaxStages; ++i) a.radix[i] = i < p.nst ? p.radix[i] : 0;
     a.tw = p.d_tw;
     a.fx = &p.fx;
-    a.fast = p.fx.ct ? 7 : 6;
+    a.fast = p.fx.ct ? 7 : p.fx.rt ? 8 : 6;
     a.tpl = p.fx.tpl;
-    a.L = fx_lines_per_cta(p.fx, p.n, contiguous, a.nlines, contiguous ? 1 : a.nv, forced_L);
+    a.L = fx_lines_per_cta(p.fx, p.n, prec, contiguous, a.nlines, contiguous ? 1 : a.nv, forced_L);
     return;
   }
   if (split && split_length(p.n)) {
@@ -1245,6 +1279,10 @@ int engine_init_host(gbfft_engine_s* e, int format, int nx, int ny, int nz, int 
       e->ax[d].fx = fx_plan(lens[d], threads < 512.0 * kSmsDefault ? 4 : 10,
                            (double)(nx + 8) * ny < (double)(1 << 28));
     }
+    // FP32 lengths without a compile-time plan: the smooth-length kernel
+    if (prec == GBFFT_PREC_SINGLE && !e->ax[d].big && !fast_length(lens[d]) && !mixed_length(lens[d]) &&
+        !gen_length(lens[d]) && (double)(nx + 8) * ny < (double)(1 << 28))
+      e->ax[d].fx = rt_plan(lens[d], (double)nx * ny * nz / 16 < 512.0 * kSmsDefault ? 10 : 16, false);
     if (form != GBFFT_FORM_PLAIN && split_length(lens[d])) e->ax[d].fast_e = 16;  // radix-16 stages for the tensor cores
   }
   *tune_out = tune;
@@ -2025,7 +2063,7 @@ int setup_dtt_axis(DttAxis& a, int kind, int first, int ndismiss, int naxis, int
     if (rc == GBFFT_OK) rc = upload_ints(&a.w_fx, q62_table(w));
     if (rc != GBFFT_OK) return rc;
     // small grids (two real lines a complex one): radix 4, as the axis passes
-    a.plan.fx = fx_plan(a.M, cells / 2 / kFxPoints < 512.0 * kSmsDefault ? 4 : 10, true);
+    a.plan.fx = fx_plan(a.M, cells / 2 / kFxPoints < 512.0 * kSmsDefault ? 4 : 10, fxc_shape(a.M).tpl > 0);
     return upload_fx(a.plan);
   }
   a.M = ext;
@@ -2181,11 +2219,13 @@ int gbfft_exec_r2r(gbfft_dtt_t d, void* d_in, void* d_out, int isign, void* stre
       a.pair_vec = !contiguous && nx % 2 == 0 && ((uintptr_t)src | (uintptr_t)dst) % (2 * (size_t)d->prec) == 0;
       const long long lines = dtt_complex_lines(a);
       a.tpl = a.fx->tpl;
-      a.L = fx_lines_per_cta(*a.fx, a.M, contiguous, lines, a.nv, 0);
+      a.L = fx_lines_per_cta(*a.fx, a.M, d->prec, contiguous, lines, a.nv, 0);
       // one real line each: twice as many for the same row segments
       const int maxt = a.fx->ct ? fxc_max_threads(a.tpl) : kFxMaxThreads;
       if (a.kind % 4 == 0 && a.n % 2 == 0 && !contiguous)
-        while (2 * a.L <= 16 && 2 * a.L * a.tpl <= maxt && 2 * a.L <= lines) a.L *= 2;
+        while (2 * a.L <= 16 && 2 * a.L * a.tpl <= maxt && 2 * a.L <= lines &&
+               (a.fx->ct ? fxc_smem_bytes(a.M, 2 * a.L) : fx_smem_bytes(a.M, 2 * a.L)) <= kFxMaxSmem)
+          a.L *= 2;
       cudaError_t err = launch_dtt_pass(d->prec, contiguous, a, st);
       if (err != cudaSuccess) return cuda_fail(err, "r2r pass launch");
       continue;

@@ -117,6 +117,8 @@ cudaError_t launch_axis_one(int prec_bytes, int kind, bool contiguous, const Pas
     if (!tc_pass_supported(prec_bytes, kind, contiguous, a)) return cudaErrorInvalidValue;
     return launch_tc_pass(a, stream);
   }
+  if (a.fast == 8)
+    return prec_bytes == 4 ? launch_rt_f32(kind, contiguous, a, stream) : launch_rt_f64(kind, contiguous, a, stream);
   if (a.fast == 7) return prec_bytes == 8 ? launch_fxc(kind, contiguous, a, stream) : cudaErrorInvalidValue;
   if (a.fast == 6) return prec_bytes == 8 ? launch_fx(kind, contiguous, a, stream) : cudaErrorInvalidValue;
   if (a.fast && prec_bytes != 4) return cudaErrorInvalidValue;  // the other compile-time kernels are FP32's

@@ -326,6 +326,24 @@ __device__ __forceinline__ void dft_odd(C* v) {
   });
 }
 
+// The factor of R that is a power of its smallest prime: R = P Q with P and Q
+// coprime, unless R is a prime power (P = R).
+constexpr int coprime_part(int r) {
+  int p = 2, v = 1;
+  while (r % p) ++p;
+  while (r % p == 0) {
+    v *= p;
+    r /= p;
+  }
+  return v;
+}
+// k mod P Q with k = k1 mod P and k = k2 mod Q.
+constexpr int crt(int P, int Q, int k1, int k2) {
+  for (int k = k1; k < P * Q; k += P)
+    if (k % Q == k2) return k;
+  return 0;
+}
+
 // Forward DFT of size R in registers, natural order in and out.
 template <int R, typename C>
 __device__ __forceinline__ void dftg(C* v) {
@@ -373,7 +391,6 @@ __device__ __forceinline__ void dftg(C* v) {
     });
   }
 }
-
 
 // ---------------------------------------------------------------------------
 // Per-thread view of one line: shared-memory slots and global addressing.

@@ -318,6 +318,26 @@ __device__ __forceinline__ void dft_pq(I2* v) {
     dev::static_for<0, Q>([&](auto I) { v[k1 + P * decltype(I)::value] = u[decltype(I)::value]; });
   });
 }
+// R = P Q coprime, without twiddles (as dev::dftg)
+template <int R, int P>
+__device__ __forceinline__ void dft_coprime(I2* v) {
+  constexpr int Q = R / P;
+  I2 a[R];
+  dev::static_for<0, Q>([&](auto I) {
+    constexpr int n2 = decltype(I)::value;
+    I2 t[P];
+    dev::static_for<0, P>([&](auto J) { t[decltype(J)::value] = v[(Q * decltype(J)::value + P * n2) % R]; });
+    dft<P>(t);
+    dev::static_for<0, P>([&](auto K) { a[n2 * P + decltype(K)::value] = t[decltype(K)::value]; });
+  });
+  dev::static_for<0, P>([&](auto K) {
+    constexpr int k1 = decltype(K)::value;
+    I2 u[Q];
+    dev::static_for<0, Q>([&](auto I) { u[decltype(I)::value] = a[decltype(I)::value * P + k1]; });
+    dft<Q>(u);
+    dev::static_for<0, Q>([&](auto I) { v[dev::crt(P, Q, k1, decltype(I)::value)] = u[decltype(I)::value]; });
+  });
+}
 template <int R>
 __device__ __forceinline__ void dft(I2* v) {
   if constexpr (R == 1) {
@@ -331,14 +351,12 @@ __device__ __forceinline__ void dft(I2* v) {
     dft4v(v[0], v[1], v[2], v[3]);
   } else if constexpr (R == 5) {
     dft5p(v);
+  } else if constexpr (dev::coprime_part(R) != R) {
+    dft_coprime<R, dev::coprime_part(R)>(v);
   } else if constexpr (R % 4 == 0) {
     dft_pq<R, 4>(v);
-  } else if constexpr (R % 5 == 0) {
-    dft_pq<R, 5>(v);
   } else if constexpr (R % 3 == 0) {
     dft_pq<R, 3>(v);
-  } else if constexpr (R % 2 == 0) {
-    dft_pq<R, 2>(v);
   } else {
     dft_odd<R>(v, [&](int m, I2 x) { v[m] = x; });
   }

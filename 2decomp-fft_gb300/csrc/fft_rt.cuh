@@ -1,0 +1,415 @@
+// Runtime-planned axis passes of smooth lengths, one kernel for FP32 and for
+// FP64 in fixed point: radices of at most 16 (fixed point: 10), the first
+// stage on the points as they are loaded, the last one stored from its
+// registers, twiddles from a stage-major table.
+//
+// The general runtime kernels (fft_axis.cu, fft_fx.cu) load the lines into
+// shared memory, run every prime or power-of-two stage from one buffer to
+// another with the divisions and 64-bit addresses of arbitrary lengths, and
+// store from there.  They stay for lines with other factors.  What bounds
+// them is the instructions and barriers of their stages (225 = 3 3 5 5 there,
+// 15 15 here), not memory.
+#pragma once
+
+#include "fft_fx.cuh"
+
+namespace gbfft {
+namespace rt {
+
+using namespace dev;
+
+// Forward DFT of size R in registers (FP32).  R = P Q coprime goes without
+// twiddles between (Good's mapping: n = Q n1 + P n2 mod R gives W_R^(n k) =
+// W_P^(n1 k) W_Q^(n2 k), and result k sits at (k mod P, k mod Q)).
+template <int R>
+__device__ __forceinline__ void dft_f32(float2* v) {
+  if constexpr (R == 1 || coprime_part(R) == R) {
+    dftg<R>(v);
+  } else {
+    constexpr int P = coprime_part(R), Q = R / P;
+    float2 a[R];
+    static_for<0, Q>([&](auto I2) {
+      constexpr int n2 = decltype(I2)::value;
+      float2 t[P];
+      static_for<0, P>([&](auto I1) { t[decltype(I1)::value] = v[(Q * decltype(I1)::value + P * n2) % R]; });
+      dft_f32<P>(t);
+      static_for<0, P>([&](auto K1) { a[n2 * P + decltype(K1)::value] = t[decltype(K1)::value]; });
+    });
+    static_for<0, P>([&](auto K1) {
+      constexpr int k1 = decltype(K1)::value;
+      float2 u[Q];
+      static_for<0, Q>([&](auto I2) { u[decltype(I2)::value] = a[decltype(I2)::value * P + k1]; });
+      dft_f32<Q>(u);
+      static_for<0, Q>([&](auto K2) { v[crt(P, Q, k1, decltype(K2)::value)] = u[decltype(K2)::value]; });
+    });
+  }
+}
+
+// FP32 on the CUDA cores.  The table twiddles are a high and a low part: on a
+// line with a few large modes the rounding errors of a table add up in the
+// modes' bins.  (Over 70 random boxes the rel-L2 against 64 bits is 0.96 of
+// the general kernel's on average, 0.83 to 1.08 on single ones; with rounded
+// twiddles 0.98.)
+struct F32 {
+  using T = float;
+  using C = float2;
+  using W = float4;  // real, imaginary: high parts, low parts
+  static constexpr int kMaxR = 16;
+  static constexpr bool kFixed = false;
+  static constexpr int kPadShift = 4;
+  __device__ __forceinline__ static W root(const W* p) { return __ldg(p); }
+  __device__ __forceinline__ static C mul(C a, W w, int) {
+    return make_float2(fmaf(a.x, w.x, fmaf(-a.y, w.y, fmaf(-a.y, w.w, a.x * w.z))),
+                       fmaf(a.x, w.y, fmaf(a.y, w.x, fmaf(a.y, w.z, a.x * w.w))));
+  }
+  __device__ __forceinline__ static C first(C a) { return a; }
+  template <int R>
+  __device__ __forceinline__ static void dft(C* v) { dft_f32<R>(v); }
+};
+// FP64 in fixed point.
+struct Fixed {
+  using T = double;
+  using C = fx::I2;
+  using W = fx::W4;
+  static constexpr int kMaxR = 10;
+  static constexpr bool kFixed = true;
+  static constexpr int kPadShift = 3;
+  __device__ __forceinline__ static W root(const W* p) { return fx::ldw(p); }
+  __device__ __forceinline__ static C mul(C a, W w, int r) { return fx::mul_tw(a, w, r); }
+  __device__ __forceinline__ static C first(C a) { return fx::mk(fx::scale_down(a.x), fx::scale_down(a.y)); }
+  template <int R>
+  __device__ __forceinline__ static void dft(C* v) { fx::dft<R>(v); }
+};
+
+// Calls f(integral_constant<R>) for the runtime radix R.
+template <class A, class F>
+__device__ __forceinline__ void with_radix(int R, F&& f) {
+  switch (R) {
+    case 2: f(std::integral_constant<int, 2>{}); break;
+    case 3: f(std::integral_constant<int, 3>{}); break;
+    case 4: f(std::integral_constant<int, 4>{}); break;
+    case 5: f(std::integral_constant<int, 5>{}); break;
+    case 6: f(std::integral_constant<int, 6>{}); break;
+    case 7: f(std::integral_constant<int, 7>{}); break;
+    case 8: f(std::integral_constant<int, 8>{}); break;
+    case 9: f(std::integral_constant<int, 9>{}); break;
+    case 10: f(std::integral_constant<int, 10>{}); break;
+    default:
+      if constexpr (!A::kFixed) {
+        if (R == 11) f(std::integral_constant<int, 11>{});
+        else if (R == 12) f(std::integral_constant<int, 12>{});
+        else if (R == 13) f(std::integral_constant<int, 13>{});
+        else if (R == 14) f(std::integral_constant<int, 14>{});
+        else if (R == 15) f(std::integral_constant<int, 15>{});
+        else f(std::integral_constant<int, 16>{});
+      }
+      break;
+  }
+}
+
+// Exchange slots of a tile: strided dense (the lanes walk the lines),
+// contiguous lines with a pad entry per 128 bytes.
+template <class A, bool CONTIG>
+struct Slots {
+  int base, L;
+  __device__ __forceinline__ int operator()(int n) const {
+    return CONTIG ? base + n + (n >> A::kPadShift) : n * L + base;
+  }
+};
+
+// Global accesses of a thread's points t + n: one multiply-add an address
+// (the row strides are below 2^28 elements).
+template <typename T, int KIND, bool CONTIG>
+struct Io {
+  using C = Cx<T>;
+  const LineCtx<T, KIND, CONTIG>& c;
+  const char *s0, *s1;
+  char *d0, *d1;
+  unsigned ss, ds;
+  __device__ __forceinline__ explicit Io(const LineCtx<T, KIND, CONTIG>& ctx) : c(ctx) {
+    constexpr int SB = (KIND == K_R2C ? 1 : 2) * sizeof(T), DB = (KIND == K_C2R ? 1 : 2) * sizeof(T);
+    ss = (unsigned)c.ssn * SB;
+    ds = (unsigned)c.dsn * DB;
+    s0 = reinterpret_cast<const char*>(c.src) + c.sb0 * SB + (unsigned long long)ss * (unsigned)c.t;
+    s1 = reinterpret_cast<const char*>(c.src) + c.sb1 * SB + (unsigned long long)ss * (unsigned)c.t;
+    d0 = reinterpret_cast<char*>(c.dst) + c.db0 * DB + (unsigned long long)ds * (unsigned)c.t;
+    d1 = reinterpret_cast<char*>(c.dst) + c.db1 * DB + (unsigned long long)ds * (unsigned)c.t;
+  }
+  __device__ __forceinline__ static C zero() { return cmk<C>(T(0), T(0)); }
+#ifdef GB_DEBUG_BOUNDS
+  __device__ __forceinline__ C load(int n) const { return c.gload_raw(c.t + n); }
+  __device__ __forceinline__ void halves(int n, C& a, C& b) const {
+    a = c.half(0, c.t + n);
+    b = c.half(1, c.t + n);
+  }
+  __device__ __forceinline__ void store(int n, C v) const { c.gstore_raw(c.t + n, v); }
+  __device__ __forceinline__ void put_halves(int n, C a, C b) const {
+    c.put_half(0, c.t + n, a);
+    c.put_half(1, c.t + n, b);
+  }
+#else
+  __device__ __forceinline__ unsigned long long so(int n) const { return (unsigned long long)(unsigned)n * ss; }
+  __device__ __forceinline__ unsigned long long dof(int n) const { return (unsigned long long)(unsigned)n * ds; }
+  template <typename V>
+  __device__ __forceinline__ static V ld(const char* p) {
+    return LineCtx<T, KIND, CONTIG>::ld(reinterpret_cast<const V*>(p));
+  }
+  // c2c: the point; r2c: both real lines' values
+  __device__ __forceinline__ C load(int n) const {
+    if (!c.valid) return zero();
+    if (KIND == K_C2C || (!CONTIG && c.pvec && c.has1)) return ld<C>(s0 + so(n));
+    return cmk<C>(ld<T>(s0 + so(n)), c.has1 ? ld<T>(s1 + so(n)) : T(0));
+  }
+  // c2r: both half spectra's points
+  __device__ __forceinline__ void halves(int n, C& a, C& b) const {
+    a = b = zero();
+    if (!c.valid) return;
+    if constexpr (sizeof(T) == 4) {
+      if (c.cvec && c.has1) {
+        const float4 q = *reinterpret_cast<const float4*>(s0 + so(n));
+        a = make_float2(q.x, q.y);
+        b = make_float2(q.z, q.w);
+        return;
+      }
+    }
+    a = ld<C>(s0 + so(n));
+    if (c.has1) b = ld<C>(s1 + so(n));
+  }
+  __device__ __forceinline__ void store(int n, C v) const {
+    if (!c.valid) return;
+    if (KIND == K_C2C || (!CONTIG && c.pvec && c.has1)) {
+      *reinterpret_cast<C*>(d0 + dof(n)) = v;
+      return;
+    }
+    *reinterpret_cast<T*>(d0 + dof(n)) = v.x;
+    if (c.has1) *reinterpret_cast<T*>(d1 + dof(n)) = v.y;
+  }
+  __device__ __forceinline__ void put_halves(int n, C a, C b) const {
+    if (!c.valid) return;
+    if constexpr (sizeof(T) == 4) {
+      if (c.cvec && c.has1) {
+        *reinterpret_cast<float4*>(d0 + dof(n)) = make_float4(a.x, a.y, b.x, b.y);
+        return;
+      }
+    }
+    *reinterpret_cast<C*>(d0 + dof(n)) = a;
+    if (c.has1) *reinterpret_cast<C*>(d1 + dof(n)) = b;
+  }
+#endif
+};
+
+// How a result leaves the arithmetic.
+template <class A>
+struct Out {
+  int adj, flip;
+  __device__ __forceinline__ float2 operator()(float2 v) const {
+    return make_float2(v.x, __int_as_float(__float_as_int(v.y) ^ flip));
+  }
+  __device__ __forceinline__ double2 operator()(fx::I2 v) const {
+    return make_double2(fx::to_double(v.x, adj), fx::to_double(v.y, adj, flip));
+  }
+};
+
+template <class A, int KIND, bool CONTIG>
+__global__ void __launch_bounds__(rt_threads(sizeof(typename A::T)), 2) rt_pass_kernel(const __grid_constant__ PassArgs a,
+                                                                const __grid_constant__ FxPlan p) {
+  using T = typename A::T;
+  using C = typename A::C;
+  using W = typename A::W;
+  using G = Cx<T>;
+  constexpr int MR = A::kMaxR;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  chained_entry();
+  LineCtx<T, KIND, CONTIG> c;
+  c.init(a);
+  const Io<T, KIND, CONTIG> io(c);
+  const int N = c.N, tpl = c.tpl, t = c.t, last = p.nst - 1;
+  C* buf0 = reinterpret_cast<C*>(smem_raw);
+  C* buf1 = buf0 + rt_entries(N, a.L);
+  Slots<A, CONTIG> slot;
+  slot.L = a.L;
+  slot.base = CONTIG ? c.line * (N + (N >> A::kPadShift) + 1) : c.line;
+  const W* tw = reinterpret_cast<const W*>(p.tw);
+  const int back = KIND == K_C2R || (KIND == K_C2C && c.inverse) ? (int)0x80000000 : 0;
+  Out<A> out{0, back};
+
+  // the points of butterfly t of the first stage (c2r: the half spectra,
+  // points t, t + tpl, ... of both)
+  const int R0 = p.radix[0], nb0 = N / R0, h = N / 2 + 1;
+  constexpr int Q = KIND == K_C2R ? 2 * (MR / 2 + 1) : MR;
+  G x[Q];
+  if constexpr (KIND == K_C2R) {
+#pragma unroll
+    for (int i = 0; i < Q / 2; ++i) {
+      const int j = t + i * tpl;
+      x[2 * i] = x[2 * i + 1] = io.zero();
+      if (j < h) io.halves(i * tpl, x[2 * i], x[2 * i + 1]);
+      if (j == 0 || 2 * j == N) x[2 * i].y = x[2 * i + 1].y = 0;  // Im of the DC and Nyquist bins is ignored
+    }
+  } else {
+#pragma unroll
+    for (int r = 0; r < MR; ++r) x[r] = r < R0 && t < nb0 ? io.load(r * nb0) : io.zero();
+  }
+  C v[MR];
+  if constexpr (A::kFixed) {
+    int* smax = reinterpret_cast<int*>(smem_raw + rt_smem_bytes(8, N, a.L, p.nst) - (size_t)a.L * 8);
+    unsigned* ssum = reinterpret_cast<unsigned*>(smax + a.L);
+    const int threads = blockDim.x * blockDim.y;
+    for (int i = threadIdx.x + threadIdx.y * blockDim.x; i < 2 * a.L; i += threads) smax[i] = 0;
+    __syncthreads();
+    fx::Scale sc;
+    if (!sc.template find<Q>(x, &smax[c.line], &ssum[c.line])) {
+      fx::fallback<KIND, CONTIG>(a, reinterpret_cast<double2*>(smem_raw));
+      return;
+    }
+    constexpr int X = KIND == K_C2R ? 1 : 0;  // a point combines two values
+    int top = -1021 + X;
+#pragma unroll 1
+    for (int s = 0; s <= last; ++s) top = max(top, sc.bound(p.lg[s], X) - p.shift[s]);
+    const int sh = sc.shift(top);
+    out.adj = (sc.em - 62 + top + p.shift[last]) << 20;
+    if constexpr (KIND == K_C2R) {
+#pragma unroll
+      for (int i = 0; i < Q / 2; ++i) {
+        const int j = t + i * tpl;
+        if (j < h) {
+          const fx::ll ax = fx::to_fixed(x[2 * i].x, sh), ay = fx::to_fixed(x[2 * i].y, sh);
+          const fx::ll bx = fx::to_fixed(x[2 * i + 1].x, sh), by = fx::to_fixed(x[2 * i + 1].y, sh);
+          // z = x1 + i x2, conjugated for the inverse-by-conjugation
+          buf0[slot(j)] = fx::mk(ax - by, -(ay + bx));
+          if (j > 0 && 2 * j < N) buf0[slot(N - j)] = fx::mk(ax + by, ay - bx);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < MR; ++r) v[r] = fx::mk(fx::to_fixed(x[r].x, sh), fx::to_fixed(x[r].y, sh, back));
+    }
+  } else if constexpr (KIND == K_C2R) {
+#pragma unroll
+    for (int i = 0; i < Q / 2; ++i) {
+      const int j = t + i * tpl;
+      if (j < h) {
+        const G u = x[2 * i], w = x[2 * i + 1];
+        buf0[slot(j)] = make_float2(u.x - w.y, -(u.y + w.x));
+        if (j > 0 && 2 * j < N) buf0[slot(N - j)] = make_float2(u.x + w.y, u.y - w.x);
+      }
+    }
+  } else {
+#pragma unroll
+    for (int r = 0; r < MR; ++r) v[r] = make_float2(x[r].x, __int_as_float(__float_as_int(x[r].y) ^ back));
+  }
+
+  // stage 0, from the registers (c2r: from buffer 0) into buffer 0
+  C* A0 = buf0;
+  C* B = buf1;
+  if constexpr (KIND == K_C2R) {
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < MR; ++r)
+      if (r < R0 && t < nb0) v[r] = buf0[slot(t + r * nb0)];
+    __syncthreads();
+  }
+  if (t < nb0) {
+    with_radix<A>(R0, [&](auto RC) {
+      constexpr int R = decltype(RC)::value;
+      A::template dft<R>(v);
+#pragma unroll
+      for (int r = 0; r < R; ++r) A0[slot(t * R + r)] = v[r];
+    });
+  }
+  __syncthreads();
+  // the stages between, from buffer to buffer
+  int s = 1;
+#pragma unroll 1
+  for (; s < last; ++s) {
+    const int Ns = p.ns[s];
+    const unsigned magic = p.magic[s];
+    with_radix<A>(p.radix[s], [&](auto RC) {
+      constexpr int R = decltype(RC)::value;
+      const int nb = N / R;
+#pragma unroll 1
+      for (int b = t; b < nb; b += tpl) {
+        const int k = b - (int)__umulhi((unsigned)b, magic) * Ns, base = (b - k) * R + k;
+        const W* w = tw + (Ns - 1) + k;
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = A0[slot(b + r * nb)];
+        v[0] = A::first(v[0]);
+#pragma unroll
+        for (int r = 1; r < R; ++r) v[r] = A::mul(v[r], A::root(w + (r - 1) * Ns), r);
+        A::template dft<R>(v);
+#pragma unroll
+        for (int r = 0; r < R; ++r) B[slot(base + r * Ns)] = v[r];
+      }
+    });
+    __syncthreads();
+    C* const q = A0;
+    A0 = B;
+    B = q;
+  }
+  // the last stage: its outputs are points b + r ns
+  {
+    const int Ns = p.ns[last];
+    with_radix<A>(p.radix[last], [&](auto RC) {
+      constexpr int R = decltype(RC)::value;
+#pragma unroll 1
+      for (int b = t; b < Ns; b += tpl) {  // n / R = ns butterflies, k = b
+        const W* w = tw + (Ns - 1) + b;
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = A0[slot(b + r * Ns)];
+        v[0] = A::first(v[0]);
+#pragma unroll
+        for (int r = 1; r < R; ++r) v[r] = A::mul(v[r], A::root(w + (r - 1) * Ns), r);
+        A::template dft<R>(v);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          // in place for r2c: the thread's own points
+          if constexpr (KIND == K_R2C) A0[slot(b + r * Ns)] = v[r];
+          else io.store(b - t + r * Ns, out(v[r]));
+        }
+      }
+    });
+  }
+  if constexpr (KIND == K_R2C) {
+    __syncthreads();
+    if constexpr (A::kFixed) out.adj -= 1 << 20;  // the halves of both spectra
+#pragma unroll 1
+    for (int k = t; k < h; k += tpl) {
+      const C zk = A0[slot(k)], zm = A0[slot(k == 0 ? 0 : N - k)];
+      if constexpr (A::kFixed) {
+        io.put_halves(k - t, out(fx::mk(zk.x + zm.x, zk.y - zm.y)), out(fx::mk(zk.y + zm.y, zm.x - zk.x)));
+      } else {
+        io.put_halves(k - t, make_float2((zk.x + zm.x) * 0.5f, (zk.y - zm.y) * 0.5f),
+                      make_float2((zk.y + zm.y) * 0.5f, (zm.x - zk.x) * 0.5f));
+      }
+    }
+  }
+}
+
+template <class A, int KIND, bool CONTIG>
+cudaError_t launch_k(const PassArgs& a, cudaStream_t stream) {
+  const FxPlan& p = *a.fx;
+  const size_t smem = rt_smem_bytes((int)sizeof(typename A::T), a.n, a.L, p.nst);
+  if (p.nst < 2 || a.L < 1 || a.L * a.tpl > rt_threads((int)sizeof(typename A::T)) || a.tpl * p.radix[0] < a.n || smem > kFxMaxSmem)
+    return cudaErrorInvalidValue;
+  auto kern = rt_pass_kernel<A, KIND, CONTIG>;
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  const dim3 block = CONTIG ? dim3(a.tpl, a.L) : dim3(a.L, a.tpl);
+  const dim3 grid((unsigned)((a.nlines + a.L - 1) / a.L), CONTIG ? 1u : (unsigned)a.nv);
+  const cudaError_t err = launch_chained(kern, grid, block, smem, stream, a, p);
+  add_launches(1);
+  return err != cudaSuccess ? err : cudaGetLastError();
+}
+
+template <class A>
+cudaError_t launch(int kind, bool contiguous, const PassArgs& a, cudaStream_t s) {
+  if (kind == K_C2C) return contiguous ? launch_k<A, K_C2C, true>(a, s) : launch_k<A, K_C2C, false>(a, s);
+  if (kind == K_R2C) return contiguous ? launch_k<A, K_R2C, true>(a, s) : launch_k<A, K_R2C, false>(a, s);
+  if (kind == K_C2R) return contiguous ? launch_k<A, K_C2R, true>(a, s) : launch_k<A, K_C2R, false>(a, s);
+  return cudaErrorInvalidValue;
+}
+
+}  // namespace rt
+}  // namespace gbfft

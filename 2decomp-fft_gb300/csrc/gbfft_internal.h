@@ -61,8 +61,9 @@ struct BlueTables {
 // direct-sum stage costs that many multiply-adds a point.
 constexpr int kBluePrime = 256;
 
-// Fixed-point plan of one FP64 axis (fft_fx.cu): radix stages after ns
-// points, and for the line's scale, per stage, the exponent that bounds how
+// Plan of one axis for the fixed-point FP64 kernels (fft_fx.cu) and the
+// smooth-length kernels (fft_rt.cuh): radix stages after ns points, and for
+// the scale of a fixed-point line, per stage, the exponent that bounds how
 // many inputs a value then sums (lg) and the powers of two it was divided
 // by (shift).  Built by the engine for one length; the struct lives on the
 // host and travels as a kernel argument.
@@ -73,10 +74,11 @@ struct FxPlan {
   unsigned magic[kMaxStages];  // ceil(2^32 / ns)
   int lg[kMaxStages];
   int shift[kMaxStages];
-  const void* tw;    // stage-major Q62 roots (stage_twiddles order)
+  const void* tw;    // stage-major roots (stage_twiddles order), Q62 or FP32
   const void* root;  // the n roots in Q62, for direct-sum stages
   int tpl;           // threads a line (runtime plans: at least n / kFxPoints)
   int ct;            // 1: a compile-time plan (fft_fxc.cuh)
+  int rt;            // 1: a smooth-length runtime plan (fft_rt.cuh)
 };
 constexpr int kFxPoints = 8;        // points a thread loads at most
 constexpr int kFxMaxThreads = 512;  // threads of a CTA
@@ -152,7 +154,8 @@ struct PassArgs {
                    // 3: split-precision tensor-core kernel (mma.sync), 4:
                    // balanced non-power-of-two plan, 5: split-precision
                    // tcgen05 kernel (fft_tc.cu), 6: fixed-point FP64 kernel
-                   // (fft_fx.cu), 7: its compile-time plans (fft_fxc.cuh)
+                   // (fft_fx.cu), 7: its compile-time plans (fft_fxc.cuh),
+                   // 8: runtime plans of smooth lengths (fft_rt.cuh)
   int pair_vec;    // r2c/c2r on strided lines, bit 0: the two real lines of a
                    // pair are adjacent and aligned (read/write as one pair);
                    // bit 1 (FP32): so are their two complex lines, 16-byte
@@ -176,8 +179,8 @@ struct PassArgs {
                    // caught an access outside an array (null: not recorded)
   long long src_elems, dst_elems;  // extents of the two arrays in elements of
                                    // each side's type (bounds-checked build)
-  const FxPlan* fx;  // fast == 6: host-side plan of the fixed-point FP64 pass
-                     // (fft_fx.cu); never read on the device
+  const FxPlan* fx;  // fast 6, 7, 8: the axis's host-side plan; the kernels get
+                     // a copy
   const BlueTables* blue;  // host-side tables of the chirp-z path (fft_long.cu),
                            // null unless the axis runs it; never read on the device
   int radix[kMaxStages];
@@ -283,6 +286,21 @@ cudaError_t launch_fast_f32_real(int kind, bool contiguous, const PassArgs& a, c
 
 // Compile-time plans, one function a kind and layout and group of lengths.
 cudaError_t launch_fxc(int kind, bool contiguous, const PassArgs& a, cudaStream_t s);
+// Runtime plans of smooth lengths (fft_rt.cuh), FP32 and fixed point.
+// threads of a CTA: two CTAs an SM leave 64 registers a thread (FP32), 80
+// (fixed point)
+__host__ __device__ constexpr int rt_threads(int prec_bytes) { return prec_bytes == 4 ? 512 : 384; }
+constexpr int rt_max_radix(int prec_bytes) { return prec_bytes == 4 ? 16 : 10; }
+// buffer entries of L lines: a pad entry per 8
+__host__ __device__ constexpr size_t rt_entries(int n, int L) { return ((size_t)n + n / 8 + 2) * (size_t)L + 2; }
+// one buffer for two stages, two for more (the fixed-point kernel's FP64
+// fallback needs two for a single line), and the lines' scale words
+__host__ __device__ constexpr size_t rt_smem_bytes(int prec_bytes, int n, int L, int nst) {
+  return (nst > 2 || (prec_bytes == 8 && L == 1) ? 2 : 1) * rt_entries(n, L) * (size_t)(2 * prec_bytes) + 32 +
+         (size_t)L * 8;
+}
+cudaError_t launch_rt_f32(int kind, bool contiguous, const PassArgs& a, cudaStream_t s);
+cudaError_t launch_rt_f64(int kind, bool contiguous, const PassArgs& a, cudaStream_t s);
 cudaError_t launch_fx(int kind, bool contiguous, const PassArgs& a, cudaStream_t s);
 
 // The x and y passes of one z-plane run by one fused kernel
