@@ -68,36 +68,36 @@ cudaError_t launch_typed(const PassArgs& a, cudaStream_t stream) {
   return err != cudaSuccess ? err : cudaGetLastError();
 }
 
-// Identity copy, 16 bytes per access, 4 accesses in flight per thread.
-__global__ void __launch_bounds__(256) copy16_kernel(const uint4* __restrict__ s, uint4* __restrict__ d,
-                                                      size_t n) {
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  for (; i + 3 * stride < n; i += 4 * stride) {
-    uint4 a0 = s[i], a1 = s[i + stride], a2 = s[i + 2 * stride], a3 = s[i + 3 * stride];
-    d[i] = a0;
-    d[i + stride] = a1;
-    d[i + 2 * stride] = a2;
-    d[i + 3 * stride] = a3;
-  }
-  for (; i < n; i += stride) d[i] = s[i];
+// Identity copy.  A block of 1024 threads moves 2048 consecutive words of the
+// widest type both arrays are aligned to, two a thread, both loads in flight;
+// the last block also moves the bytes after the last whole word.  One block
+// per 32 KB instead of a grid that strides over the array: the blocks reach
+// DRAM in address order (256^3 complex128, 268 MB: 90.4 -> 79.2 us, 6.8 TB/s;
+// 256 x 4, 256 x 8, 512 x 4 words, 32-byte words and streaming hints measured
+// 79.7 to 80.7), and a chain of small copies overlaps its launches.
+constexpr int kCopyThreads = 1024;
+template <typename V>
+__global__ void __launch_bounds__(kCopyThreads) copy_kernel(const V* s, V* d, size_t n, int tail) {
+  chained_entry();
+  const size_t i = (size_t)blockIdx.x * (2 * kCopyThreads) + threadIdx.x;
+  const bool two = i + kCopyThreads < n;
+  V a, b;
+  if (i < n) a = s[i];
+  if (two) b = s[i + kCopyThreads];
+  if (i < n) d[i] = a;
+  if (two) d[i + kCopyThreads] = b;
+  if (blockIdx.x + 1 == gridDim.x && (int)threadIdx.x < tail)
+    reinterpret_cast<unsigned char*>(d + n)[threadIdx.x] = reinterpret_cast<const unsigned char*>(s + n)[threadIdx.x];
 }
 
-__global__ void copy1_kernel(const unsigned char* __restrict__ s, unsigned char* __restrict__ d,
-                             size_t n) {
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) d[i] = s[i];
-}
-
-int sm_count() {
-  static std::atomic<int> cached{0};
-  int v = cached.load();
-  if (v) return v;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 152;
-  if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) v = 152;
-  cached.store(v);
-  return v;
+template <typename V>
+cudaError_t launch_copy_as(const void* src, void* dst, size_t bytes, cudaStream_t stream) {
+  const size_t n = bytes / sizeof(V), blocks = (n + 2 * kCopyThreads - 1) / (2 * kCopyThreads);
+  const cudaError_t err =
+      launch_chained(copy_kernel<V>, dim3((unsigned)(blocks ? blocks : 1)), dim3(kCopyThreads), 0, stream,
+                     reinterpret_cast<const V*>(src), reinterpret_cast<V*>(dst), n, (int)(bytes % sizeof(V)));
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return err != cudaSuccess ? err : cudaGetLastError();
 }
 
 }  // namespace
@@ -172,32 +172,12 @@ cudaError_t launch_axis_pass(int prec_bytes, int kind, bool contiguous, const Pa
 
 cudaError_t launch_copy(const void* src, void* dst, size_t bytes, cudaStream_t stream) {
   if (bytes == 0 || src == dst) return cudaSuccess;
-  const int blocks_max = sm_count() * 8;
-  const uintptr_t ps = (uintptr_t)src, pd = (uintptr_t)dst;
-  size_t head = 0;
-  if (((ps | pd) & 15) == 0) {
-    const size_t n16 = bytes / 16;
-    if (n16) {
-      const size_t want = (n16 + 4 * 256 - 1) / (4 * 256);
-      const int blocks = (int)(want < (size_t)blocks_max ? (want ? want : 1) : blocks_max);
-      copy16_kernel<<<blocks, 256, 0, stream>>>(reinterpret_cast<const uint4*>(src),
-                                                 reinterpret_cast<uint4*>(dst), n16);
-      g_launches.fetch_add(1, std::memory_order_relaxed);
-      cudaError_t e = cudaGetLastError();
-      if (e != cudaSuccess) return e;
-    }
-    head = n16 * 16;
-  }
-  if (head < bytes) {
-    const size_t rest = bytes - head;
-    const size_t want = (rest + 255) / 256;
-    const int blocks = (int)(want < (size_t)blocks_max ? want : blocks_max);
-    copy1_kernel<<<blocks, 256, 0, stream>>>(reinterpret_cast<const unsigned char*>(src) + head,
-                                              reinterpret_cast<unsigned char*>(dst) + head, rest);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    return cudaGetLastError();
-  }
-  return cudaSuccess;
+  const uintptr_t at = (uintptr_t)src | (uintptr_t)dst;
+  if (at % 16 == 0) return launch_copy_as<uint4>(src, dst, bytes, stream);
+  if (at % 8 == 0) return launch_copy_as<uint2>(src, dst, bytes, stream);
+  if (at % 4 == 0) return launch_copy_as<unsigned>(src, dst, bytes, stream);
+  // blocks of 2 KB of single bytes: up to 4 TB in one grid
+  return launch_copy_as<unsigned char>(src, dst, bytes, stream);
 }
 
 long long launch_counter() { return g_launches.load(); }
