@@ -477,7 +477,8 @@ std::vector<long double> roots_ld(int n) {
 std::vector<int> q62_table(const std::vector<long double>& t) {
   std::vector<int> q(2 * t.size());
   for (size_t i = 0; i < t.size(); ++i) {
-    const long long x = llrintl(ldexpl(t[i], 62));
+    long long x = llrintl(ldexpl(t[i], 62));
+    if ((unsigned)(unsigned long long)x == 0x80000000u) ++x;  // the kernels negate the halves
     const int lo = (int)(unsigned)(unsigned long long)x;
     q[2 * i] = lo;
     q[2 * i + 1] = (int)((x - lo) >> 32);

@@ -10,10 +10,11 @@
 // line next to a large one keeps all its digits.
 //
 // Formats: a value is a signed 64-bit integer v, |v| < 2^62.  Table twiddles
-// are Q62 (w 2^62) and multiplying by one divides by 2, after a stage of
-// radix 16 by 4 (a value grows by sqrt(R) in a stage of radix R on noise and
-// by nothing on a line with one large point; a division by more loses bits);
-// constants of the butterflies are Q64 and keep the scale.  Every product is rounded to
+// are Q62 (w 2^62) and multiplying by one divides by 2, in the compile-time
+// plans after a stage of radix 8 or more by 4, which is cheaper (a value grows
+// by sqrt(R) in a stage of radix R on noise and by nothing on a line with one
+// large point; dividing by more than the growth loses bits); constants of the
+// butterflies are Q64 and keep the scale.  Every product is rounded to
 // nearest at 2^-64 of its factors' range; the low 32 x 32 product (below
 // half a unit) is left out.
 #pragma once
@@ -30,7 +31,7 @@ struct alignas(16) I2 {
   ll x, y;
 };
 // Q62 root: real and imaginary parts as balanced 32-bit halves (both signed,
-// value = hi 2^32 + lo)
+// neither -2^31, value = hi 2^32 + lo)
 struct alignas(16) W4 {
   int xl, xh, yl, yh;
 };
@@ -43,17 +44,12 @@ __device__ __forceinline__ I2 mk(ll a, ll b) {
 }
 __device__ __forceinline__ I2 add(I2 a, I2 b) { return mk(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ I2 sub(I2 a, I2 b) { return mk(a.x - b.x, a.y - b.y); }
-// a * b + c and a * b, 32 x 32 -> 64 bits.  Spelt out: from (ll)a * b the
+// a * b + c, 32 x 32 -> 64 bits.  Spelt out: from (ll)a * b the
 // compiler made unsigned products and sign corrections (76 of 313
 // instructions a point of a 256-point pass).
 __device__ __forceinline__ ll madw(int a, int b, ll c) {
   ll d;
   asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ ll mulw(int a, int b) {
-  ll d;
-  asm("mul.wide.s32 %0, %1, %2;" : "=l"(d) : "r"(a), "r"(b));
   return d;
 }
 // balanced halves: v = hi(v) 2^32 + lo(v), both signed
@@ -181,9 +177,10 @@ __device__ __forceinline__ I2 mul_tw(I2 a, W4 w, int r) {
   const int xd = xh * (3 - SH), yd = yh * (3 - SH);
   const int odd = (0x6996 >> (r & 15)) & 1;
   const ll ur = kHalf / (3 - SH) - odd, ui = kHalf / (3 - SH) - 1 + odd;
-  const ll mr = madw(xl, w.xh, madw(xh, w.xl, ur)) - madw(yl, w.yh, mulw(yh, w.yl));
+  const int nh = -w.yh, nl = -w.yl;
+  const ll mr = madw(yl, nh, madw(yh, nl, madw(xl, w.xh, madw(xh, w.xl, ur))));
   const ll mi = madw(yl, w.xh, madw(yh, w.xl, madw(xl, w.yh, madw(xh, w.yl, ui))));
-  return mk(madw(xd, w.xh, mr >> (30 + SH)) - mulw(yd, w.yh), madw(yd, w.xh, madw(xd, w.yh, mi >> (30 + SH))));
+  return mk(madw(yd, nh, madw(xd, w.xh, mr >> (30 + SH))), madw(yd, w.xh, madw(xd, w.yh, mi >> (30 + SH))));
 }
 // v / 2^SH, rounded to nearest even: the scale of a value that meets the
 // twiddle 1 (a bias common to all of them would add up in one bin)
@@ -379,12 +376,13 @@ __device__ __forceinline__ int share_base(int em) { return (em - 127) << 20; }
 __device__ __forceinline__ unsigned share_units(float sum, int count) {
   return (unsigned)(sum * 131072.0f) + (unsigned)count + 1;  // units of 2^(em - 1040)
 }
-// an integer as a double times 2^(adj >> 20) (the result is normal or zero);
-// `flip` = 0x80000000 negates
+// an integer as a double times 2^(adj >> 20), exponent and sign added to its
+// high word unless that is zero (the result is normal or zero; `flip` =
+// 0x80000000 negates)
 __device__ __forceinline__ double to_double(ll v, int adj, int flip = 0) {
   const double d = __ll2double_rn(v);
-  const int h = __double2hiint(d);
-  return __hiloint2double((h != 0 ? h + adj : 0) ^ flip, __double2loint(d));
+  const unsigned h = (unsigned)__double2hiint(d);
+  return __hiloint2double((int)(h + min(h, 1u) * ((unsigned)adj + (unsigned)flip)), __double2loint(d));
 }
 
 // The scale of a line, from the values its threads hold.
@@ -428,16 +426,19 @@ struct Scale {
 };
 
 // x as an integer, rounded: 61 mantissa bits shifted right by sh - e (not
-// negative); `flip` = 0x80000000 negates.
+// negative).  One bit more is kept until the sign is in: w and ~w become
+// w + 1 and -w, whose halves are x and -x rounded.  (Cutting the bits off
+// instead shrinks every value the same way, which adds up where a line's
+// values meet in one output.)  `flip` = 0x80000000 negates.
 __device__ __forceinline__ ll to_fixed(double x, int sh, int flip = 0) {
   const int h = __double2hiint(x);
   const unsigned l = (unsigned)__double2loint(x);
-  int s = sh - ((h >> 20) & 0x7ff);
+  int s = sh - ((h & 0x7fffffff) >> 20);
   s = s < 63 ? s : 63;
-  const unsigned mh = (unsigned)(h & 0xfffff) | 0x100000u;
-  const unsigned long long m = (((unsigned long long)mh << 32) | l) << 9;
-  const ll v = (ll)(((m >> s) + 1) >> 1);
-  return (h ^ flip) < 0 ? -v : v;
+  const int sg = (h ^ flip) >> 31;
+  const unsigned mh = (__funnelshift_l(l, (unsigned)h, 9) & 0x1fffffffu) | 0x20000000u;
+  const ll m = (ll)(((unsigned long long)(mh ^ (unsigned)sg) << 32) | ((l << 9) ^ (unsigned)sg));
+  return ((m >> s) + 1) >> 1;
 }
 // The lines of a CTA that fixed point does not take, in FP64: as many lines
 // at a time as two buffers of the CTA's shared memory hold.

@@ -38,7 +38,7 @@ struct Plan {
     return e;
   }
   // powers of two that stage s divides its inputs by (its twiddles do)
-  __host__ __device__ static constexpr int sh(int s) { return s == 0 ? 0 : radix(s - 1) >= 16 ? 2 : 1; }
+  __host__ __device__ static constexpr int sh(int s) { return s == 0 ? 0 : radix(s - 1) >= 8 ? 2 : 1; }
   __host__ __device__ static constexpr int shift(int s) {
     int v = 0;
     for (int i = 0; i <= s; ++i) v += sh(i);
