@@ -24,7 +24,7 @@ NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O2",
 
 # Sources compiled once more for each part (a define that selects the
 # instantiations of one object file), so that they compile in parallel.
-PARTS = {"fft_fxc.cu": ["-DGBFFT_FXC_PART=%d" % i for i in range(16)]}
+PARTS = {"fft_fxc.cu": ["-DGBFFT_FXC_PART=%d" % i for i in range(40)]}
 
 
 def nvcc():

@@ -42,8 +42,10 @@ cudaError_t GBFFT_CAT(launch_fxc_part, GBFFT_FXC_PART)(const Args& a, cudaStream
 
 namespace gbfft {
 
-#define GBFFT_FXC_PARTS(X) X(0) X(1) X(2) X(3) X(4) X(5) X(8) X(9) X(10) X(11) X(12) X(13)
-#define GBFFT_FXC_R2R_PARTS(X) X(6) X(7) X(14) X(15)
+#define GBFFT_FXC_PARTS(X) \
+  X(0) X(1) X(2) X(3) X(4) X(5) X(8) X(9) X(10) X(11) X(12) X(13) X(16) X(17) X(18) \
+  X(19) X(20) X(21) X(24) X(25) X(26) X(27) X(28) X(29) X(32) X(33) X(34) X(35) X(36) X(37)
+#define GBFFT_FXC_R2R_PARTS(X) X(6) X(7) X(14) X(15) X(22) X(23) X(30) X(31) X(38) X(39)
 #define GBFFT_FXC_DECL(p) cudaError_t launch_fxc_part##p(const PassArgs& a, cudaStream_t s);
 #define GBFFT_FXC_R2R_DECL(p) cudaError_t launch_fxc_part##p(const DttArgs& a, cudaStream_t s);
 GBFFT_FXC_PARTS(GBFFT_FXC_DECL)

@@ -100,26 +100,69 @@ __host__ __device__ constexpr size_t fxc_smem_bytes(int n, int L) {
 // of 256 threads an SM) but for 1024, 2048 and 4096 points, and the threads a line
 // are those that leave the fewest idle over the stages.  `group` splits the
 // instantiations over translation units.
-#define GBFFT_FXC_PLANS(X) \
-  X(0, 16, 4, 4, 4, 1, 1)     \
-  X(0, 32, 4, 8, 4, 1, 1)     \
-  X(0, 48, 8, 8, 6, 1, 1)     \
-  X(0, 64, 8, 8, 8, 1, 1)     \
-  X(0, 96, 12, 8, 4, 3, 1)    \
-  X(0, 126, 14, 9, 7, 2, 1)   \
-  X(0, 128, 16, 8, 4, 4, 1)   \
-  X(0, 160, 20, 10, 4, 4, 1)  \
-  X(0, 180, 20, 10, 9, 2, 1)  \
-  X(0, 192, 24, 8, 8, 3, 1)   \
-  X(1, 243, 27, 9, 9, 3, 1)   \
-  X(1, 256, 32, 8, 8, 4, 1)   \
-  X(1, 320, 40, 10, 8, 4, 1)  \
-  X(1, 384, 48, 8, 8, 6, 1)   \
-  X(1, 400, 50, 10, 8, 5, 1)  \
-  X(1, 512, 64, 8, 8, 8, 1)   \
-  X(1, 1024, 64, 16, 8, 8, 1) \
-  X(1, 2048, 128, 16, 16, 8, 1) \
-  X(1, 4096, 256, 16, 16, 16, 1)
+// The list holds the powers of two and the smooth lengths that grids are
+// commonly given; the others take the runtime plans (fft_rt.cuh).  r2c / c2r x
+// passes of 24 M points, us, here and on the runtime plan:
+//   72  118 / 117   144 / 158      450  205 / 208   238 / 254
+//   144 146 / 148   188 / 209      540  192 / 196   218 / 236
+//   225 176 / 174   203 / 222      720  189 / 187   225 / 233
+//   360 183 / 178   216 / 231      960  194 / 189   223 / 244
+// 600 points have no plan of ten points a thread that keeps three stages: with
+// four (10 10 3 2) 242 / 242, on the runtime plan 203 / 220.
+#define GBFFT_FXC_PLANS(X)         \
+  X(0, 16, 4, 4, 4, 1, 1)          \
+  X(0, 32, 4, 8, 4, 1, 1)          \
+  X(0, 48, 8, 8, 6, 1, 1)          \
+  X(0, 64, 8, 8, 8, 1, 1)          \
+  X(0, 96, 12, 8, 4, 3, 1)         \
+  X(0, 126, 14, 9, 7, 2, 1)        \
+  X(0, 128, 16, 8, 4, 4, 1)        \
+  X(0, 160, 20, 10, 4, 4, 1)       \
+  X(0, 180, 20, 10, 9, 2, 1)       \
+  X(0, 192, 24, 8, 8, 3, 1)        \
+  X(1, 243, 27, 9, 9, 3, 1)        \
+  X(1, 256, 32, 8, 8, 4, 1)        \
+  X(1, 320, 40, 10, 8, 4, 1)       \
+  X(1, 384, 48, 8, 8, 6, 1)        \
+  X(1, 400, 50, 10, 8, 5, 1)       \
+  X(1, 512, 64, 8, 8, 8, 1)        \
+  X(1, 1024, 64, 16, 8, 8, 1)      \
+  X(1, 2048, 128, 16, 16, 8, 1)    \
+  X(1, 4096, 256, 16, 16, 16, 1)   \
+  X(2, 72, 9, 9, 8, 1, 1)          \
+  X(2, 100, 10, 10, 10, 1, 1)      \
+  X(2, 144, 24, 6, 6, 4, 1)        \
+  X(2, 200, 20, 10, 10, 2, 1)      \
+  X(2, 225, 25, 9, 5, 5, 1)        \
+  X(2, 270, 30, 10, 9, 3, 1)       \
+  X(2, 324, 41, 9, 9, 4, 1)        \
+  X(2, 450, 50, 10, 9, 5, 1)       \
+  X(2, 540, 60, 10, 9, 3, 2)       \
+  X(2, 640, 80, 10, 8, 8, 1)       \
+  X(2, 768, 96, 8, 8, 4, 3)        \
+  X(2, 960, 120, 10, 8, 4, 3)      \
+  X(3, 80, 10, 10, 8, 1, 1)        \
+  X(3, 108, 18, 6, 6, 3, 1)        \
+  X(3, 150, 30, 6, 5, 5, 1)        \
+  X(3, 210, 42, 7, 6, 5, 1)        \
+  X(3, 240, 30, 10, 8, 3, 1)       \
+  X(3, 288, 36, 9, 8, 4, 1)        \
+  X(3, 360, 45, 10, 9, 4, 1)       \
+  X(3, 480, 60, 10, 4, 4, 3)       \
+  X(3, 576, 72, 9, 8, 8, 1)        \
+  X(3, 648, 108, 6, 6, 6, 3)       \
+  X(3, 800, 100, 10, 10, 8, 1)     \
+  X(3, 1000, 100, 10, 10, 10, 1)   \
+  X(4, 90, 10, 10, 9, 1, 1)        \
+  X(4, 120, 15, 10, 4, 3, 1)       \
+  X(4, 162, 18, 9, 9, 2, 1)        \
+  X(4, 216, 36, 6, 6, 6, 1)        \
+  X(4, 250, 25, 10, 5, 5, 1)       \
+  X(4, 300, 34, 10, 10, 3, 1)      \
+  X(4, 432, 72, 6, 6, 6, 2)        \
+  X(4, 500, 50, 10, 10, 5, 1)      \
+  X(4, 720, 90, 10, 9, 8, 1)       \
+  X(4, 900, 100, 10, 10, 9, 1)
 // threads of a CTA: 256, or what four lines (64-byte rows of a strided tile)
 // take
 __host__ __device__ constexpr int fxc_max_threads(int tpl) { return tpl <= 64 ? 256 : tpl <= 128 ? 4 * tpl : 512; }
