@@ -24,7 +24,9 @@ NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O2",
 
 # Sources compiled once more for each part (a define that selects the
 # instantiations of one object file), so that they compile in parallel.
-PARTS = {"fft_fxc.cu": ["-DGBFFT_FXC_PART=%d" % i for i in range(40)]}
+MIXED_R1 = [32, 30, 28, 27, 26, 25, 24, 22, 21, 20, 18, 16, 15, 14, 13, 12, 11, 10, 9, 8, 7, 6]
+PARTS = {"fft_fxc.cu": [["-DGBFFT_FXC_PART=%d" % i] for i in range(40)],
+         "mixed_f32.cu": [["-DGBFFT_MIXED_R1=%d" % r, "-DGBFFT_MIXED_KIND=%d" % k] for r in MIXED_R1 for k in range(3)]}
 
 
 def nvcc():
@@ -58,9 +60,9 @@ def paths(variant=""):
 VARIANT_FLAGS = {"": [], "debug": ["-DGB_DEBUG_BOUNDS"]}
 
 
-def _compile(src, extra, obj_dir=OBJ, part=""):
-    obj = os.path.join(obj_dir, os.path.basename(src) + part.replace("-D", ".").replace("=", "") + ".o")
-    extra = extra + ([part] if part else [])
+def _compile(src, extra, obj_dir=OBJ, part=()):
+    obj = os.path.join(obj_dir, os.path.basename(src) + "".join(part).replace("-D", ".").replace("=", "") + ".o")
+    extra = extra + list(part)
     cmd = [nvcc()] + ARCH + NVCC_FLAGS + extra + ["-c", src, "-o", obj]
     if src.endswith(".cpp"):
         cmd[1:1] = ["-x", "cu"]
@@ -79,7 +81,7 @@ def build(force=False, verbose=False, extra=(), variant=""):
     if not force and os.path.exists(lib_path) and os.path.getmtime(lib_path) >= _newest_input():
         return lib_path
     # the parts are the longest compilations: first
-    jobs = [(s, p) for s in sources() for p in PARTS.get(os.path.basename(s), [])] + [(s, "") for s in sources()]
+    jobs = [(s, p) for s in sources() for p in PARTS.get(os.path.basename(s), [])] + [(s, ()) for s in sources()]
     flags = list(extra) + VARIANT_FLAGS[variant]
     with cf.ThreadPoolExecutor(max_workers=min(len(jobs), os.cpu_count() or 4)) as ex:
         results = list(ex.map(lambda j: _compile(j[0], flags, obj_dir, j[1]), jobs))

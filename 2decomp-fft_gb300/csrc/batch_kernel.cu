@@ -180,13 +180,14 @@ int batch_tile_lines(int n, bool contiguous) {
 
 size_t batch_smem_bytes() {
   // largest tile: lines of every supported length, plus one padding line
-  long long best = 0;
+  size_t best = 0;
   for (int n : {32, 48, 64, 96, 128, 192, 256})
     for (int c = 0; c < 2; ++c) {
-      const long long e = fast_smem_entries(n, batch_tile_lines(n, c != 0) + 1);
-      if (e > best) best = e;
+      const int lines = batch_tile_lines(n, c != 0) + 1;
+      const size_t b = mixed_length(n) ? mixed_smem_bytes(mixed_r0(n), n / mixed_r0(n), lines) : (size_t)fast_smem_entries(n, lines) * sizeof(float2);
+      if (b > best) best = b;
     }
-  return (size_t)best * sizeof(float2);
+  return best;
 }
 
 cudaError_t launch_batch_f32(const BatchDesc* d_desc, const long long* d_prefix, int ndesc, int* d_sync,

@@ -84,6 +84,9 @@ struct AxisPlan {
   int radix[kMaxStages] = {0};
   int tpl = 1;        // threads per line
   int fast_e = 16;    // points per thread of the power-of-two kernel
+  int mixed = 0;          // FP32: second radix of the two-stage plan of
+                          // mixed_length(), 0 where it cannot run
+  bool plan_set = false;  // fast_e was asked for, not the default
   bool big = false;   // lines do not fit one shared-memory tile: the
                       // multi-kernel long-axis path (fft_long.cu)
   bool blue = false;  // a prime factor above kBluePrime: the chirp-z path
@@ -219,6 +222,14 @@ int upload_table(void** dst, const std::vector<double>& t, int prec) {
   return GBFFT_OK;
 }
 
+// Whether an FP32 axis runs its balanced plan (fft_gen.cuh): when asked for,
+// where the two-stage plan cannot run, and for 243 = 9 x 27, whose second stage
+// would leave two threads in three idle (243 x 400 x 384 x pass 66 us, two-stage
+// 93).  The other lengths are faster on two stages (figures at fft_mixed.cuh).
+bool uses_gen(const AxisPlan& p) {
+  return gen_length(p.n) && p.fast_e == gen_points(p.n) && (p.plan_set || p.n == 243 || !p.mixed);
+}
+
 // Radices of an axis's compile-time plan (power of two: fast_e points a
 // thread; balanced non-power-of-two plan when fast_e = gen_points(n); the
 // two-stage mixed-radix plan otherwise); empty when the axis has none.
@@ -226,10 +237,10 @@ std::vector<int> plan_radices(const AxisPlan& p) {
   std::vector<int> radices;
   if (fast_length(p.n)) {
     for (int s = 0; s < fast_nst(p.n, p.fast_e); ++s) radices.push_back(fast_radix(p.n, p.fast_e, s));
-  } else if (gen_length(p.n) && p.fast_e == gen_points(p.n)) {
+  } else if (uses_gen(p)) {
     for (int s = 0; gen_radix(p.n, s) > 0; ++s) radices.push_back(gen_radix(p.n, s));
-  } else if (mixed_length(p.n)) {
-    radices = {mixed_r0(p.n), p.n / mixed_r0(p.n)};
+  } else if (p.mixed) {
+    radices = {p.n / p.mixed, p.mixed};
   }
   return radices;
 }
@@ -789,20 +800,21 @@ int fast_lines_per_cta(int n, int prec, bool contiguous, long long nlines, int f
   return L;
 }
 
-// Fill the plan-dependent fields of a pass.
-// Lines per CTA for the mixed-radix kernel (R1 = n / mixed_r0(n) threads a
-// line, at most 256 threads a CTA).
-int mixed_lines_per_cta(int n, int prec, bool contiguous, long long nlines, int forced_L) {
-  const int tpl = n / mixed_r0(n);
-  if (forced_L > 0) return forced_L;
-  int L = contiguous ? 192 / tpl : 256 / tpl;
-  if (!contiguous) {
-    const int min_l = (int)(64 / (2 * prec));
-    if (L < min_l) L = min_l;
-  }
-  while (L > 1 && L * tpl > 256) --L;
-  while (L > 1 && (size_t)fast_smem_entries(n, L) * 2 * prec > 100 * 1024) --L;
-  if (L < 1) L = 1;
+// Lines per CTA for the two-stage kernel (tpl, the second radix, threads a
+// line, at most 256 threads a CTA).  Contiguous lines: about three warps, one
+// line from 25 threads a line on (r2c x passes of 24 M points, us: 900 points
+// 43.6 with one line, 49.7 with six; 225 points 45.5 with six, 47.2 with
+// twelve; 120 points 47.3 with eight, 49.3 with sixteen).  Strided tiles: a
+// power of two of lines, at least a 64-byte row segment (60 points, c2c y 36.9
+// with 16 lines, 40.3 with 24; r2c z 45.2 and 52.4).
+int mixed_lines_per_cta(int n, int tpl, bool contiguous, long long nlines, long long nv, int forced_L) {
+  if (forced_L > 0 && forced_L * tpl <= 256 && mixed_smem_bytes(n / tpl, tpl, forced_L) <= kFxMaxSmem) return forced_L;
+  int L = contiguous ? (tpl > 24 ? 1 : 96 / tpl) : 8;
+  if (!contiguous)
+    while (L < 32 && 2 * L * tpl <= 256) L *= 2;
+  // small grids: fewer lines a CTA until there are two CTAs per SM
+  const int min_l = contiguous ? 1 : 8;
+  while (L > min_l && ((nlines + L - 1) / L) * nv < 2LL * kSmsDefault) L = std::max(min_l, L / 2);
   if (L > 1 && nlines < L) L = (int)nlines;
   return L;
 }
@@ -879,7 +891,7 @@ void fill_plan(PassArgs& a, const AxisPlan& p, int prec, bool contiguous, int ki
     (void)kind;
     return;
   }
-  if (gen_length(p.n) && p.fast_e == gen_points(p.n)) {
+  if (uses_gen(p)) {
     a.n = p.n;
     a.nst = 0;
     a.tw = p.d_twf;
@@ -890,13 +902,13 @@ void fill_plan(PassArgs& a, const AxisPlan& p, int prec, bool contiguous, int ki
     a.last_fused = kind != K_R2C;
     return;
   }
-  if (mixed_length(p.n)) {
+  if (p.mixed) {
     a.n = p.n;
     a.nst = 0;
     a.tw = p.d_twf;
     a.fast = 2;
-    a.tpl = p.n / mixed_r0(p.n);
-    a.L = mixed_lines_per_cta(p.n, prec, contiguous, a.nlines, forced_L);
+    a.tpl = p.mixed;
+    a.L = mixed_lines_per_cta(p.n, p.mixed, contiguous, a.nlines, contiguous ? 1 : a.nv, forced_L);
     a.first_fused = 1;
     a.last_fused = kind != K_R2C;
     return;
@@ -1271,8 +1283,10 @@ int engine_init_host(gbfft_engine_s* e, int format, int nx, int ny, int nz, int 
     }
     if (gen_length(lens[d])) e->ax[d].fast_e = gen_points(lens[d]);
     if (fast_has_alt(lens[d]) && tune.e[d] > 0 && fast_e_ok(lens[d], tune.e[d])) e->ax[d].fast_e = tune.e[d];
-    if (gen_length(lens[d]) && (tune.e[d] == gen_points(lens[d]) || tune.e[d] == 2))
+    if (gen_length(lens[d]) && (tune.e[d] == gen_points(lens[d]) || tune.e[d] == 2)) {
       e->ax[d].fast_e = tune.e[d];
+      e->ax[d].plan_set = true;
+    }
     // FP64 lines of one tile: fixed point; small grids (under about 16 warps
     // per SM at 8 points a thread) take radix 4 and twice the threads
     if (prec == GBFFT_PREC_DOUBLE && !e->ax[d].big && fx_length(lens[d])) {
@@ -1280,9 +1294,12 @@ int engine_init_host(gbfft_engine_s* e, int format, int nx, int ny, int nz, int 
       e->ax[d].fx = fx_plan(lens[d], threads < 512.0 * kSmsDefault ? 4 : 10,
                            (double)(nx + 8) * ny < (double)(1 << 28));
     }
-    // FP32 lengths without a compile-time plan: the smooth-length kernel
-    if (prec == GBFFT_PREC_SINGLE && !e->ax[d].big && !fast_length(lens[d]) && !mixed_length(lens[d]) &&
-        !gen_length(lens[d]) && (double)(nx + 8) * ny < (double)(1 << 28))
+    // FP32: the two-stage plan where the length has one and rows lie below
+    // 2^28 elements apart; else the smooth-length kernel
+    const bool near = (double)(nx + 8) * ny < (double)(1 << 28);
+    if (prec == GBFFT_PREC_SINGLE && near && mixed_length(lens[d])) e->ax[d].mixed = lens[d] / mixed_r0(lens[d]);
+    if (prec == GBFFT_PREC_SINGLE && !e->ax[d].big && !fast_length(lens[d]) && !e->ax[d].mixed &&
+        !gen_length(lens[d]) && near)
       e->ax[d].fx = rt_plan(lens[d], (double)nx * ny * nz / 16 < 512.0 * kSmsDefault ? 10 : 16, false);
     if (form != GBFFT_FORM_PLAIN && split_length(lens[d])) e->ax[d].fast_e = 16;  // radix-16 stages for the tensor cores
   }
@@ -1690,6 +1707,11 @@ int gbfft_engine_set_profiling(gbfft_engine_t e, int enable) {
   return GBFFT_OK;
 }
 
+// Lengths whose tiles are checked against the two-stage kernel's limits; the
+// other lengths' against the general kernel's, and a tile the two-stage kernel
+// cannot run keeps the built-in one.
+static bool two_plans(int n) { return gen_length(n) || n == 48 || n == 96 || n == 192 || n == 210; }
+
 int gbfft_engine_set_tile(gbfft_engine_t e, int kind, int lines) {
   if (!valid_engine(e)) return fail(GBFFT_ERR_INVALID, "not an engine");
   if (kind < 0 || kind >= GBFFT_PASS_KINDS) return fail(GBFFT_ERR_INVALID, "bad pass kind");
@@ -1721,7 +1743,7 @@ int gbfft_engine_set_tile(gbfft_engine_t e, int kind, int lines) {
     e->tile_L[kind] = lines;
     return GBFFT_OK;
   }
-  if (mixed_length(p.n)) {
+  if (two_plans(p.n)) {
     const int tpl_m = p.n / mixed_r0(p.n);
     if (lines * tpl_m > 256) return fail(GBFFT_ERR_INVALID, "tile exceeds the kernel's thread limit");
     if ((size_t)fast_smem_entries(p.n, lines) * 2 * (size_t)e->prec > 200 * 1024)
@@ -1831,19 +1853,24 @@ int gbfft_engine_set_plan(gbfft_engine_t e, int axis, int points) {
       return fail(GBFFT_ERR_INVALID, "points per thread must be 32 or 16 (512 and 1024 points) or 16, 8, 4 "
                                      "(8: at most 256 points, 4: at most 128)");
   }
-  if (p.fast_e == points) return GBFFT_OK;
+  if (p.fast_e == points && (p.plan_set || !gen_length(p.n))) return GBFFT_OK;
   if (p.fx.nst) {  // FP64 passes in fixed point have one plan: only the setting is kept
+    if (p.fast_e == points) return GBFFT_OK;
     p.fast_e = points;
     for (int k = 0; k < GBFFT_PASS_KINDS; ++k) e->tile_L[k] = 0;
     return GBFFT_OK;
   }
   void* old = p.d_twf;
   const int old_e = p.fast_e;
+  const bool old_set = p.plan_set;
   p.fast_e = points;
+  p.plan_set = true;
   p.d_twf = nullptr;
-  int rc = upload_table(&p.d_twf, stage_twiddles(plan_radices(p)), e->prec);
+  const std::vector<int> radices = plan_radices(p);  // none where the general kernel runs
+  int rc = radices.empty() ? GBFFT_OK : upload_table(&p.d_twf, stage_twiddles(radices), e->prec);
   if (rc != GBFFT_OK) {
     p.fast_e = old_e;
+    p.plan_set = old_set;
     p.d_twf = old;
     return rc;
   }

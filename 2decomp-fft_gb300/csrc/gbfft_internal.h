@@ -266,8 +266,10 @@ __host__ __device__ constexpr int fast_radix(int n, int e, int s) {
 // kernel still run several CTAs per SM.
 constexpr int kFastMaxThreadsF32 = 1024;
 constexpr int kFastMaxThreadsF64 = 256;
-// Mixed-radix lengths with a compile-time-planned kernel (fft_mixed.cuh):
-// n = R0 * R1, R0 <= R1 <= 32, the most balanced such split.
+// Lengths with a compile-time two-stage plan (fft_mixed.cuh): n = R0 * R1,
+// R0 <= R1 <= 32, the most balanced such split, R1 at most 3 R0 (only R0 of
+// the R1 threads work in the second stage), of the primes up to 13 (a larger
+// prime's butterfly costs its square).
 __host__ __device__ constexpr int mixed_r0(int n) {
   int best = 0;
   for (int a = 2; a <= 32; ++a)
@@ -275,9 +277,21 @@ __host__ __device__ constexpr int mixed_r0(int n) {
   return best;
 }
 __host__ __device__ constexpr bool mixed_length(int n) {
-  return n == 48 || n == 96 || n == 192 || n == 210 || n == 243 || n == 270 || n == 360 ||
-         n == 384 || n == 400;
+  if (n < 33 || n > 1024 || (n & (n - 1)) == 0 || n > 3 * mixed_r0(n) * mixed_r0(n)) return false;
+  for (int p = 2; p <= 13; ++p)
+    while (n % p == 0) n /= p;
+  return n == 1;
 }
+// Shared memory of L lines: the exchange matrix with its odd pitch.
+__host__ __device__ constexpr size_t mixed_smem_bytes(int r0, int r1, int L) {
+  return (size_t)r1 * (size_t)(r0 | 1) * (size_t)L * 8;
+}
+// the second radices of these lengths (build.py's list)
+#define GBFFT_MIXED_R1S(X)                                                                                          \
+  X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16) X(18) X(20) X(21) X(22) X(24) X(25) X(26) X(27) X(28) \
+  X(30) X(32)
+template <int R1, int KIND>
+cudaError_t launch_mixed_part(bool contiguous, const PassArgs& a, cudaStream_t s);
 cudaError_t launch_mixed_f32(int kind, bool contiguous, const PassArgs& a, cudaStream_t s);
 // Non-power-of-two lengths with a balanced compile-time plan (fft_gen.cuh,
 // fast::GenPlan): E points a thread, n / E threads a line.
