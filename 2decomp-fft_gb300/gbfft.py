@@ -187,17 +187,19 @@ def tma_pass_count():
     return int(lib().gbfft_tma_pass_count())
 
 
+# Device addresses and streams as plain integers (every entry point declares
+# its pointer arguments): a small transform is bound by the host's calls.
 def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
 
 
 def _stream(stream):
     if stream is None:
         import torch
-        return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
     if isinstance(stream, int):
-        return ctypes.c_void_p(stream)
-    return ctypes.c_void_p(stream.cuda_stream)
+        return stream
+    return stream.cuda_stream
 
 
 def _int3(x):
