@@ -24,7 +24,7 @@ NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O2",
 
 # Sources compiled once more for each part (a define that selects the
 # instantiations of one object file), so that they compile in parallel.
-MIXED_R1 = [32, 30, 28, 27, 26, 25, 24, 22, 21, 20, 18, 16, 15, 14, 13, 12, 11, 10, 9, 8, 7, 6]
+MIXED_R1 = [32, 30, 28, 27, 26, 25, 24, 22, 21, 20, 18, 16, 15, 14, 13, 12, 11, 10, 9, 8, 7, 6, 5, 4]
 PARTS = {"fft_fxc.cu": [["-DGBFFT_FXC_PART=%d" % i] for i in range(40)],
          "mixed_f32.cu": [["-DGBFFT_MIXED_R1=%d" % r, "-DGBFFT_MIXED_KIND=%d" % k] for r in MIXED_R1 for k in range(3)]}
 

@@ -546,7 +546,8 @@ int upload_twiddles(AxisPlan& p, int prec) {
     p.fx.tw = p.d_fxtw;
     return rc;
   }
-  int rc = upload_table(&p.d_tw, twiddles(p.n), prec);
+  // an axis with a two-stage plan reads its stage-major table alone
+  int rc = p.mixed ? GBFFT_OK : upload_table(&p.d_tw, twiddles(p.n), prec);
   const std::vector<int> radices = plan_radices(p);
   if (rc == GBFFT_OK && !radices.empty()) rc = upload_table(&p.d_twf, stage_twiddles(radices), prec);
   if (rc == GBFFT_OK && p.blue) rc = upload_blue(p, prec);
@@ -780,8 +781,10 @@ int fast_lines_per_cta(int n, int prec, bool contiguous, long long nlines, int f
     // overlap their load, exchange and store phases
     L = tpl > 32 ? 1 : 128 / tpl;
   } else {
+    // 256 threads (256 points: c2c y pass of 24 M points 35.7 us, with 512
+    // threads 40.4; z r2c 41.3 and 43.5)
     const int min_l = (int)(64 / (2 * prec));
-    L = 512 / tpl;
+    L = 256 / tpl;
     if (L > 32) L = 32;
     if (L < min_l) L = min_l;
   }
@@ -1277,7 +1280,11 @@ int engine_init_host(gbfft_engine_s* e, int format, int nx, int ny, int nz, int 
       // short lines of a small grid: fewer points a thread until the pass
       // has about 16 warps per SM (lines of a full-grid pass: grid / n)
       const double lines = (double)nx * ny * nz / lens[d];
-      int pe = 16;
+      // contiguous FP32 lines: four or eight threads a line at least, for
+      // whole sectors a load (us a pass of 24 M points with 16 points a
+      // thread and so: 16 points r2c 136, 66; 32 points 78, 60; 64 points
+      // 58, 44, c2c x 37, 32; 128 points no gain)
+      int pe = d == 0 && prec == GBFFT_PREC_SINGLE ? (lens[d] <= 16 ? 4 : lens[d] <= 64 ? 8 : 16) : 16;
       while (pe > 4 && fast_e_ok(lens[d], pe / 2) && lines * (lens[d] / pe) < 512.0 * kSmsDefault) pe /= 2;
       e->ax[d].fast_e = pe;
     }

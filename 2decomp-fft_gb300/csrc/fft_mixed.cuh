@@ -9,13 +9,14 @@
 //            splits the two real lines' spectra).
 //
 // What bounds them is memory: two stages are one exchange, the fewest that
-// lines of 33 to 1024 points can have, the radices and strides are compile-time
+// lines of 12 to 1024 points can have, the radices and strides are compile-time
 // constants, and 20 to 32 points in flight a thread cover the latency.  Runtime
 // plans of radices up to 16 spend 1.2 to 2.2 times as long in index arithmetic
 // and in more exchanges.  Passes of 24 M points, us (28 at the copy rate), and in
-// brackets the runtime plan (225, 900) or the balanced three-stage one (360):
+// brackets the runtime plan (24, 225, 900) or the balanced three-stage one (360):
 //   225  r2c x 47 (82)  c2r x 47 (84)  r2c z 43 (52)  c2r z 39 (72)  c2c y 38 (46)
 //   360  r2c x 49 (73)  c2r x 49 (70)  r2c z 46 (76)  c2r z 40 (64)  c2c y 40 (73)
+//   24   r2c x 54 (68)  c2r x 55 (79)  r2c z 45 (45)  c2r z 43 (58)  c2c y 36 (41)
 //   900  r2c x 43 (93)  c2r x 44 (105) r2c z 53 (89)  c2r z 49 (126) c2c y 48 (81)
 // The rel-L2 error against 64 bits is on average 0.98 of the plans' before (68
 // random boxes).

@@ -277,7 +277,7 @@ __host__ __device__ constexpr int mixed_r0(int n) {
   return best;
 }
 __host__ __device__ constexpr bool mixed_length(int n) {
-  if (n < 33 || n > 1024 || (n & (n - 1)) == 0 || n > 3 * mixed_r0(n) * mixed_r0(n)) return false;
+  if (n < 12 || n > 1024 || (n & (n - 1)) == 0 || n > 3 * mixed_r0(n) * mixed_r0(n)) return false;
   for (int p = 2; p <= 13; ++p)
     while (n % p == 0) n /= p;
   return n == 1;
@@ -288,8 +288,8 @@ __host__ __device__ constexpr size_t mixed_smem_bytes(int r0, int r1, int L) {
 }
 // the second radices of these lengths (build.py's list)
 #define GBFFT_MIXED_R1S(X)                                                                                          \
-  X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16) X(18) X(20) X(21) X(22) X(24) X(25) X(26) X(27) X(28) \
-  X(30) X(32)
+  X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16) X(18) X(20) X(21) X(22) X(24) X(25) X(26)  \
+  X(27) X(28) X(30) X(32)
 template <int R1, int KIND>
 cudaError_t launch_mixed_part(bool contiguous, const PassArgs& a, cudaStream_t s);
 cudaError_t launch_mixed_f32(int kind, bool contiguous, const PassArgs& a, cudaStream_t s);
