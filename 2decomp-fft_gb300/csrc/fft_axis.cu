@@ -14,8 +14,9 @@
 //  * This file holds the runtime-planned kernel, which handles any length up
 //    to kMaxN: lines are loaded into shared memory, each stage ping-pongs
 //    between two shared buffers, and the result is stored from the last one.
-//    Power-of-two lengths run the compile-time-planned kernels of
-//    fft_fast.cu instead.
+//    FP32 powers of two and smooth lengths run compile-time plans
+//    (fft_fast.cuh, fft_mixed.cuh) or the smooth-length kernel (fft_rt.cuh)
+//    instead, and FP64 lines the fixed-point kernels (fft_fx.cuh).
 //  * Along y and z the lanes of a warp walk neighbouring x positions, so the
 //    strided transforms still read and write contiguous x segments.
 //  * r2c/c2r carry two real lines in one complex line (z = a + i b) and

@@ -348,7 +348,10 @@ int gbfft_tune_cache_path(const char* path); /* NULL = default, "" = none */
  * points a thread is one warp); 243, 270, 360, 384 or 400 points with the
  * balanced plan (points = 9, 30, 30, 24, 20: 9 9 3, 15 6 3, 10 6 6, 8 8 6,
  * 20 20) or points = 2 for the two-stage plan n = R0 R1.  Resets the tile
- * shapes.  Waits for the device. */
+ * shapes.  Waits for the device.  Unless asked, axes of 270, 360, 384 and 400
+ * points run the two-stage plan (the query below then reports the balanced
+ * plan's points).  FP64 axes whose lines run in fixed point have one plan: the
+ * setting is kept and reported, but changes nothing. */
 int gbfft_engine_set_plan(gbfft_engine_t engine, int axis, int points);
 /* Current fusion switch, lines per CTA per pass kind (GBFFT_PASS_KINDS
  * ints, 0 = built-in) and points per thread per axis (3 ints, 0 = the axis
