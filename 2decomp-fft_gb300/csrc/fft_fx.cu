@@ -128,10 +128,10 @@ __global__ void __launch_bounds__(kFxMaxThreads) fx_pass_kernel(const __grid_con
   I2* buf0 = reinterpret_cast<I2*>(smem_raw);
   I2* buf1 = buf0 + (e + (e >> 4) + 1);
   int* smax = reinterpret_cast<int*>(buf1 + (e + (e >> 4) + 1));
-  unsigned* ssum = reinterpret_cast<unsigned*>(smax + a.L);
+  unsigned* ssum = reinterpret_cast<unsigned*>(smax + 2 * a.L);
   {
     const int threads = blockDim.x * blockDim.y;
-    for (int i = threadIdx.x + threadIdx.y * blockDim.x; i < 2 * a.L; i += threads) smax[i] = 0;
+    for (int i = threadIdx.x + threadIdx.y * blockDim.x; i < 4 * a.L; i += threads) smax[i] = 0;
   }
   __syncthreads();
 
@@ -151,29 +151,27 @@ __global__ void __launch_bounds__(kFxMaxThreads) fx_pass_kernel(const __grid_con
       v[i] = n < cnt ? c.gload_raw(n) : make_double2(0, 0);
     }
   }
-  fx::Scale sc;
-  if (!sc.find<J * W>(v, &smax[c.line], &ssum[c.line])) {
+  fx::PassScale<KIND> sc;
+  if (!sc.template find<J * W>(v, &smax[2 * c.line], &ssum[2 * c.line])) {
     fx::fallback<KIND, CONTIG>(a, reinterpret_cast<double2*>(smem_raw));
     return;
   }
-  constexpr int X = KIND == K_C2R ? 1 : 0;  // a point combines two values
-  int top = -1021 + X;
 #pragma unroll 1
-  for (int s = 0; s < p.nst; ++s) top = max(top, sc.bound(p.lg[s], X) - p.shift[s]);
+  for (int s = 0; s < p.nst; ++s) sc.stage(p.lg[s], p.shift[s]);
   // r2c adds two values that no twiddle has halved
-  if (KIND == K_R2C && p.shift[p.nst - 1] == 0) ++top;
-  const int sh = sc.shift(top);
-  int adj = (sc.em - 62 + top + p.shift[p.nst - 1]) << 20;  // exponent of a result's unit, in a high word
-
+  if (KIND == K_R2C && p.shift[p.nst - 1] == 0) sc.headroom();
+  const int sa = sc.shift_a(), sb = sc.shift_b();
   // backward: conjugated on the way in (c2r: by its combination) and out
   const int flip = c.inverse ? (int)0x80000000 : 0;
+  const fx::Back<KIND> out = sc.back(p.shift[p.nst - 1], flip);
+
   if constexpr (KIND == K_C2R) {
 #pragma unroll
     for (int i = 0; i < J; ++i) {
       const int j = t + i * tpl;
       if (j < cnt) {
-        const ll ax = fx::to_fixed(v[2 * i].x, sh), ay = fx::to_fixed(v[2 * i].y, sh);
-        const ll bx = fx::to_fixed(v[2 * i + 1].x, sh), by = fx::to_fixed(v[2 * i + 1].y, sh);
+        const ll ax = fx::to_fixed(v[2 * i].x, sa), ay = fx::to_fixed(v[2 * i].y, sa);
+        const ll bx = fx::to_fixed(v[2 * i + 1].x, sb), by = fx::to_fixed(v[2 * i + 1].y, sb);
         // z = x1 + i x2, conjugated for the inverse-by-conjugation
         buf0[c.sidx(j)] = fx::mk(ax - by, -(ay + bx));
         if (j > 0 && 2 * j < N) buf0[c.sidx(N - j)] = fx::mk(ax + by, ay - bx);
@@ -183,7 +181,7 @@ __global__ void __launch_bounds__(kFxMaxThreads) fx_pass_kernel(const __grid_con
 #pragma unroll
     for (int i = 0; i < J; ++i) {
       const int n = t + i * tpl;
-      if (n < N) buf0[c.sidx(n)] = fx::mk(fx::to_fixed(v[i].x, sh), fx::to_fixed(v[i].y, sh, flip));
+      if (n < N) buf0[c.sidx(n)] = fx::mk(fx::to_fixed(v[i].x, sa), fx::to_fixed(v[i].y, sb, flip));
     }
   }
   __syncthreads();
@@ -191,19 +189,15 @@ __global__ void __launch_bounds__(kFxMaxThreads) fx_pass_kernel(const __grid_con
   const I2* A = fx_stages(c, p, buf0, buf1);
 
   if constexpr (KIND == K_R2C) {
-    adj -= 1 << 20;  // the halves of X1 = (Z_k + conj Z_{n-k}) / 2, X2 = (Z_k - conj Z_{n-k}) / 2i
 #pragma unroll 1
     for (int k = t; 2 * k <= N; k += tpl) {
       const I2 zk = A[c.sidx(k)], zm = A[c.sidx(k == 0 ? 0 : N - k)];
-      c.put_half(0, k, make_double2(fx::to_double(zk.x + zm.x, adj), fx::to_double(zk.y - zm.y, adj)));
-      c.put_half(1, k, make_double2(fx::to_double(zk.y + zm.y, adj), fx::to_double(zm.x - zk.x, adj)));
+      c.put_half(0, k, out.half_a(zk, zm));
+      c.put_half(1, k, out.half_b(zk, zm));
     }
   } else {
 #pragma unroll 1
-    for (int n = t; n < N; n += tpl) {
-      const I2 z = A[c.sidx(n)];
-      c.gstore_raw(n, make_double2(fx::to_double(z.x, adj), fx::to_double(z.y, adj, flip)));
-    }
+    for (int n = t; n < N; n += tpl) c.gstore_raw(n, out.point(A[c.sidx(n)]));
   }
 }
 
@@ -252,8 +246,8 @@ __global__ void __launch_bounds__(kFxMaxThreads) fx_r2r_kernel(const __grid_cons
     const int j = t + i * tpl;
     x[i] = j < cnt ? ln.element(j) : make_double2(0, 0);
   }
-  r2r::PairScale sc;
-  if (!sc.find<kE>(x, &smax[2 * c.line], &ssum[2 * c.line], ln.single)) {
+  fx::PairScale sc;
+  if (!sc.find<false, kE>(x, &smax[2 * c.line], &ssum[2 * c.line], ln.single)) {
     r2r::fallback<CONTIG>(a, reinterpret_cast<double2*>(smem_raw));
     return;
   }

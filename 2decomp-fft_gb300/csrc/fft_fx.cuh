@@ -6,8 +6,9 @@
 // transform exceeds the sum of the moduli of its inputs, so a line can be
 // transformed in integers that share one power-of-two scale, chosen from
 // that sum: 64 bits for numbers that hold 53, of which at most a few go to
-// headroom.  The scale is the line's own (never a neighbour's), so a small
-// line next to a large one keeps all its digits.
+// headroom.  The scale is the line's own (never a neighbour's; of two real
+// lines that share a complex one, each its own), so a small line next to a
+// large one keeps all its digits.
 //
 // Formats: a value is a signed 64-bit integer v, |v| < 2^62.  Table twiddles
 // are Q62 (w 2^62) and multiplying by one divides by 2, in the compile-time
@@ -425,6 +426,63 @@ struct Scale {
   __device__ __forceinline__ double out(ll v, int adj) const { return m == 0 ? 0.0 : to_double(v, adj); }
 };
 
+// The scales of the two real lines a, b that a complex line a + i b carries,
+// each its own (their transforms separate exactly, so a small line next to a
+// large one keeps its digits); of one line alone (`single`), the same twice.
+struct PairScale {
+  Scale a, b;
+  // smax, ssum: two words each, at zero.  HALVES: x[2 i], x[2 i + 1] are
+  // points of the lines' half spectra, else x[i] holds a point of a and b.
+  template <bool HALVES, int Q>
+  __device__ __forceinline__ bool find(const double2 (&x)[Q], int* smax, unsigned* ssum, bool single = false) {
+    constexpr int S = HALVES ? 2 : 1;
+    auto ha = [&](int i) { return HALVES ? max_hi(x[i]) : abs_hi(x[i].x); };
+    auto hb = [&](int i) { return HALVES ? max_hi(x[i + 1]) : abs_hi(x[i].y); };
+    int ma = 0, mb = 0;
+#pragma unroll
+    for (int i = 0; i < Q; i += S) {
+      ma = max(ma, ha(i));
+      mb = max(mb, hb(i));
+    }
+    if (single) ma = mb = max(ma, mb);
+    atomicMax(smax, ma);
+    atomicMax(smax + 1, mb);
+    __syncthreads();
+    a.m = smax[0];
+    b.m = smax[1];
+    a.em = a.m >> 20;
+    b.em = b.m >> 20;
+    float sa = 0, sb = 0;
+    const int ba = share_base(a.em), bb = share_base(b.em);
+#pragma unroll
+    for (int i = 0; i < Q; i += S) {
+      sa += share(ha(i), ba);
+      sb += share(hb(i), bb);
+    }
+    if (single) sa = sb = sa + sb;
+    atomicAdd(ssum, share_units(sa, 2 * Q));
+    atomicAdd(ssum + 1, share_units(sb, 2 * Q));
+    int bad = outside(a) | outside(b);
+    if (a.m == 0 || b.m == 0) {  // all zero, or subnormals below 2^-1042
+#pragma unroll
+      for (int i = 0; i < Q; i += S) {
+        if (a.m == 0) bad |= HALVES ? any_lo(x[i]) : __double2loint(x[i].x);
+        if (b.m == 0) bad |= HALVES ? any_lo(x[i + 1]) : __double2loint(x[i].y);
+      }
+    }
+    if (__syncthreads_or(bad)) return false;
+    // a complex point's modulus is at most sqrt 2 times its larger component;
+    // one bit for the other line: the moduli of a + i b sum to at most both
+    const unsigned ta = ssum[0], tb = ssum[1];
+    a.es = 33 - __clz((int)(HALVES ? ta + (ta >> 1) : ta)) - 1040;
+    b.es = 33 - __clz((int)(HALVES ? tb + (tb >> 1) : tb)) - 1040;
+    return true;
+  }
+  __device__ __forceinline__ static int outside(const Scale& s) {
+    return s.m != 0 && (s.em < kMinExp || s.em > kMaxExp);
+  }
+};
+
 // x as an integer, rounded: 61 mantissa bits shifted right by sh - e (not
 // negative).  One bit more is kept until the sign is in: w and ~w become
 // w + 1 and -w, whose halves are x and -x rounded.  (Cutting the bits off
@@ -440,6 +498,64 @@ __device__ __forceinline__ ll to_fixed(double x, int sh, int flip = 0) {
   const ll m = (ll)(((unsigned long long)(mh ^ (unsigned)sg) << 32) | ((l << 9) ^ (unsigned)sg));
   return ((m >> s) + 1) >> 1;
 }
+// From the integers of a pass's complex line back to doubles: the exponent of
+// each line's unit, in a high word, and the sign of the imaginary part.  A
+// zero line that shares its transform is zero whatever the other's rounding
+// left there.
+template <int KIND>
+struct Back {
+  int adj_a, adj_b, flip;
+  bool za, zb;
+  // c2c, c2r: a point (c2r: of both lines)
+  __device__ __forceinline__ double2 point(I2 v) const {
+    return make_double2(za ? 0.0 : to_double(v.x, adj_a), zb ? 0.0 : to_double(v.y, adj_b, flip));
+  }
+  // r2c: points of the two half spectra, X1 = (Z_k + conj Z_{n-k}) / 2,
+  // X2 = (Z_k - conj Z_{n-k}) / 2i, from Z_k and Z_{n-k}
+  __device__ __forceinline__ double2 half_a(I2 zk, I2 zm) const { return half(zk.x + zm.x, zk.y - zm.y, adj_a, za); }
+  __device__ __forceinline__ double2 half_b(I2 zk, I2 zm) const { return half(zk.y + zm.y, zm.x - zk.x, adj_b, zb); }
+  __device__ __forceinline__ static double2 half(ll x, ll y, int adj, bool zero) {
+    const int h = adj - (1 << 20);
+    return zero ? make_double2(0.0, 0.0) : make_double2(to_double(x, h), to_double(y, h));
+  }
+};
+
+// The scale of a pass's complex line and the way back from it: one scale for
+// c2c, one for each of the two real lines of r2c and c2r.
+template <int KIND>
+struct PassScale {
+  static constexpr int X = KIND == K_C2R ? 1 : 0;  // a point combines two values
+  PairScale p;  // c2c: p.a alone
+  int ta = -1021 + X, tb = -1021 + X;
+  // smax, ssum: two words each, at zero
+  template <int Q>
+  __device__ __forceinline__ bool find(const double2 (&x)[Q], int* smax, unsigned* ssum) {
+    if constexpr (KIND == K_C2C) return p.a.find<Q>(x, smax, ssum);
+    else return p.find<KIND == K_C2R, Q>(x, smax, ssum);
+  }
+  // stage of at most 2^lg summed inputs, divided by 2^shift so far
+  __device__ __forceinline__ void stage(int lg, int shift) {
+    ta = max(ta, p.a.bound(lg, X) - shift);
+    if constexpr (KIND != K_C2C) tb = max(tb, p.b.bound(lg, X) - shift);
+  }
+  __device__ __forceinline__ void headroom() {
+    ++ta;
+    ++tb;
+  }
+  // right shifts of to_fixed for the two lines (c2c: components)
+  __device__ __forceinline__ int shift_a() const { return p.a.shift(ta); }
+  __device__ __forceinline__ int shift_b() const { return KIND == K_C2C ? p.a.shift(ta) : p.b.shift(tb); }
+  __device__ __forceinline__ Back<KIND> back(int shift, int flip) const {
+    Back<KIND> r;
+    r.adj_a = (p.a.em - 62 + ta + shift) << 20;
+    r.adj_b = KIND == K_C2C ? r.adj_a : (p.b.em - 62 + tb + shift) << 20;
+    r.flip = flip;
+    r.za = KIND != K_C2C && p.a.m == 0;
+    r.zb = KIND != K_C2C && p.b.m == 0;
+    return r;
+  }
+};
+
 // The lines of a CTA that fixed point does not take, in FP64: as many lines
 // at a time as two buffers of the CTA's shared memory hold.
 template <int KIND, bool CONTIG>

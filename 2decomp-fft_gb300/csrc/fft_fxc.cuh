@@ -113,9 +113,9 @@ struct Io {
 };
 
 // The stages from S on.  KIND K_R2C: the last one leaves its outputs in Sm.
-template <class P, int S, bool FROM_SMEM, int KIND, bool CONTIG, class Out>
+template <class P, int S, bool FROM_SMEM, int KIND, bool CONTIG, class Out, class Bk>
 __device__ __forceinline__ void run(const Out& io, int t, I2* Sm, const Slots<P, CONTIG>& slot, const W4* __restrict__ tw,
-                                    I2 (&v)[P::points()], int adj, int flip) {
+                                    I2 (&v)[P::points()], const Bk& back) {
   constexpr int R = P::radix(S), NS = P::ns(S), NB = P::N / R, MB = P::mb(S), TPL = P::TPL;
   constexpr bool LAST = S == P::NST - 1;
   if constexpr (FROM_SMEM) {
@@ -146,8 +146,7 @@ __device__ __forceinline__ void run(const Out& io, int t, I2* Sm, const Slots<P,
       const int b = t + m * TPL;
       if ((NB % TPL != 0 && b >= NB)) break;
 #pragma unroll
-      for (int r = 0; r < R; ++r)
-        io.store(m * TPL + r * NS, make_double2(to_double(v[m * R + r].x, adj), to_double(v[m * R + r].y, adj, flip)));
+      for (int r = 0; r < R; ++r) io.store(m * TPL + r * NS, back.point(v[m * R + r]));
     }
   } else {
     if constexpr (FROM_SMEM) __syncthreads();  // every point read before the outputs overwrite them
@@ -160,7 +159,7 @@ __device__ __forceinline__ void run(const Out& io, int t, I2* Sm, const Slots<P,
       for (int r = 0; r < R; ++r) Sm[slot(base + r * NS)] = v[m * R + r];
     }
     __syncthreads();
-    if constexpr (!LAST) run<P, S + 1, true, KIND, CONTIG>(io, t, Sm, slot, tw, v, adj, flip);
+    if constexpr (!LAST) run<P, S + 1, true, KIND, CONTIG>(io, t, Sm, slot, tw, v, back);
   }
 }
 
@@ -186,9 +185,9 @@ __global__ void __launch_bounds__(fxc_max_threads(P::TPL), min_ctas<P>())
   slot.base = CONTIG ? c.line * Slots<P, CONTIG>::kLine : c.line;
   slot.L = L;
   // the lines' scale words, behind the exchange buffer
-  int* smax = reinterpret_cast<int*>(smem_raw + fxc_smem_bytes(N, L) - (size_t)L * 8);
-  unsigned* ssum = reinterpret_cast<unsigned*>(smax + L);
-  for (int i = threadIdx.x + threadIdx.y * blockDim.x; i < 2 * L; i += blockDim.x * blockDim.y) smax[i] = 0;
+  int* smax = reinterpret_cast<int*>(smem_raw + fxc_smem_bytes(N, L) - (size_t)L * 16);
+  unsigned* ssum = reinterpret_cast<unsigned*>(smax + 2 * L);
+  for (int i = threadIdx.x + threadIdx.y * blockDim.x; i < 4 * L; i += blockDim.x * blockDim.y) smax[i] = 0;
   __syncthreads();
 
   // 1. load: c2r both half spectra (point j in x[2 i], x[2 i + 1]), else the
@@ -215,21 +214,19 @@ __global__ void __launch_bounds__(fxc_max_threads(P::TPL), min_ctas<P>())
     }
   }
   // 2. the line's scale
-  Scale sc;
-  if (!sc.find<Q>(x, &smax[c.line], &ssum[c.line])) {
+  PassScale<KIND> sc;
+  if (!sc.template find<Q>(x, &smax[2 * c.line], &ssum[2 * c.line])) {
     fallback<KIND, CONTIG>(a, reinterpret_cast<double2*>(smem_raw));
     return;
   }
-  constexpr int X = KIND == K_C2R ? 1 : 0;  // a point combines two values
-  int top = -1021 + X;
 #pragma unroll
-  for (int s = 0; s < P::NST; ++s) top = max(top, sc.bound(P::lg(s), X) - P::shift(s));
+  for (int s = 0; s < P::NST; ++s) sc.stage(P::lg(s), P::shift(s));
   // r2c adds two values that no twiddle has halved
-  if (KIND == K_R2C && P::NST == 1) ++top;
-  const int sh = sc.shift(top);
-  int adj = (sc.em - 62 + top + P::shift(P::NST - 1)) << 20;
+  if (KIND == K_R2C && P::NST == 1) sc.headroom();
+  const int sa = sc.shift_a(), sb = sc.shift_b();
   // backward c2c: conjugated on the way in and out (c2r: out)
   const int flip_in = KIND == K_C2C && c.inverse ? (int)0x80000000 : 0;
+  const Back<KIND> back = sc.back(P::shift(P::NST - 1), KIND == K_C2R ? (int)0x80000000 : flip_in);
   // 3. integers, and the stages
   I2 v[E];
   if constexpr (KIND == K_C2R) {
@@ -237,8 +234,8 @@ __global__ void __launch_bounds__(fxc_max_threads(P::TPL), min_ctas<P>())
     for (int i = 0; i < J; ++i) {
       const int j = t + i * TPL;
       if (j < H) {
-        const ll ax = to_fixed(x[2 * i].x, sh), ay = to_fixed(x[2 * i].y, sh);
-        const ll bx = to_fixed(x[2 * i + 1].x, sh), by = to_fixed(x[2 * i + 1].y, sh);
+        const ll ax = to_fixed(x[2 * i].x, sa), ay = to_fixed(x[2 * i].y, sa);
+        const ll bx = to_fixed(x[2 * i + 1].x, sb), by = to_fixed(x[2 * i + 1].y, sb);
         // z = x1 + i x2, conjugated for the inverse-by-conjugation
         Sm[slot(j)] = mk(ax - by, -(ay + bx));
         if (j > 0 && 2 * j < N) Sm[slot(N - j)] = mk(ax + by, ay - bx);
@@ -247,19 +244,18 @@ __global__ void __launch_bounds__(fxc_max_threads(P::TPL), min_ctas<P>())
     __syncthreads();
   } else {
 #pragma unroll
-    for (int i = 0; i < Q; ++i) v[i] = mk(to_fixed(x[i].x, sh), to_fixed(x[i].y, sh, flip_in));
+    for (int i = 0; i < Q; ++i) v[i] = mk(to_fixed(x[i].x, sa), to_fixed(x[i].y, sb, flip_in));
   }
-  run<P, 0, KIND == K_C2R, KIND, CONTIG>(io, t, Sm, slot, tw, v, adj, KIND == K_C2R ? (int)0x80000000 : flip_in);
+  run<P, 0, KIND == K_C2R, KIND, CONTIG>(io, t, Sm, slot, tw, v, back);
   if constexpr (KIND == K_R2C) {
-    adj -= 1 << 20;  // the halves of X1 = (Z_k + conj Z_{n-k}) / 2, X2 = (Z_k - conj Z_{n-k}) / 2i
     constexpr int K = (H + TPL - 1) / TPL;
 #pragma unroll
     for (int i = 0; i < K; ++i) {
       const int k = t + i * TPL;
       if (k < H) {
         const I2 zk = Sm[slot(k)], zm = Sm[slot(k == 0 ? 0 : N - k)];
-        io.put_half(0, i * TPL, make_double2(to_double(zk.x + zm.x, adj), to_double(zk.y - zm.y, adj)));
-        io.put_half(1, i * TPL, make_double2(to_double(zk.y + zm.y, adj), to_double(zm.x - zk.x, adj)));
+        io.put_half(0, i * TPL, back.half_a(zk, zm));
+        io.put_half(1, i * TPL, back.half_b(zk, zm));
       }
     }
   }
@@ -289,8 +285,8 @@ __global__ void __launch_bounds__(fxc_max_threads(P::TPL), min_ctas<P>())
     const int j = t + i * TPL;
     x[i] = j < cnt ? ln.element(j) : make_double2(0, 0);
   }
-  r2r::PairScale sc;
-  if (!sc.find<Q>(x, &smax[2 * line], &ssum[2 * line], ln.single)) {
+  PairScale sc;
+  if (!sc.find<false, Q>(x, &smax[2 * line], &ssum[2 * line], ln.single)) {
     r2r::fallback<CONTIG>(a, reinterpret_cast<double2*>(smem_raw));
     return;
   }
@@ -319,7 +315,7 @@ __global__ void __launch_bounds__(fxc_max_threads(P::TPL), min_ctas<P>())
     __syncthreads();
   }
   I2 v[P::points()];
-  run<P, 0, true, K_R2C, CONTIG>(ln, t, Sm, slot, tw, v, 0, 0);
+  run<P, 0, true, K_R2C, CONTIG>(ln, t, Sm, slot, tw, v, 0);
 #pragma unroll 1
   for (int k = t; k < mp.steps(); k += TPL)
     mp.finish(

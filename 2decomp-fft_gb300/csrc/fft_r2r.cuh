@@ -255,57 +255,6 @@ struct Lines {
 };
 __device__ __forceinline__ int elements(int kind, int n) { return single_line(kind, n) ? n / 2 : n; }
 
-// The scales of a complex line's two real lines, each its own (their
-// transforms separate exactly, so a small line next to a large one keeps its
-// digits); of one line alone, the same twice.
-struct PairScale {
-  fx::Scale a, b;
-  // smax, ssum: two words each, at zero
-  template <int Q>
-  __device__ __forceinline__ bool find(const double2 (&x)[Q], int* smax, unsigned* ssum, bool single) {
-    int ma = 0, mb = 0;
-#pragma unroll
-    for (int i = 0; i < Q; ++i) {
-      ma = max(ma, fx::abs_hi(x[i].x));
-      mb = max(mb, fx::abs_hi(x[i].y));
-    }
-    if (single) ma = mb = max(ma, mb);
-    atomicMax(smax, ma);
-    atomicMax(smax + 1, mb);
-    __syncthreads();
-    a.m = smax[0];
-    b.m = smax[1];
-    a.em = a.m >> 20;
-    b.em = b.m >> 20;
-    float sa = 0, sb = 0;
-    const int ba = fx::share_base(a.em), bb = fx::share_base(b.em);
-#pragma unroll
-    for (int i = 0; i < Q; ++i) {
-      sa += fx::share(fx::abs_hi(x[i].x), ba);
-      sb += fx::share(fx::abs_hi(x[i].y), bb);
-    }
-    if (single) sa = sb = sa + sb;
-    atomicAdd(ssum, fx::share_units(sa, 2 * Q));
-    atomicAdd(ssum + 1, fx::share_units(sb, 2 * Q));
-    int bad = outside(a) | outside(b);
-    if (a.m == 0 || b.m == 0) {  // all zero, or subnormals below 2^-1042
-#pragma unroll
-      for (int i = 0; i < Q; ++i) {
-        if (a.m == 0) bad |= __double2loint(x[i].x);
-        if (b.m == 0) bad |= __double2loint(x[i].y);
-      }
-    }
-    if (__syncthreads_or(bad)) return false;
-    // one bit for the other line: the moduli of a + i b sum to at most both
-    a.es = 33 - __clz((int)ssum[0]) - 1040;
-    b.es = 33 - __clz((int)ssum[1]) - 1040;
-    return true;
-  }
-  __device__ __forceinline__ static int outside(const fx::Scale& s) {
-    return s.m != 0 && (s.em < fx::kMinExp || s.em > fx::kMaxExp);
-  }
-};
-
 // Shared-memory slots of a runtime-planned tile (LineCtx's layout).
 template <class Ctx>
 struct CtxSlot {

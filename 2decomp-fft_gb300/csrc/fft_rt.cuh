@@ -91,15 +91,17 @@ struct Slots {
   }
 };
 
-// How a result leaves the arithmetic.
-template <class A>
-struct Out {
-  int adj, flip;
-  __device__ __forceinline__ float2 operator()(float2 v) const {
+// How a result leaves FP32 (fixed point: fx::Back).
+struct Turn {
+  int flip;
+  __device__ __forceinline__ float2 point(float2 v) const {
     return make_float2(v.x, __int_as_float(__float_as_int(v.y) ^ flip));
   }
-  __device__ __forceinline__ double2 operator()(fx::I2 v) const {
-    return make_double2(fx::to_double(v.x, adj), fx::to_double(v.y, adj, flip));
+  __device__ __forceinline__ float2 half_a(float2 zk, float2 zm) const {
+    return make_float2((zk.x + zm.x) * 0.5f, (zk.y - zm.y) * 0.5f);
+  }
+  __device__ __forceinline__ float2 half_b(float2 zk, float2 zm) const {
+    return make_float2((zk.y + zm.y) * 0.5f, (zm.x - zk.x) * 0.5f);
   }
 };
 
@@ -124,7 +126,8 @@ __global__ void __launch_bounds__(rt_threads(sizeof(typename A::T)), 2) rt_pass_
   slot.base = CONTIG ? c.line * (N + (N >> A::kPadShift) + 1) : c.line;
   const W* tw = reinterpret_cast<const W*>(p.tw);
   const int back = KIND == K_C2R || (KIND == K_C2C && c.inverse) ? (int)0x80000000 : 0;
-  Out<A> out{0, back};
+  std::conditional_t<A::kFixed, fx::Back<KIND>, Turn> out;
+  out.flip = back;
 
   // the points of butterfly t of the first stage (c2r: the half spectra,
   // points t, t + tpl, ... of both)
@@ -145,29 +148,27 @@ __global__ void __launch_bounds__(rt_threads(sizeof(typename A::T)), 2) rt_pass_
   }
   C v[MR];
   if constexpr (A::kFixed) {
-    int* smax = reinterpret_cast<int*>(smem_raw + rt_smem_bytes(8, N, a.L, p.nst) - (size_t)a.L * 8);
-    unsigned* ssum = reinterpret_cast<unsigned*>(smax + a.L);
+    int* smax = reinterpret_cast<int*>(smem_raw + rt_smem_bytes(8, N, a.L, p.nst) - (size_t)a.L * 16);
+    unsigned* ssum = reinterpret_cast<unsigned*>(smax + 2 * a.L);
     const int threads = blockDim.x * blockDim.y;
-    for (int i = threadIdx.x + threadIdx.y * blockDim.x; i < 2 * a.L; i += threads) smax[i] = 0;
+    for (int i = threadIdx.x + threadIdx.y * blockDim.x; i < 4 * a.L; i += threads) smax[i] = 0;
     __syncthreads();
-    fx::Scale sc;
-    if (!sc.template find<Q>(x, &smax[c.line], &ssum[c.line])) {
+    fx::PassScale<KIND> sc;
+    if (!sc.template find<Q>(x, &smax[2 * c.line], &ssum[2 * c.line])) {
       fx::fallback<KIND, CONTIG>(a, reinterpret_cast<double2*>(smem_raw));
       return;
     }
-    constexpr int X = KIND == K_C2R ? 1 : 0;  // a point combines two values
-    int top = -1021 + X;
 #pragma unroll 1
-    for (int s = 0; s <= last; ++s) top = max(top, sc.bound(p.lg[s], X) - p.shift[s]);
-    const int sh = sc.shift(top);
-    out.adj = (sc.em - 62 + top + p.shift[last]) << 20;
+    for (int s = 0; s <= last; ++s) sc.stage(p.lg[s], p.shift[s]);
+    const int sa = sc.shift_a(), sb = sc.shift_b();
+    out = sc.back(p.shift[last], back);
     if constexpr (KIND == K_C2R) {
 #pragma unroll
       for (int i = 0; i < Q / 2; ++i) {
         const int j = t + i * tpl;
         if (j < h) {
-          const fx::ll ax = fx::to_fixed(x[2 * i].x, sh), ay = fx::to_fixed(x[2 * i].y, sh);
-          const fx::ll bx = fx::to_fixed(x[2 * i + 1].x, sh), by = fx::to_fixed(x[2 * i + 1].y, sh);
+          const fx::ll ax = fx::to_fixed(x[2 * i].x, sa), ay = fx::to_fixed(x[2 * i].y, sa);
+          const fx::ll bx = fx::to_fixed(x[2 * i + 1].x, sb), by = fx::to_fixed(x[2 * i + 1].y, sb);
           // z = x1 + i x2, conjugated for the inverse-by-conjugation
           buf0[slot(j)] = fx::mk(ax - by, -(ay + bx));
           if (j > 0 && 2 * j < N) buf0[slot(N - j)] = fx::mk(ax + by, ay - bx);
@@ -175,7 +176,7 @@ __global__ void __launch_bounds__(rt_threads(sizeof(typename A::T)), 2) rt_pass_
       }
     } else {
 #pragma unroll
-      for (int r = 0; r < MR; ++r) v[r] = fx::mk(fx::to_fixed(x[r].x, sh), fx::to_fixed(x[r].y, sh, back));
+      for (int r = 0; r < MR; ++r) v[r] = fx::mk(fx::to_fixed(x[r].x, sa), fx::to_fixed(x[r].y, sb, back));
     }
   } else if constexpr (KIND == K_C2R) {
 #pragma unroll
@@ -257,23 +258,17 @@ __global__ void __launch_bounds__(rt_threads(sizeof(typename A::T)), 2) rt_pass_
         for (int r = 0; r < R; ++r) {
           // in place for r2c: the thread's own points
           if constexpr (KIND == K_R2C) A0[slot(b + r * Ns)] = v[r];
-          else io.store(b - t + r * Ns, out(v[r]));
+          else io.store(b - t + r * Ns, out.point(v[r]));
         }
       }
     });
   }
   if constexpr (KIND == K_R2C) {
     __syncthreads();
-    if constexpr (A::kFixed) out.adj -= 1 << 20;  // the halves of both spectra
 #pragma unroll 1
     for (int k = t; k < h; k += tpl) {
       const C zk = A0[slot(k)], zm = A0[slot(k == 0 ? 0 : N - k)];
-      if constexpr (A::kFixed) {
-        io.put_halves(k - t, out(fx::mk(zk.x + zm.x, zk.y - zm.y)), out(fx::mk(zk.y + zm.y, zm.x - zk.x)));
-      } else {
-        io.put_halves(k - t, make_float2((zk.x + zm.x) * 0.5f, (zk.y - zm.y) * 0.5f),
-                      make_float2((zk.y + zm.y) * 0.5f, (zm.x - zk.x) * 0.5f));
-      }
+      io.put_halves(k - t, out.half_a(zk, zm), out.half_b(zk, zm));
     }
   }
 }

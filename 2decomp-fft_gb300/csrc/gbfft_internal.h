@@ -354,7 +354,7 @@ __host__ __device__ constexpr size_t rt_entries(int n, int L) { return ((size_t)
 // fallback needs two for a single line), and the lines' scale words
 __host__ __device__ constexpr size_t rt_smem_bytes(int prec_bytes, int n, int L, int nst) {
   return (nst > 2 || (prec_bytes == 8 && L == 1) ? 2 : 1) * rt_entries(n, L) * (size_t)(2 * prec_bytes) + 32 +
-         (size_t)L * 8;
+         (size_t)L * 16;
 }
 cudaError_t launch_rt_f32(int kind, bool contiguous, const PassArgs& a, cudaStream_t s);
 cudaError_t launch_rt_f64(int kind, bool contiguous, const PassArgs& a, cudaStream_t s);
