@@ -127,12 +127,8 @@ __global__ void __launch_bounds__(kFxMaxThreads) fx_pass_kernel(const __grid_con
   const int e = N * a.L;
   I2* buf0 = reinterpret_cast<I2*>(smem_raw);
   I2* buf1 = buf0 + (e + (e >> 4) + 1);
-  int* smax = reinterpret_cast<int*>(buf1 + (e + (e >> 4) + 1));
-  unsigned* ssum = reinterpret_cast<unsigned*>(smax + 2 * a.L);
-  {
-    const int threads = blockDim.x * blockDim.y;
-    for (int i = threadIdx.x + threadIdx.y * blockDim.x; i < 4 * a.L; i += threads) smax[i] = 0;
-  }
+  const fx::Words words(smem_raw + fx_smem_bytes(N, a.L), a.L);
+  words.clear(a.L);
   __syncthreads();
 
   // c2r: two half spectra of N / 2 + 1 points, point j of both in v[2 i], v[2 i + 1]
@@ -152,7 +148,7 @@ __global__ void __launch_bounds__(kFxMaxThreads) fx_pass_kernel(const __grid_con
     }
   }
   fx::PassScale<KIND> sc;
-  if (!sc.template find<J * W>(v, &smax[2 * c.line], &ssum[2 * c.line])) {
+  if (!sc.find(v, words, c.line, t == 0, [&](int i) { return t + i * tpl < cnt; })) {
     fx::fallback<KIND, CONTIG>(a, reinterpret_cast<double2*>(smem_raw));
     return;
   }
@@ -192,12 +188,18 @@ __global__ void __launch_bounds__(kFxMaxThreads) fx_pass_kernel(const __grid_con
 #pragma unroll 1
     for (int k = t; 2 * k <= N; k += tpl) {
       const I2 zk = A[c.sidx(k)], zm = A[c.sidx(k == 0 ? 0 : N - k)];
-      c.put_half(0, k, out.half_a(zk, zm));
-      c.put_half(1, k, out.half_b(zk, zm));
+      double2 xa = out.half_a(zk, zm), xb = out.half_b(zk, zm);
+      if (out.off && k == 0) out.dc(xa, xb, N);
+      c.put_half(0, k, xa);
+      c.put_half(1, k, xb);
     }
   } else {
 #pragma unroll 1
-    for (int n = t; n < N; n += tpl) c.gstore_raw(n, out.point(A[c.sidx(n)]));
+    for (int n = t; n < N; n += tpl) {
+      double2 z = out.point(A[c.sidx(n)]);
+      if (KIND == K_C2C && out.off && n == 0) out.dc(z, N);
+      c.gstore_raw(n, z);
+    }
   }
 }
 
@@ -235,10 +237,8 @@ __global__ void __launch_bounds__(kFxMaxThreads) fx_r2r_kernel(const __grid_cons
   const int e = a.M * a.L, t = c.t, tpl = c.tpl, cnt = r2r::elements(a.kind, a.n);
   I2* buf0 = reinterpret_cast<I2*>(smem_raw);
   I2* buf1 = buf0 + (e + (e >> 4) + 1);
-  int* smax = reinterpret_cast<int*>(buf1 + (e + (e >> 4) + 1));
-  unsigned* ssum = reinterpret_cast<unsigned*>(smax + 2 * a.L);
-  const int threads = blockDim.x * blockDim.y;
-  for (int i = threadIdx.x + threadIdx.y * blockDim.x; i < 4 * a.L; i += threads) smax[i] = 0;
+  const fx::Words words(smem_raw + fx_smem_bytes(a.M, a.L), a.L);
+  words.clear(a.L);
   __syncthreads();
   double2 x[kE];
 #pragma unroll
@@ -247,7 +247,15 @@ __global__ void __launch_bounds__(kFxMaxThreads) fx_r2r_kernel(const __grid_cons
     x[i] = j < cnt ? ln.element(j) : make_double2(0, 0);
   }
   fx::PairScale sc;
-  if (!sc.find<false, kE>(x, &smax[2 * c.line], &ssum[2 * c.line], ln.single)) {
+  int* const wm = words.m + 2 * c.line;
+  unsigned* const ws = words.s + 2 * c.line;
+  fx::Found found = sc.find<false, true>(x, wm, ws, ln.single, r2r::keeps_mean(a.kind));
+  const bool off = found == fx::Found::flat;
+  if (__builtin_expect(off, 0)) {
+    fx::take_means(x, words, c.line, t == 0, [&](int i) { return t + i * tpl < cnt; });
+    found = sc.find<false, false>(x, wm, ws, ln.single);
+  }
+  if (found != fx::Found::yes) {
     r2r::fallback<CONTIG>(a, reinterpret_cast<double2*>(smem_raw));
     return;
   }
@@ -281,6 +289,7 @@ __global__ void __launch_bounds__(kFxMaxThreads) fx_r2r_kernel(const __grid_cons
     mp.finish(
         A, k, [&](int i, ll ya, ll yb) { ln.store(i, sc.a.out(ya, adj_a), sc.b.out(yb, adj_b)); },
         [&](int i, ll y) { ln.store1(i, sc.a.out(y, adj_a)); });
+  if (off && t == 0) ln.add_mean(words.ref[c.line]);
   ln.pass_through(a.naxis, t, tpl);
 }
 

@@ -386,16 +386,58 @@ __device__ __forceinline__ double to_double(ll v, int adj, int flip = 0) {
   return __hiloint2double((int)(h + min(h, 1u) * ((unsigned)adj + (unsigned)flip)), __double2loint(d));
 }
 
+// A tile's scale words, in the kFxWordBytes a line at the end of its shared
+// memory: a reference value, and for each of a line's one or two scales the
+// largest high word, the sum of moduli and a mark.
+struct Words {
+  double2* ref;
+  int *m, *far;
+  unsigned* s;
+  __device__ __forceinline__ Words(unsigned char* end, int L)
+      : ref(reinterpret_cast<double2*>(end - (size_t)L * kFxWordBytes)),
+        m(reinterpret_cast<int*>(ref + L)),
+        far(m + 2 * L),
+        s(reinterpret_cast<unsigned*>(far + 2 * L)) {}
+  // zero but for the references
+  __device__ __forceinline__ void clear(int L) const {
+    for (int i = threadIdx.x + threadIdx.y * blockDim.x; i < 6 * L; i += blockDim.x * blockDim.y) m[i] = 0;
+  }
+};
+
+// What a CTA's lines need, the same for all its threads.
+enum class Found {
+  yes,   // nothing
+  fp64,  // a line must run in FP64
+  flat   // a thread's values are all near its line's largest (FLAT: looked for)
+};
+template <bool FLAT>
+__device__ __forceinline__ Found cta_found(int bad, int flat) {
+  if (!__syncthreads_or(bad | flat)) return Found::yes;
+  return FLAT && !__syncthreads_or(bad) ? Found::flat : Found::fp64;
+}
+constexpr int kNear = 1 << 18;  // of high words: 2^-3 to 2^-2 of a value
+// Whether a thread's moduli, of high words up to `most` and, zeros passed over
+// (places past a line's points hold them), from least + 1 on, are all near the
+// line's largest, m.
+__device__ __forceinline__ int near_all(int most, unsigned least, int m) {
+  const int from = max(m - kNear, 1 << 20);
+  return most >= from && least >= (unsigned)from - 1;
+}
+
 // The scale of a line, from the values its threads hold.
 struct Scale {
   int m, em, es;  // largest high word, its exponent, exponent of the sum of moduli (over 2^em)
-  // The line's scale words start at zero.  False (for the whole CTA): a line
-  // of the CTA must run in FP64.
-  template <int Q>
-  __device__ __forceinline__ bool find(const double2 (&x)[Q], int* smax, unsigned* ssum) {
-    m = 0;
+  // The line's scale words start at zero.
+  template <bool FLAT, int Q>
+  __device__ __forceinline__ Found find(const double2 (&x)[Q], int* smax, unsigned* ssum) {
+    int most = 0;
+    unsigned least = ~0u;
 #pragma unroll
-    for (int i = 0; i < Q; ++i) m = max(m, max_hi(x[i]));
+    for (int i = 0; i < Q; ++i) {
+      most = max(most, max_hi(x[i]));
+      least = min(least, (unsigned)max_hi(x[i]) - 1);
+    }
+    m = most;
     atomicMax(smax, m);
     __syncthreads();
     m = *smax;
@@ -409,10 +451,11 @@ struct Scale {
 #pragma unroll
       for (int i = 0; i < Q; ++i) bad |= any_lo(x[i]);
     }
-    if (__syncthreads_or(bad)) return false;
+    const Found f = cta_found<FLAT>(bad, FLAT && near_all(most, least, m));
+    if (f != Found::yes) return f;
     const unsigned s = *ssum;
     es = 32 - __clz((int)(s + (s >> 1))) - 1040;  // a modulus is at most sqrt 2 times the larger component
-    return true;
+    return f;
   }
   // Exponent (less em) that bounds the modulus of a sum of at most 2^lg
   // values, each raised by at most 2^grow: the sum of all, or 2^lg times the
@@ -433,16 +476,20 @@ struct PairScale {
   Scale a, b;
   // smax, ssum: two words each, at zero.  HALVES: x[2 i], x[2 i + 1] are
   // points of the lines' half spectra, else x[i] holds a point of a and b.
-  template <bool HALVES, int Q>
-  __device__ __forceinline__ bool find(const double2 (&x)[Q], int* smax, unsigned* ssum, bool single = false) {
+  template <bool HALVES, bool FLAT, int Q>
+  __device__ __forceinline__ Found find(const double2 (&x)[Q], int* smax, unsigned* ssum, bool single = false,
+                                        bool flat = true) {
     constexpr int S = HALVES ? 2 : 1;
     auto ha = [&](int i) { return HALVES ? max_hi(x[i]) : abs_hi(x[i].x); };
     auto hb = [&](int i) { return HALVES ? max_hi(x[i + 1]) : abs_hi(x[i].y); };
     int ma = 0, mb = 0;
+    unsigned la = ~0u, lb = ~0u;
 #pragma unroll
     for (int i = 0; i < Q; i += S) {
       ma = max(ma, ha(i));
       mb = max(mb, hb(i));
+      la = min(la, (unsigned)ha(i) - 1);
+      lb = min(lb, (unsigned)hb(i) - 1);
     }
     if (single) ma = mb = max(ma, mb);
     atomicMax(smax, ma);
@@ -470,13 +517,14 @@ struct PairScale {
         if (b.m == 0) bad |= HALVES ? any_lo(x[i + 1]) : __double2loint(x[i].y);
       }
     }
-    if (__syncthreads_or(bad)) return false;
+    const Found f = cta_found<FLAT>(bad, FLAT && flat && (near_all(ma, la, a.m) | near_all(mb, lb, b.m)));
+    if (f != Found::yes) return f;
     // a complex point's modulus is at most sqrt 2 times its larger component;
     // one bit for the other line: the moduli of a + i b sum to at most both
     const unsigned ta = ssum[0], tb = ssum[1];
     a.es = 33 - __clz((int)(HALVES ? ta + (ta >> 1) : ta)) - 1040;
     b.es = 33 - __clz((int)(HALVES ? tb + (tb >> 1) : tb)) - 1040;
-    return true;
+    return f;
   }
   __device__ __forceinline__ static int outside(const Scale& s) {
     return s.m != 0 && (s.em < kMinExp || s.em > kMaxExp);
@@ -498,6 +546,46 @@ __device__ __forceinline__ ll to_fixed(double x, int sh, int flip = 0) {
   const ll m = (ll)(((unsigned long long)(mh ^ (unsigned)sg) << 32) | ((l << 9) ^ (unsigned)sg));
   return ((m >> s) + 1) >> 1;
 }
+// Takes the mean off a thread's points of a line: its first value, in the
+// components (c2c: real and imaginary part; else: lines) whose values all lie
+// near that, zero in the others.
+//
+// On its own scale a mean would leave the rest of the line with the bits
+// below it, where an FP64 transform of numbers of few digits cancels it
+// exactly (101325 + 100 g of FP32 origin, 512 points, rel-L2 of all but bin 0:
+// 1.4e-14, FP64 1.7e-16).  Within kNear the differences are exact, and a mean
+// that stands out less costs no more bits than fixed point has to spare.  Only
+// CTAs of which a thread saw nothing but near values come here, and scale
+// their lines anew.  Thread `first` holds point 0 in x[0]; mine(i): the thread
+// has a point in x[i]; the scale words are left cleared and the mean in w.ref.
+template <int Q, class Mine>
+__device__ __forceinline__ void take_means(double2 (&x)[Q], const Words& w, int line, bool first, Mine&& mine) {
+  if (first) w.ref[line] = x[0];
+  __syncthreads();
+  const double2 r = w.ref[line];
+  const int hx = __double2hiint(r.x), hy = __double2hiint(r.y);
+  unsigned dx = 0, dy = 0;  // distances, kNear added
+#pragma unroll
+  for (int i = 0; i < Q; ++i)
+    if (mine(i)) {
+      dx = max(dx, (unsigned)(__double2hiint(x[i].x) - hx + kNear));
+      dy = max(dy, (unsigned)(__double2hiint(x[i].y) - hy + kNear));
+    }
+  if (dx > 2 * kNear || abs_hi(r.x) < 1 << 20) w.far[2 * line] = 1;
+  if (dy > 2 * kNear || abs_hi(r.y) < 1 << 20) w.far[2 * line + 1] = 1;
+  __syncthreads();
+  const double2 mean = make_double2(w.far[2 * line] ? 0.0 : r.x, w.far[2 * line + 1] ? 0.0 : r.y);
+#pragma unroll
+  for (int i = 0; i < Q; ++i)
+    if (mine(i)) x[i] = make_double2(x[i].x - mean.x, x[i].y - mean.y);
+  if (first) {
+    w.ref[line] = mean;
+    w.m[2 * line] = w.m[2 * line + 1] = 0;
+    w.s[2 * line] = w.s[2 * line + 1] = 0;
+  }
+  __syncthreads();
+}
+
 // From the integers of a pass's complex line back to doubles: the exponent of
 // each line's unit, in a high word, and the sign of the imaginary part.  A
 // zero line that shares its transform is zero whatever the other's rounding
@@ -506,6 +594,15 @@ template <int KIND>
 struct Back {
   int adj_a, adj_b, flip;
   bool za, zb;
+  bool off;             // the lines went without their
+  const double2* mean;  // mean, which their n-point transform has in bin 0
+  __device__ __forceinline__ void dc(double2& v, int n) const {
+    v = make_double2(__fma_rn((double)n, mean->x, v.x), __fma_rn((double)n, mean->y, v.y));
+  }
+  __device__ __forceinline__ void dc(double2& va, double2& vb, int n) const {
+    va.x = __fma_rn((double)n, mean->x, va.x);
+    vb.x = __fma_rn((double)n, mean->y, vb.x);
+  }
   // c2c, c2r: a point (c2r: of both lines)
   __device__ __forceinline__ double2 point(I2 v) const {
     return make_double2(za ? 0.0 : to_double(v.x, adj_a), zb ? 0.0 : to_double(v.y, adj_b, flip));
@@ -527,11 +624,28 @@ struct PassScale {
   static constexpr int X = KIND == K_C2R ? 1 : 0;  // a point combines two values
   PairScale p;  // c2c: p.a alone
   int ta = -1021 + X, tb = -1021 + X;
-  // smax, ssum: two words each, at zero
-  template <int Q>
-  __device__ __forceinline__ bool find(const double2 (&x)[Q], int* smax, unsigned* ssum) {
-    if constexpr (KIND == K_C2C) return p.a.find<Q>(x, smax, ssum);
-    else return p.find<KIND == K_C2R, Q>(x, smax, ssum);
+  bool off = false;
+  const double2* mean;
+  // False (for the whole CTA): a line must run in FP64.  w: cleared; thread
+  // `first` of a line holds its point 0 in x[0], mine(i): the thread has a
+  // point in x[i].
+  template <int Q, class Mine>
+  __device__ __forceinline__ bool find(double2 (&x)[Q], const Words& w, int line, bool first, Mine&& mine) {
+    mean = &w.ref[line];
+    int* m = w.m + 2 * line;
+    unsigned* s = w.s + 2 * line;
+    auto look = [&](auto flat) {
+      constexpr bool FLAT = decltype(flat)::value;
+      if constexpr (KIND == K_C2C) return p.a.find<FLAT>(x, m, s);
+      else return p.find<KIND == K_C2R, FLAT>(x, m, s);
+    };
+    Found f = look(std::integral_constant<bool, KIND != K_C2R>{});
+    if (KIND != K_C2R && __builtin_expect(f == Found::flat, 0)) {
+      take_means(x, w, line, first, mine);
+      off = true;
+      f = look(std::false_type{});
+    }
+    return f == Found::yes;
   }
   // stage of at most 2^lg summed inputs, divided by 2^shift so far
   __device__ __forceinline__ void stage(int lg, int shift) {
@@ -552,6 +666,8 @@ struct PassScale {
     r.flip = flip;
     r.za = KIND != K_C2C && p.a.m == 0;
     r.zb = KIND != K_C2C && p.b.m == 0;
+    r.off = off;
+    r.mean = mean;
     return r;
   }
 };

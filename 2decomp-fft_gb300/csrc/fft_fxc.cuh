@@ -146,7 +146,11 @@ __device__ __forceinline__ void run(const Out& io, int t, I2* Sm, const Slots<P,
       const int b = t + m * TPL;
       if ((NB % TPL != 0 && b >= NB)) break;
 #pragma unroll
-      for (int r = 0; r < R; ++r) io.store(m * TPL + r * NS, back.point(v[m * R + r]));
+      for (int r = 0; r < R; ++r) {
+        double2 z = back.point(v[m * R + r]);
+        if (KIND == K_C2C && m == 0 && r == 0 && back.off && t == 0) back.dc(z, P::N);
+        io.store(m * TPL + r * NS, z);
+      }
     }
   } else {
     if constexpr (FROM_SMEM) __syncthreads();  // every point read before the outputs overwrite them
@@ -184,10 +188,8 @@ __global__ void __launch_bounds__(fxc_max_threads(P::TPL), min_ctas<P>())
   Slots<P, CONTIG> slot;
   slot.base = CONTIG ? c.line * Slots<P, CONTIG>::kLine : c.line;
   slot.L = L;
-  // the lines' scale words, behind the exchange buffer
-  int* smax = reinterpret_cast<int*>(smem_raw + fxc_smem_bytes(N, L) - (size_t)L * 16);
-  unsigned* ssum = reinterpret_cast<unsigned*>(smax + 2 * L);
-  for (int i = threadIdx.x + threadIdx.y * blockDim.x; i < 4 * L; i += blockDim.x * blockDim.y) smax[i] = 0;
+  const Words words(smem_raw + fxc_smem_bytes(N, L), L);
+  words.clear(L);
   __syncthreads();
 
   // 1. load: c2r both half spectra (point j in x[2 i], x[2 i + 1]), else the
@@ -215,7 +217,7 @@ __global__ void __launch_bounds__(fxc_max_threads(P::TPL), min_ctas<P>())
   }
   // 2. the line's scale
   PassScale<KIND> sc;
-  if (!sc.template find<Q>(x, &smax[2 * c.line], &ssum[2 * c.line])) {
+  if (!sc.find(x, words, c.line, t == 0, [&](int i) { return NB0 % TPL == 0 || t + i / R0 * TPL < NB0; })) {
     fallback<KIND, CONTIG>(a, reinterpret_cast<double2*>(smem_raw));
     return;
   }
@@ -254,8 +256,10 @@ __global__ void __launch_bounds__(fxc_max_threads(P::TPL), min_ctas<P>())
       const int k = t + i * TPL;
       if (k < H) {
         const I2 zk = Sm[slot(k)], zm = Sm[slot(k == 0 ? 0 : N - k)];
-        io.put_half(0, i * TPL, back.half_a(zk, zm));
-        io.put_half(1, i * TPL, back.half_b(zk, zm));
+        double2 xa = back.half_a(zk, zm), xb = back.half_b(zk, zm);
+        if (i == 0 && back.off && t == 0) back.dc(xa, xb, N);
+        io.put_half(0, i * TPL, xa);
+        io.put_half(1, i * TPL, xb);
       }
     }
   }
@@ -274,9 +278,8 @@ __global__ void __launch_bounds__(fxc_max_threads(P::TPL), min_ctas<P>())
   Slots<P, CONTIG> slot;
   slot.base = CONTIG ? line * Slots<P, CONTIG>::kLine : line;
   slot.L = L;
-  int* smax = reinterpret_cast<int*>(smem_raw + fxc_smem_bytes(N, L) - (size_t)L * 16);
-  unsigned* ssum = reinterpret_cast<unsigned*>(smax + 2 * L);
-  for (int i = threadIdx.x + threadIdx.y * blockDim.x; i < 4 * L; i += blockDim.x * blockDim.y) smax[i] = 0;
+  const Words words(smem_raw + fxc_smem_bytes(N, L), L);
+  words.clear(L);
   __syncthreads();
   const int cnt = r2r::elements(a.kind, a.n);
   double2 x[Q];
@@ -286,7 +289,15 @@ __global__ void __launch_bounds__(fxc_max_threads(P::TPL), min_ctas<P>())
     x[i] = j < cnt ? ln.element(j) : make_double2(0, 0);
   }
   PairScale sc;
-  if (!sc.find<false, Q>(x, &smax[2 * line], &ssum[2 * line], ln.single)) {
+  int* const wm = words.m + 2 * line;
+  unsigned* const ws = words.s + 2 * line;
+  Found found = sc.find<false, true>(x, wm, ws, ln.single, r2r::keeps_mean(a.kind));
+  const bool off = found == Found::flat;
+  if (__builtin_expect(off, 0)) {
+    take_means(x, words, line, t == 0, [&](int i) { return t + i * TPL < cnt; });
+    found = sc.find<false, false>(x, wm, ws, ln.single);
+  }
+  if (found != Found::yes) {
     r2r::fallback<CONTIG>(a, reinterpret_cast<double2*>(smem_raw));
     return;
   }
@@ -321,6 +332,7 @@ __global__ void __launch_bounds__(fxc_max_threads(P::TPL), min_ctas<P>())
     mp.finish(
         Sm, k, [&](int i, ll ya, ll yb) { ln.store(i, sc.a.out(ya, adj_a), sc.b.out(yb, adj_b)); },
         [&](int i, ll y) { ln.store1(i, sc.a.out(y, adj_a)); });
+  if (off && t == 0) ln.add_mean(words.ref[line]);
   ln.pass_through(a.naxis, t, TPL);
 }
 

@@ -193,6 +193,10 @@ struct Maps {
   __device__ __forceinline__ int tail() const { return kind == 2 || kind == 6 || single_line(kind, n) ? 1 : 0; }
 };
 
+// Kinds that have a constant line's whole transform in output 0 (DCT-I,
+// DCT-II): 2 (n - 1) and 2 n times it.
+__device__ __forceinline__ bool keeps_mean(int kind) { return kind == 1 || kind == 2; }
+
 // The real lines behind complex line cl of an r2r pass.
 template <typename T, bool CONTIG>
 struct Lines {
@@ -242,6 +246,14 @@ struct Lines {
   }
   __device__ __forceinline__ void store1(int i, T y) const {
     if (valid) dst[b0 + (long long)(off + i) * sn] = y;
+  }
+  // puts the lines' means back into output 0, which the calling thread has stored
+  __device__ __forceinline__ void add_mean(double2 mean) const {
+    if (!valid) return;
+    const double w = 2 * (kind == 1 ? n - 1 : n);
+    const long long at = (long long)off * sn;
+    dst[b0 + at] = __fma_rn(w, mean.x, dst[b0 + at]);
+    if (has1) dst[b1 + at] = __fma_rn(w, mean.y, dst[b1 + at]);
   }
   // points outside the window, copied through when dst is another array
   __device__ __forceinline__ void pass_through(int naxis, int t, int tpl) const {

@@ -148,13 +148,11 @@ __global__ void __launch_bounds__(rt_threads(sizeof(typename A::T)), 2) rt_pass_
   }
   C v[MR];
   if constexpr (A::kFixed) {
-    int* smax = reinterpret_cast<int*>(smem_raw + rt_smem_bytes(8, N, a.L, p.nst) - (size_t)a.L * 16);
-    unsigned* ssum = reinterpret_cast<unsigned*>(smax + 2 * a.L);
-    const int threads = blockDim.x * blockDim.y;
-    for (int i = threadIdx.x + threadIdx.y * blockDim.x; i < 4 * a.L; i += threads) smax[i] = 0;
+    const fx::Words words(smem_raw + rt_smem_bytes(8, N, a.L, p.nst), a.L);
+    words.clear(a.L);
     __syncthreads();
     fx::PassScale<KIND> sc;
-    if (!sc.template find<Q>(x, &smax[2 * c.line], &ssum[2 * c.line])) {
+    if (!sc.find(x, words, c.line, t == 0, [&](int r) { return r < R0 && t < nb0; })) {
       fx::fallback<KIND, CONTIG>(a, reinterpret_cast<double2*>(smem_raw));
       return;
     }
@@ -258,7 +256,12 @@ __global__ void __launch_bounds__(rt_threads(sizeof(typename A::T)), 2) rt_pass_
         for (int r = 0; r < R; ++r) {
           // in place for r2c: the thread's own points
           if constexpr (KIND == K_R2C) A0[slot(b + r * Ns)] = v[r];
-          else io.store(b - t + r * Ns, out.point(v[r]));
+          else {
+            G z = out.point(v[r]);
+            if constexpr (A::kFixed && KIND == K_C2C)
+              if (r == 0 && out.off && b == 0) out.dc(z, N);
+            io.store(b - t + r * Ns, z);
+          }
         }
       }
     });
@@ -268,7 +271,10 @@ __global__ void __launch_bounds__(rt_threads(sizeof(typename A::T)), 2) rt_pass_
 #pragma unroll 1
     for (int k = t; k < h; k += tpl) {
       const C zk = A0[slot(k)], zm = A0[slot(k == 0 ? 0 : N - k)];
-      io.put_halves(k - t, out.half_a(zk, zm), out.half_b(zk, zm));
+      G xa = out.half_a(zk, zm), xb = out.half_b(zk, zm);
+      if constexpr (A::kFixed)
+        if (out.off && k == 0) out.dc(xa, xb, N);
+      io.put_halves(k - t, xa, xb);
     }
   }
 }

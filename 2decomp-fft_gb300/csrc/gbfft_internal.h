@@ -83,17 +83,18 @@ struct FxPlan {
 constexpr int kFxPoints = 8;        // points a thread loads at most
 constexpr int kFxMaxThreads = 512;  // threads of a CTA
 constexpr size_t kFxMaxSmem = 200 * 1024;
+constexpr size_t kFxWordBytes = 48;  // scale words of a line (fx::Words)
 // Shared memory of L lines of n points: two padded buffers and the lines'
-// scale words (two a line, four for two real lines).
+// scale words.
 __host__ __device__ constexpr size_t fx_smem_bytes(int n, int L) {
   const size_t e = (size_t)n * (size_t)L;
-  return 2 * (e + (e >> 4) + 1) * 16 + (size_t)L * 16;
+  return 2 * (e + (e >> 4) + 1) * 16 + (size_t)L * kFxWordBytes;
 }
 // ... and of the compile-time plans (fft_fxc.cuh): one buffer, padded by an
 // entry in eight; a single line keeps room for the two of its FP64 fallback.
 __host__ __device__ constexpr size_t fxc_smem_bytes(int n, int L) {
   const size_t one = ((size_t)n + n / 8 + 2) * (size_t)L;
-  return (L == 1 ? 2 * one : one) * 16 + 32 + (size_t)L * 16;
+  return (L == 1 ? 2 * one : one) * 16 + 32 + (size_t)L * kFxWordBytes;
 }
 // Lengths with a compile-time plan (fft_fxc.cuh): X(group, n, threads a line,
 // radices).  The radices stay at most 10 (64 registers a thread, four CTAs
@@ -354,7 +355,7 @@ __host__ __device__ constexpr size_t rt_entries(int n, int L) { return ((size_t)
 // fallback needs two for a single line), and the lines' scale words
 __host__ __device__ constexpr size_t rt_smem_bytes(int prec_bytes, int n, int L, int nst) {
   return (nst > 2 || (prec_bytes == 8 && L == 1) ? 2 : 1) * rt_entries(n, L) * (size_t)(2 * prec_bytes) + 32 +
-         (size_t)L * 16;
+         (size_t)L * kFxWordBytes;
 }
 cudaError_t launch_rt_f32(int kind, bool contiguous, const PassArgs& a, cudaStream_t s);
 cudaError_t launch_rt_f64(int kind, bool contiguous, const PassArgs& a, cudaStream_t s);

@@ -10,7 +10,7 @@ scipy_fft = pytest.importorskip("scipy.fft")
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
-from test_gpu_fixed_point import TOL, engine, rel, to_device, to_lines  # noqa: E402
+from test_gpu_fixed_point import TOL, engine, r2r, rel, to_device, to_lines  # noqa: E402
 
 # a compile-time plan, the smooth-length kernel, the general kernel (factors 11
 # and 19), a plan with idle threads in a stage
@@ -44,3 +44,63 @@ def test_real_neighbours_have_their_own_scales(n, axis):
     for got, ref in real_passes(a, axis):
         for i in range(exps.size):
             assert not got[i].any() if i == 4 else rel(got[i], ref[i]) <= TOL, i
+
+
+def spread(kind, shape, rng):
+    """Lines (complex) of few digits near a value whose part of the sums FP64
+    cancels exactly."""
+    g = rng.standard_normal(shape) + 1j * rng.standard_normal(shape)
+    if kind == "fp32 mean":
+        return (101325 + 100 * g).astype(np.complex64).astype(np.complex128)
+    if kind == "integers":
+        return 2.0 ** 20 + rng.integers(-8, 9, shape) + 1j * rng.integers(-8, 9, shape)
+    if kind == "negative":
+        return -1 - 1j + np.rint(g * 2.0 ** 20) * 2.0 ** -40
+    if kind == "one component":
+        return 1e6 + 1j * g.imag
+    # every second line a constant one, the others noise
+    return np.where(np.arange(shape[0])[:, None] % 2 == 0, 300.0 + 0j, g * 1e-3)
+
+
+@pytest.mark.parametrize("axis", [0, 1])
+@pytest.mark.parametrize("n", KERNELS + [2, 17, 512, 1024, 4096])
+def test_a_mean_leaves_the_rest_its_digits(n, axis):
+    """c2c both ways and r2c of lines near a constant of few digits: the other
+    bins, whose exact values are taken on the line less that constant, are as
+    accurate as those of a line without it; bin 0 is within two roundings."""
+    rng = np.random.default_rng(n)
+    for kind in ("fp32 mean", "integers", "negative", "one component", "neighbours"):
+        a = spread(kind, (7, n), rng)
+        for real in (False, True):
+            rows = np.ascontiguousarray(a.real) if real else a
+            mean = rows[:, :1] * (np.abs(rows[:, :1]) > 0.5)
+            rest = rows.astype(np.clongdouble) - mean
+            e = engine(n, 7, axis, real)
+            x = to_device(rows, axis, real)
+            for sign in (-1,) if real else (-1, 1):
+                y = e.empty_spectral() if real else torch.empty_like(x)
+                e.r2c(x, y) if real else e.c2c(x, y, sign)
+                got = to_lines(y, axis, real)
+                ref = scipy_fft.fft(rest, axis=1) if sign < 0 else scipy_fft.ifft(rest, axis=1) * n
+                ref = ref[:, :got.shape[1]]
+                dc, of = rows.astype(np.clongdouble).sum(axis=1), mean[:, 0].real != 0
+                assert (np.abs(got[of, 0] - dc[of]) <= 2.0 ** -51 * np.abs(dc[of])).all(), (kind, real)
+                for i in range(7):
+                    err = np.sqrt((np.abs(got[i, 1:] - ref[i, 1:]) ** 2).sum())
+                    assert err <= TOL * np.sqrt((np.abs(ref[i]) ** 2).sum()), (kind, real, i)
+
+
+@pytest.mark.parametrize("axis", [0, 1])
+@pytest.mark.parametrize("kind", [1, 2])
+@pytest.mark.parametrize("n", [9, 33, 64, 129, 257])
+def test_r2r_of_a_mean_leaves_the_rest_its_digits(n, kind, axis):
+    rng = np.random.default_rng(n)
+    rows = np.rint(101325 * 64 + 6400 * rng.standard_normal((5, n))) / 64
+    rows[2] = 300.0
+    got = r2r(rows, kind, axis)
+    rest = scipy_fft.dct(rows.astype(np.longdouble) - rows[:, :1], type=kind, axis=1)
+    dc = scipy_fft.dct(rows.astype(np.longdouble), type=kind, axis=1)[:, 0]
+    assert (np.abs(got[:, 0] - dc) <= 2.0 ** -51 * np.abs(dc)).all()
+    for i in range(5):
+        err = np.sqrt((np.abs(got[i, 1:] - rest[i, 1:]) ** 2).sum())
+        assert err <= TOL * np.sqrt((np.abs(rest[i]) ** 2).sum()), i
