@@ -34,9 +34,10 @@ using fx::W4;
 
 constexpr int kE = kFxPoints;
 
+// dc: what joins every output of the line, or null
 template <int R, class Ctx>
 __device__ __forceinline__ void fx_stage(const Ctx& c, const I2* A, I2* B, const W4* __restrict__ tw, int Ns,
-                                         unsigned magic) {
+                                         unsigned magic, const I2* dc) {
   const int nb = c.N / R;
 #pragma unroll 1
   for (int b = c.t; b < nb; b += c.tpl) {
@@ -51,6 +52,7 @@ __device__ __forceinline__ void fx_stage(const Ctx& c, const I2* A, I2* B, const
 #pragma unroll
       for (int r = 1; r < R; ++r) v[r] = fx::mul_tw(v[r], fx::ldw(w + (r - 1) * Ns), r);
     }
+    if (dc) v[0] = fx::add(v[0], *dc);
     const int base = (b - k) * R + k;
     if constexpr (R > 5 && R % 2 == 1 && R % 3 != 0) {
       fx::dft_odd<R>(v, [&](int m, I2 x) { B[c.sidx(base + m * Ns)] = x; });
@@ -64,13 +66,14 @@ __device__ __forceinline__ void fx_stage(const Ctx& c, const I2* A, I2* B, const
 
 // Any other prime: every output a direct sum over R inputs, half of each.
 template <class Ctx>
-__device__ void fx_stage_generic(const Ctx& c, const I2* A, I2* B, const W4* __restrict__ root, int R, int Ns) {
+__device__ void fx_stage_generic(const Ctx& c, const I2* A, I2* B, const W4* __restrict__ root, int R, int Ns,
+                                 const I2* dc) {
   const int N = c.N, nb = N / R, tstride = N / (Ns * R);
 #pragma unroll 1
   for (int o = c.t; o < N; o += c.tpl) {
     const int k = o % Ns, r = (o / Ns) % R, b = o / (Ns * R) * Ns + k;
     const int step = (k * tstride + r * nb) % N;
-    I2 acc = fx::mk(0, 0);
+    I2 acc = dc ? *dc : fx::mk(0, 0);
     int e = 0;
 #pragma unroll 1
     for (int j = 0; j < R; ++j) {
@@ -83,9 +86,10 @@ __device__ void fx_stage_generic(const Ctx& c, const I2* A, I2* B, const W4* __r
 }
 
 // The stages of a plan on the lines in A, ping-ponging with B; returns the
-// buffer that holds the result.
+// buffer that holds the result.  dc: see fx_stage, in the last stage.
 template <class Ctx>
-__device__ __forceinline__ const I2* fx_stages(const Ctx& c, const FxPlan& p, I2* first, I2* second) {
+__device__ __forceinline__ const I2* fx_stages(const Ctx& c, const FxPlan& p, I2* first, I2* second,
+                                               const I2* dc = nullptr) {
   const I2* A = first;
   I2* B = second;
   const W4* tw = reinterpret_cast<const W4*>(p.tw);
@@ -93,20 +97,21 @@ __device__ __forceinline__ const I2* fx_stages(const Ctx& c, const FxPlan& p, I2
   for (int s = 0; s < p.nst; ++s) {
     const int R = p.radix[s], Ns = p.ns[s];
     const unsigned mg = p.magic[s];
+    const I2* const add = s == p.nst - 1 ? dc : nullptr;
     switch (R) {
-      case 2: fx_stage<2>(c, A, B, tw, Ns, mg); break;
-      case 3: fx_stage<3>(c, A, B, tw, Ns, mg); break;
-      case 4: fx_stage<4>(c, A, B, tw, Ns, mg); break;
-      case 5: fx_stage<5>(c, A, B, tw, Ns, mg); break;
-      case 6: fx_stage<6>(c, A, B, tw, Ns, mg); break;
-      case 7: fx_stage<7>(c, A, B, tw, Ns, mg); break;
-      case 8: fx_stage<8>(c, A, B, tw, Ns, mg); break;
-      case 9: fx_stage<9>(c, A, B, tw, Ns, mg); break;
-      case 10: fx_stage<10>(c, A, B, tw, Ns, mg); break;
-      case 11: fx_stage<11>(c, A, B, tw, Ns, mg); break;
-      case 13: fx_stage<13>(c, A, B, tw, Ns, mg); break;
-      case 17: fx_stage<17>(c, A, B, tw, Ns, mg); break;
-      default: fx_stage_generic(c, A, B, reinterpret_cast<const W4*>(p.root), R, Ns); break;
+      case 2: fx_stage<2>(c, A, B, tw, Ns, mg, add); break;
+      case 3: fx_stage<3>(c, A, B, tw, Ns, mg, add); break;
+      case 4: fx_stage<4>(c, A, B, tw, Ns, mg, add); break;
+      case 5: fx_stage<5>(c, A, B, tw, Ns, mg, add); break;
+      case 6: fx_stage<6>(c, A, B, tw, Ns, mg, add); break;
+      case 7: fx_stage<7>(c, A, B, tw, Ns, mg, add); break;
+      case 8: fx_stage<8>(c, A, B, tw, Ns, mg, add); break;
+      case 9: fx_stage<9>(c, A, B, tw, Ns, mg, add); break;
+      case 10: fx_stage<10>(c, A, B, tw, Ns, mg, add); break;
+      case 11: fx_stage<11>(c, A, B, tw, Ns, mg, add); break;
+      case 13: fx_stage<13>(c, A, B, tw, Ns, mg, add); break;
+      case 17: fx_stage<17>(c, A, B, tw, Ns, mg, add); break;
+      default: fx_stage_generic(c, A, B, reinterpret_cast<const W4*>(p.root), R, Ns, add); break;
     }
     __syncthreads();
     I2* const done = B;
@@ -142,7 +147,11 @@ __global__ void __launch_bounds__(kFxMaxThreads) fx_pass_kernel(const __grid_con
     if constexpr (KIND == K_C2R) {
       v[2 * i] = n < cnt ? c.half(0, n) : make_double2(0, 0);
       v[2 * i + 1] = n < cnt ? c.half(1, n) : make_double2(0, 0);
-      if (n == 0 || 2 * n == N) v[2 * i].y = v[2 * i + 1].y = 0;  // Im of the DC and Nyquist bins is ignored
+      if (n == 0) {  // bins 0 apart, their Im ignored
+        words.ref[c.line] = make_double2(v[0].x, v[1].x);
+        v[0] = v[1] = make_double2(0, 0);
+      }
+      if (2 * n == N) v[2 * i].y = v[2 * i + 1].y = 0;  // Im of the Nyquist bin is ignored
     } else {
       v[i] = n < cnt ? c.gload_raw(n) : make_double2(0, 0);
     }
@@ -153,7 +162,7 @@ __global__ void __launch_bounds__(kFxMaxThreads) fx_pass_kernel(const __grid_con
     return;
   }
 #pragma unroll 1
-  for (int s = 0; s < p.nst; ++s) sc.stage(p.lg[s], p.shift[s]);
+  for (int s = 0; s < p.nst; ++s) sc.stage(p.lg[s], p.shift[s], s == p.nst - 1);
   // r2c adds two values that no twiddle has halved
   if (KIND == K_R2C && p.shift[p.nst - 1] == 0) sc.headroom();
   const int sa = sc.shift_a(), sb = sc.shift_b();
@@ -162,6 +171,7 @@ __global__ void __launch_bounds__(kFxMaxThreads) fx_pass_kernel(const __grid_con
   const fx::Back<KIND> out = sc.back(p.shift[p.nst - 1], flip);
 
   if constexpr (KIND == K_C2R) {
+    if (t == 0) sc.set_dc(words, c.line, p.shift[p.nst - 1]);
 #pragma unroll
     for (int i = 0; i < J; ++i) {
       const int j = t + i * tpl;
@@ -182,7 +192,8 @@ __global__ void __launch_bounds__(kFxMaxThreads) fx_pass_kernel(const __grid_con
   }
   __syncthreads();
 
-  const I2* A = fx_stages(c, p, buf0, buf1);
+  const I2* A =
+      fx_stages(c, p, buf0, buf1, KIND == K_C2R ? reinterpret_cast<const I2*>(&words.ref[c.line]) : nullptr);
 
   if constexpr (KIND == K_R2C) {
 #pragma unroll 1

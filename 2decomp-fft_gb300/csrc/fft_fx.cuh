@@ -475,10 +475,11 @@ struct Scale {
 struct PairScale {
   Scale a, b;
   // smax, ssum: two words each, at zero.  HALVES: x[2 i], x[2 i + 1] are
-  // points of the lines' half spectra, else x[i] holds a point of a and b.
+  // points of the lines' half spectra but for their bins 0, which lie in *dc;
+  // else x[i] holds a point of a and b.
   template <bool HALVES, bool FLAT, int Q>
   __device__ __forceinline__ Found find(const double2 (&x)[Q], int* smax, unsigned* ssum, bool single = false,
-                                        bool flat = true) {
+                                        bool flat = true, const double2* dc = nullptr) {
     constexpr int S = HALVES ? 2 : 1;
     auto ha = [&](int i) { return HALVES ? max_hi(x[i]) : abs_hi(x[i].x); };
     auto hb = [&](int i) { return HALVES ? max_hi(x[i + 1]) : abs_hi(x[i].y); };
@@ -497,6 +498,9 @@ struct PairScale {
     __syncthreads();
     a.m = smax[0];
     b.m = smax[1];
+    const double2 d = HALVES ? *dc : make_double2(0, 0);
+    if (HALVES && a.m == 0) a.m = abs_hi(d.x);
+    if (HALVES && b.m == 0) b.m = abs_hi(d.y);
     a.em = a.m >> 20;
     b.em = b.m >> 20;
     float sa = 0, sb = 0;
@@ -510,21 +514,36 @@ struct PairScale {
     atomicAdd(ssum, share_units(sa, 2 * Q));
     atomicAdd(ssum + 1, share_units(sb, 2 * Q));
     int bad = outside(a) | outside(b);
+    if constexpr (HALVES) bad |= max_hi(d) >> 20 > kMaxExp;
     if (a.m == 0 || b.m == 0) {  // all zero, or subnormals below 2^-1042
 #pragma unroll
       for (int i = 0; i < Q; i += S) {
         if (a.m == 0) bad |= HALVES ? any_lo(x[i]) : __double2loint(x[i].x);
         if (b.m == 0) bad |= HALVES ? any_lo(x[i + 1]) : __double2loint(x[i].y);
       }
+      if (a.m == 0) bad |= __double2loint(d.x);
+      if (b.m == 0) bad |= __double2loint(d.y);
     }
     const Found f = cta_found<FLAT>(bad, FLAT && flat && (near_all(ma, la, a.m) | near_all(mb, lb, b.m)));
     if (f != Found::yes) return f;
     // a complex point's modulus is at most sqrt 2 times its larger component;
     // one bit for the other line: the moduli of a + i b sum to at most both
     const unsigned ta = ssum[0], tb = ssum[1];
-    a.es = 33 - __clz((int)(HALVES ? ta + (ta >> 1) : ta)) - 1040;
-    b.es = 33 - __clz((int)(HALVES ? tb + (tb >> 1) : tb)) - 1040;
+    if constexpr (HALVES) {
+      a.es = with_dc(ta, a.em, abs_hi(d.x));
+      b.es = with_dc(tb, b.em, abs_hi(d.y));
+    } else {
+      a.es = 33 - __clz((int)ta) - 1040;
+      b.es = 33 - __clz((int)tb) - 1040;
+    }
     return f;
+  }
+  // ... of a half spectrum whose other bins sum to s units and bin 0 has high word h
+  __device__ __forceinline__ static int with_dc(unsigned s, int em, int h) {
+    const int over = (h >> 20) - em;
+    if (over <= 10) s += share_units(share(h, share_base(em)), 1);
+    const int es = 33 - __clz((int)(s + (s >> 1))) - 1040;
+    return over <= 10 ? es : max(es, over - 1021) + 1;
   }
   __device__ __forceinline__ static int outside(const Scale& s) {
     return s.m != 0 && (s.em < kMinExp || s.em > kMaxExp);
@@ -619,6 +638,11 @@ struct Back {
 
 // The scale of a pass's complex line and the way back from it: one scale for
 // c2c, one for each of the two real lines of r2c and c2r.
+//
+// c2r: the half spectra go without their bins 0, which are real and join every
+// output when the last stage adds them to its butterflies' inputs 0.  Bin 0
+// of a field with a mean is far above the others; as one of them it would be
+// what the early stages' sums are bounded by.
 template <int KIND>
 struct PassScale {
   static constexpr int X = KIND == K_C2R ? 1 : 0;  // a point combines two values
@@ -626,9 +650,9 @@ struct PassScale {
   int ta = -1021 + X, tb = -1021 + X;
   bool off = false;
   const double2* mean;
-  // False (for the whole CTA): a line must run in FP64.  w: cleared; thread
-  // `first` of a line holds its point 0 in x[0], mine(i): the thread has a
-  // point in x[i].
+  // False (for the whole CTA): a line must run in FP64.  w: cleared (c2r: the
+  // bins 0 in its references); thread `first` of a line holds its point 0 in
+  // x[0], mine(i): the thread has a point in x[i].
   template <int Q, class Mine>
   __device__ __forceinline__ bool find(double2 (&x)[Q], const Words& w, int line, bool first, Mine&& mine) {
     mean = &w.ref[line];
@@ -637,7 +661,7 @@ struct PassScale {
     auto look = [&](auto flat) {
       constexpr bool FLAT = decltype(flat)::value;
       if constexpr (KIND == K_C2C) return p.a.find<FLAT>(x, m, s);
-      else return p.find<KIND == K_C2R, FLAT>(x, m, s);
+      else return p.find<KIND == K_C2R, FLAT>(x, m, s, false, true, mean);
     };
     Found f = look(std::integral_constant<bool, KIND != K_C2R>{});
     if (KIND != K_C2R && __builtin_expect(f == Found::flat, 0)) {
@@ -647,10 +671,19 @@ struct PassScale {
     }
     return f == Found::yes;
   }
-  // stage of at most 2^lg summed inputs, divided by 2^shift so far
-  __device__ __forceinline__ void stage(int lg, int shift) {
+  // stage of at most 2^lg summed inputs, divided by 2^shift so far; the last
+  // one of c2r has bin 0 too
+  __device__ __forceinline__ void stage(int lg, int shift, bool last) {
+    if (KIND == K_C2R && last) lg = 4096;
     ta = max(ta, p.a.bound(lg, X) - shift);
     if constexpr (KIND != K_C2C) tb = max(tb, p.b.bound(lg, X) - shift);
+  }
+  // c2r: the bins 0 as what the last stage adds (conjugated, as its line is),
+  // in the line's reference; thread `first` of a line, before a barrier
+  __device__ __forceinline__ void set_dc(const Words& w, int line, int shift) const {
+    const double2 d = w.ref[line];
+    *reinterpret_cast<I2*>(&w.ref[line]) =
+        mk(to_fixed(d.x, shift_a() + shift), to_fixed(d.y, shift_b() + shift, (int)0x80000000));
   }
   __device__ __forceinline__ void headroom() {
     ++ta;

@@ -115,7 +115,7 @@ struct Io {
 // The stages from S on.  KIND K_R2C: the last one leaves its outputs in Sm.
 template <class P, int S, bool FROM_SMEM, int KIND, bool CONTIG, class Out, class Bk>
 __device__ __forceinline__ void run(const Out& io, int t, I2* Sm, const Slots<P, CONTIG>& slot, const W4* __restrict__ tw,
-                                    I2 (&v)[P::points()], const Bk& back) {
+                                    I2 (&v)[P::points()], const Bk& back, const I2* dc = nullptr) {
   constexpr int R = P::radix(S), NS = P::ns(S), NB = P::N / R, MB = P::mb(S), TPL = P::TPL;
   constexpr bool LAST = S == P::NST - 1;
   if constexpr (FROM_SMEM) {
@@ -138,6 +138,7 @@ __device__ __forceinline__ void run(const Out& io, int t, I2* Sm, const Slots<P,
 #pragma unroll
       for (int r = 1; r < R; ++r) v[m * R + r] = mul_tw<SH>(v[m * R + r], ldw(w + (r - 1) * NS), r);
     }
+    if constexpr (LAST && KIND == K_C2R) v[m * R] = add(v[m * R], *dc);
     dft<R>(&v[m * R]);
   }
   if constexpr (LAST && KIND != K_R2C) {
@@ -163,7 +164,7 @@ __device__ __forceinline__ void run(const Out& io, int t, I2* Sm, const Slots<P,
       for (int r = 0; r < R; ++r) Sm[slot(base + r * NS)] = v[m * R + r];
     }
     __syncthreads();
-    if constexpr (!LAST) run<P, S + 1, true, KIND, CONTIG>(io, t, Sm, slot, tw, v, back);
+    if constexpr (!LAST) run<P, S + 1, true, KIND, CONTIG>(io, t, Sm, slot, tw, v, back, dc);
   }
 }
 
@@ -204,7 +205,11 @@ __global__ void __launch_bounds__(fxc_max_threads(P::TPL), min_ctas<P>())
       const int j = t + i * TPL;
       x[2 * i] = j < H ? io.half(0, i * TPL) : make_double2(0, 0);
       x[2 * i + 1] = j < H ? io.half(1, i * TPL) : make_double2(0, 0);
-      if (j == 0 || 2 * j == N) x[2 * i].y = x[2 * i + 1].y = 0;  // Im of the DC and Nyquist bins is ignored
+      if (j == 0) {  // bins 0 apart, their Im ignored
+        words.ref[c.line] = make_double2(x[0].x, x[1].x);
+        x[0] = x[1] = make_double2(0, 0);
+      }
+      if (2 * j == N) x[2 * i].y = x[2 * i + 1].y = 0;  // Im of the Nyquist bin is ignored
     }
   } else {
 #pragma unroll
@@ -222,7 +227,7 @@ __global__ void __launch_bounds__(fxc_max_threads(P::TPL), min_ctas<P>())
     return;
   }
 #pragma unroll
-  for (int s = 0; s < P::NST; ++s) sc.stage(P::lg(s), P::shift(s));
+  for (int s = 0; s < P::NST; ++s) sc.stage(P::lg(s), P::shift(s), s == P::NST - 1);
   // r2c adds two values that no twiddle has halved
   if (KIND == K_R2C && P::NST == 1) sc.headroom();
   const int sa = sc.shift_a(), sb = sc.shift_b();
@@ -232,6 +237,7 @@ __global__ void __launch_bounds__(fxc_max_threads(P::TPL), min_ctas<P>())
   // 3. integers, and the stages
   I2 v[E];
   if constexpr (KIND == K_C2R) {
+    if (t == 0) sc.set_dc(words, c.line, P::shift(P::NST - 1));
 #pragma unroll
     for (int i = 0; i < J; ++i) {
       const int j = t + i * TPL;
@@ -248,7 +254,7 @@ __global__ void __launch_bounds__(fxc_max_threads(P::TPL), min_ctas<P>())
 #pragma unroll
     for (int i = 0; i < Q; ++i) v[i] = mk(to_fixed(x[i].x, sa), to_fixed(x[i].y, sb, flip_in));
   }
-  run<P, 0, KIND == K_C2R, KIND, CONTIG>(io, t, Sm, slot, tw, v, back);
+  run<P, 0, KIND == K_C2R, KIND, CONTIG>(io, t, Sm, slot, tw, v, back, reinterpret_cast<const I2*>(&words.ref[c.line]));
   if constexpr (KIND == K_R2C) {
     constexpr int K = (H + TPL - 1) / TPL;
 #pragma unroll

@@ -150,6 +150,10 @@ __global__ void __launch_bounds__(rt_threads(sizeof(typename A::T)), 2) rt_pass_
   if constexpr (A::kFixed) {
     const fx::Words words(smem_raw + rt_smem_bytes(8, N, a.L, p.nst), a.L);
     words.clear(a.L);
+    if (KIND == K_C2R && t == 0) {  // bins 0 apart
+      words.ref[c.line] = make_double2(x[0].x, x[1].x);
+      x[0] = x[1] = make_double2(0, 0);
+    }
     __syncthreads();
     fx::PassScale<KIND> sc;
     if (!sc.find(x, words, c.line, t == 0, [&](int r) { return r < R0 && t < nb0; })) {
@@ -157,10 +161,11 @@ __global__ void __launch_bounds__(rt_threads(sizeof(typename A::T)), 2) rt_pass_
       return;
     }
 #pragma unroll 1
-    for (int s = 0; s <= last; ++s) sc.stage(p.lg[s], p.shift[s]);
+    for (int s = 0; s <= last; ++s) sc.stage(p.lg[s], p.shift[s], s == last);
     const int sa = sc.shift_a(), sb = sc.shift_b();
     out = sc.back(p.shift[last], back);
     if constexpr (KIND == K_C2R) {
+      if (t == 0) sc.set_dc(words, c.line, p.shift[last]);
 #pragma unroll
       for (int i = 0; i < Q / 2; ++i) {
         const int j = t + i * tpl;
@@ -241,6 +246,9 @@ __global__ void __launch_bounds__(rt_threads(sizeof(typename A::T)), 2) rt_pass_
   // the last stage: its outputs are points b + r ns
   {
     const int Ns = p.ns[last];
+    fx::I2 dc;
+    if constexpr (A::kFixed && KIND == K_C2R)
+      dc = *reinterpret_cast<const fx::I2*>(&fx::Words(smem_raw + rt_smem_bytes(8, N, a.L, p.nst), a.L).ref[c.line]);
     with_radix<A>(p.radix[last], [&](auto RC) {
       constexpr int R = decltype(RC)::value;
 #pragma unroll 1
@@ -251,6 +259,7 @@ __global__ void __launch_bounds__(rt_threads(sizeof(typename A::T)), 2) rt_pass_
         v[0] = A::first(v[0]);
 #pragma unroll
         for (int r = 1; r < R; ++r) v[r] = A::mul(v[r], A::root(w + (r - 1) * Ns), r);
+        if constexpr (A::kFixed && KIND == K_C2R) v[0] = fx::add(v[0], dc);
         A::template dft<R>(v);
 #pragma unroll
         for (int r = 0; r < R; ++r) {
