@@ -381,7 +381,7 @@ void set_stages(FxPlan& p, const std::vector<int>& rad, bool fixed) {
     p.radix[s] = r;
     p.ns[s] = ns;
     p.magic[s] = ns > 1 ? (unsigned)(((1ull << 32) + ns - 1) / ns) : 0;
-    if (fixed && (ns > 1 || !fx_special(r))) shift += 1;
+    if (fixed) shift += !fx_special(r) ? 2 : ns > 1 ? 1 : 0;  // a direct sum takes quarters
     ns *= r;
     int lg = 0;
     while ((1 << lg) < ns) ++lg;

@@ -64,7 +64,9 @@ __device__ __forceinline__ void fx_stage(const Ctx& c, const I2* A, I2* B, const
   }
 }
 
-// Any other prime: every output a direct sum over R inputs, half of each.
+// Any other prime: every output a direct sum over R inputs, a quarter of each.
+// (Halves left c2r of a single peak less accurate than FP64 where two such
+// stages follow each other: 2047 points rel-L2 4.3e-16, FP64 3.1e-16.)
 template <class Ctx>
 __device__ void fx_stage_generic(const Ctx& c, const I2* A, I2* B, const W4* __restrict__ root, int R, int Ns,
                                  const I2* dc) {
@@ -77,7 +79,7 @@ __device__ void fx_stage_generic(const Ctx& c, const I2* A, I2* B, const W4* __r
     int e = 0;
 #pragma unroll 1
     for (int j = 0; j < R; ++j) {
-      acc = fx::add(acc, fx::mul_tw(A[c.sidx(b + j * nb)], fx::ldw(root + e), j));
+      acc = fx::add(acc, fx::mul_tw<2>(A[c.sidx(b + j * nb)], fx::ldw(root + e), j));
       e += step;
       if (e >= N) e -= N;
     }

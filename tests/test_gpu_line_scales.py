@@ -119,3 +119,19 @@ def test_bin_0_costs_the_others_no_digits(n, axis):
     got, ref = real_passes(a, axis)[1]
     for i in range(9):
         assert not got[i].any() if i == 4 else rel(got[i], ref[i]) <= 2.2e-16, i
+
+
+# rel-L2 of the FP64 kernels, c2r of the spectrum of one peak
+FP64_PEAK = {23 * 89: 3.1e-16, 41 * 43: 3.1e-16, 29 * 67: 3.6e-16, 11 * 179: 4.3e-16}
+
+
+@pytest.mark.parametrize("axis", [0, 1])
+@pytest.mark.parametrize("n", FP64_PEAK)
+def test_direct_sums_keep_fp64_accuracy(n, axis):
+    """c2r of a flat spectrum through direct-sum stages."""
+    rng = np.random.default_rng(n)
+    a = 1e-3 * rng.standard_normal((9, n))
+    a[:, n // 3] += 1e6 * (1 + rng.random())
+    got, ref = real_passes(a, axis)[1]
+    for i in range(9):
+        assert rel(got[i], ref[i]) <= FP64_PEAK[n], i
