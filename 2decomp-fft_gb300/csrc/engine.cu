@@ -427,8 +427,7 @@ FxPlan rt_plan(int n, int rmax, bool fixed) {
   return p;
 }
 // The fixed-point plan of an axis of n points; rmax bounds the radix (small
-// grids take radix 4: twice the threads a line).  near: rows lie below 2^28
-// elements apart, as the compile-time and smooth-length kernels address them.
+// grids take radix 4: twice the threads a line).  near: rows_near().
 FxPlan fx_plan(int n, int rmax, bool near) {
   FxPlan p;
   const FxcShape shape = near ? fxc_shape(n) : FxcShape{0, {0, 0, 0, 0}};
@@ -1243,6 +1242,14 @@ int check_engine_args(int format, int nx, int ny, int nz, int prec, int form) {
   return GBFFT_OK;
 }
 
+// Whether an axis's points lie less than 2^32 bytes apart, as the two-stage,
+// smooth-length and compile-time fixed-point kernels address them.  Always
+// along x and y; along z on planes of less than 4 GB, rows padded by at most 8.
+bool rows_near(int axis, int nx, int ny, int prec) {
+  const double apart = axis == 0 ? 1.0 : axis == 1 ? nx + 8.0 : (nx + 8.0) * ny;
+  return apart * 2 * prec < 4294967296.0;
+}
+
 // The host half of gbfft_engine_create: fields, the axis plans and the
 // tuning-cache line, no device memory (the caller uploads the twiddle tables
 // and allocates the work area).  Arguments are already validated.
@@ -1296,14 +1303,13 @@ int engine_init_host(gbfft_engine_s* e, int format, int nx, int ny, int nz, int 
     }
     // FP64 lines of one tile: fixed point; small grids (under about 16 warps
     // per SM at 8 points a thread) take radix 4 and twice the threads
+    const bool near = rows_near(d, nx, ny, prec);
     if (prec == GBFFT_PREC_DOUBLE && !e->ax[d].big && fx_length(lens[d])) {
       const double threads = (double)nx * ny * nz / kFxPoints;
-      e->ax[d].fx = fx_plan(lens[d], threads < 512.0 * kSmsDefault ? 4 : 10,
-                           (double)(nx + 8) * ny < (double)(1 << 28));
+      e->ax[d].fx = fx_plan(lens[d], threads < 512.0 * kSmsDefault ? 4 : 10, near);
     }
-    // FP32: the two-stage plan where the length has one and rows lie below
-    // 2^28 elements apart; else the smooth-length kernel
-    const bool near = (double)(nx + 8) * ny < (double)(1 << 28);
+    // FP32: the two-stage plan where the length has one and its rows are near;
+    // else the smooth-length kernel
     if (prec == GBFFT_PREC_SINGLE && near && mixed_length(lens[d])) e->ax[d].mixed = lens[d] / mixed_r0(lens[d]);
     if (prec == GBFFT_PREC_SINGLE && !e->ax[d].big && !fast_length(lens[d]) && !e->ax[d].mixed &&
         !gen_length(lens[d]) && near)

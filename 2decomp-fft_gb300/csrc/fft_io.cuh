@@ -37,7 +37,7 @@ __device__ __forceinline__ void dft_f32(float2* v) {
 }
 
 // Global accesses of a thread's points t + n: one multiply-add an address
-// (the row strides are below 2^28 elements).
+// (the row strides are below 2^32 bytes).
 template <typename T, int KIND, bool CONTIG, class Ctx = LineCtx<T, KIND, CONTIG>>
 struct Io {
   using C = Cx<T>;
