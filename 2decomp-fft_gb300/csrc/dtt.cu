@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(kMaxThreads) dtt_pass_kernel(const __grid_cons
 // compile-time 16-point plan (fft_fast.cuh), reading it from and leaving its
 // transform in one padded shared buffer.
 template <typename T, bool CONTIG, int M>
-__global__ void __launch_bounds__(fast_max_threads(16, sizeof(T)), 1)
+__global__ void __launch_bounds__(fast_max_threads(16), 1)
     dtt_fast_kernel(const __grid_constant__ DttArgs a) {
   using C = Cx<T>;
   using P = fast::P2Plan<M, 16>;
@@ -364,7 +364,7 @@ cudaError_t launch_mixed(const DttArgs& a, cudaStream_t s) {
 template <typename T, bool CONTIG, int M>
 cudaError_t launch_fast_m(const DttArgs& a, cudaStream_t stream) {
   constexpr int TPL = M / 16;
-  if (a.tpl != TPL || a.L * TPL > fast_max_threads(16, (int)sizeof(T))) return cudaErrorInvalidValue;
+  if (a.tpl != TPL || a.L * TPL > fast_max_threads(16)) return cudaErrorInvalidValue;
   const size_t smem = (size_t)fast_smem_entries(M, a.L) * sizeof(Cx<T>);
   auto kern = dtt_fast_kernel<T, CONTIG, M>;
   if (smem > 48 * 1024) {

@@ -772,7 +772,7 @@ int fast_lines_per_cta(int n, int prec, bool contiguous, long long nlines, int f
                        long long nv = 1) {
   const int tpl = n / e;
   if (forced_L > 0) return forced_L;
-  const int maxt = fast_max_threads(e, prec);
+  const int maxt = fast_max_threads(e);
   int L;
   if (contiguous) {
     // lines of at most 32 threads run warp-synchronous: 4 warps per CTA;
@@ -809,8 +809,11 @@ int fast_lines_per_cta(int n, int prec, bool contiguous, long long nlines, int f
 // twelve; 120 points 47.3 with eight, 49.3 with sixteen).  Strided tiles: a
 // power of two of lines, at least a 64-byte row segment (60 points, c2c y 36.9
 // with 16 lines, 40.3 with 24; r2c z 45.2 and 52.4).
+bool mixed_tile_ok(int n, int tpl, int L) {
+  return L * tpl <= 256 && mixed_smem_bytes(n / tpl, tpl, L) <= kFxMaxSmem;
+}
 int mixed_lines_per_cta(int n, int tpl, bool contiguous, long long nlines, long long nv, int forced_L) {
-  if (forced_L > 0 && forced_L * tpl <= 256 && mixed_smem_bytes(n / tpl, tpl, forced_L) <= kFxMaxSmem) return forced_L;
+  if (forced_L > 0 && mixed_tile_ok(n, tpl, forced_L)) return forced_L;
   int L = contiguous ? (tpl > 24 ? 1 : 96 / tpl) : 8;
   if (!contiguous)
     while (L < 32 && 2 * L * tpl <= 256) L *= 2;
@@ -826,7 +829,7 @@ int mixed_lines_per_cta(int n, int tpl, bool contiguous, long long nlines, long 
 // segments and about 512 threads; within the thread and 100 KB shared-memory
 // limits.
 int gen_lines_per_cta(int n, int prec, bool contiguous, long long nlines, int forced_L) {
-  const int e = gen_points(n), tpl = n / e, maxt = gen_max_threads(e, prec);
+  const int e = gen_points(n), tpl = n / e, maxt = gen_max_threads(e);
   int L;
   if (forced_L > 0) {
     L = forced_L;
@@ -848,20 +851,23 @@ int gen_lines_per_cta(int n, int prec, bool contiguous, long long nlines, int fo
 // Lines per CTA of the fixed-point and smooth-length kernels: strided tiles
 // about 256 threads and at least 64-byte row segments; contiguous lines about
 // 128 threads (512 x 512 x 256 FP64 x pass 336 us, with 256 threads 349).
-int fx_lines_per_cta(const FxPlan& f, int n, int prec, bool contiguous, long long nlines, long long nv, int forced_L) {
+size_t fx_plan_smem(const FxPlan& f, int n, int prec, int L) {
+  return f.ct ? fxc_smem_bytes(n, L) : f.rt ? rt_smem_bytes(prec, n, L, f.nst) : fx_smem_bytes(n, L);
+}
+bool fx_tile_ok(const FxPlan& f, int n, int prec, int L) {
   const int maxt = f.ct ? fxc_max_threads(f.tpl) : f.rt ? rt_threads(prec) : kFxMaxThreads;
-  auto smem = [&](int l) {
-    return f.ct ? fxc_smem_bytes(n, l) : f.rt ? rt_smem_bytes(prec, n, l, f.nst) : fx_smem_bytes(n, l);
-  };
-  if (forced_L > 0 && forced_L * f.tpl <= maxt && smem(forced_L) <= kFxMaxSmem) return forced_L;
+  return L * f.tpl <= maxt && fx_plan_smem(f, n, prec, L) <= kFxMaxSmem;
+}
+int fx_lines_per_cta(const FxPlan& f, int n, int prec, bool contiguous, long long nlines, long long nv, int forced_L) {
+  if (forced_L > 0 && fx_tile_ok(f, n, prec, forced_L)) return forced_L;
   const int seg = 64 / (2 * prec), min_l = contiguous ? 1 : seg;
   int L = (contiguous ? 128 : 256) / f.tpl;
   if (!contiguous && L > seg) L = L / seg * seg;
   if (L > 32) L = 32;
   if (L < min_l) L = min_l;
-  while (L > min_l && smem(L) > 72 * 1024) L = contiguous ? L - 1 : L - seg;
+  while (L > min_l && fx_plan_smem(f, n, prec, L) > 72 * 1024) L = contiguous ? L - 1 : L - seg;
   while (L > min_l && ((nlines + L - 1) / L) * nv < 2LL * kSmsDefault) L = std::max(min_l, L / 2);
-  while (L > 1 && (L * f.tpl > maxt || smem(L) > kFxMaxSmem)) --L;
+  while (L > 1 && !fx_tile_ok(f, n, prec, L)) --L;
   if (L > 1 && nlines < L) L = (int)nlines;
   return L;
 }
@@ -1720,10 +1726,33 @@ int gbfft_engine_set_profiling(gbfft_engine_t e, int enable) {
   return GBFFT_OK;
 }
 
-// Lengths whose tiles are checked against the two-stage kernel's limits; the
-// other lengths' against the general kernel's, and a tile the two-stage kernel
-// cannot run keeps the built-in one.
-static bool two_plans(int n) { return gen_length(n) || n == 48 || n == 96 || n == 192 || n == 210; }
+// Threads and shared memory that set_tile allows a tile of an axis, by its
+// length and points a thread alone, so that what it accepts does not depend on
+// which of the length's kernels the axis runs: the balanced plan's lengths,
+// the first two-stage lengths, powers of two, and the general kernel's.
+static bool tile_allowed(const AxisPlan& p, int prec, bool contiguous, int lines, const char** why) {
+  const bool gen = gen_length(p.n), two = !gen && (p.n == 48 || p.n == 96 || p.n == 192 || p.n == 210);
+  const bool fast = fast_length(p.n), balanced = gen && p.fast_e == gen_points(p.n);
+  int tpl = balanced || fast ? p.n / p.fast_e : gen || two ? p.n / mixed_r0(p.n) : p.tpl;
+  int maxt = kMaxThreads;
+  if (balanced) maxt = prec == GBFFT_PREC_DOUBLE ? 256 : gen_max_threads(p.fast_e);
+  else if (gen || two) maxt = 256;
+  else if (fast) maxt = prec == GBFFT_PREC_DOUBLE ? 256 : fast_max_threads(p.fast_e);
+  else if (!contiguous)
+    while (lines * tpl > kMaxThreads && tpl > 32) tpl /= 2;
+  const size_t smem =
+      gen || two || fast ? (size_t)fast_smem_entries(p.n, lines) * 2 * (size_t)prec : pass_smem_bytes(prec, p.n, lines);
+  *why = lines * tpl > maxt ? "tile exceeds the kernel's thread limit"
+         : smem > 200 * 1024 ? "tile exceeds the shared-memory limit"
+                             : nullptr;
+  return !*why;
+}
+// Whether the kernel that the axis runs holds the tile.
+static bool tile_runs(const AxisPlan& p, int prec, int lines) {
+  if (p.fx.nst) return fx_tile_ok(p.fx, p.n, prec, lines);
+  if (p.mixed && !uses_gen(p)) return mixed_tile_ok(p.n, p.mixed, lines);
+  return true;
+}
 
 int gbfft_engine_set_tile(gbfft_engine_t e, int kind, int lines) {
   if (!valid_engine(e)) return fail(GBFFT_ERR_INVALID, "not an engine");
@@ -1741,43 +1770,13 @@ int gbfft_engine_set_tile(gbfft_engine_t e, int kind, int lines) {
     e->tile_L[kind] = lines;
     return GBFFT_OK;
   }
-  int axis;
-  if (kind == GBFFT_PASS_R2C || kind == GBFFT_PASS_C2R)
-    axis = e->format == GBFFT_PHYSICAL_IN_X ? 0 : 2;
-  else
-    axis = kind - GBFFT_PASS_C2C_X;
+  const bool real = kind == GBFFT_PASS_R2C || kind == GBFFT_PASS_C2R;
+  const int axis = real ? (e->format == GBFFT_PHYSICAL_IN_X ? 0 : 2) : kind - GBFFT_PASS_C2C_X;
   const AxisPlan& p = e->ax[axis];
-  if (gen_length(p.n) && p.fast_e == gen_points(p.n)) {
-    const int tpl_g = p.n / p.fast_e;
-    if (lines * tpl_g > gen_max_threads(p.fast_e, e->prec))
-      return fail(GBFFT_ERR_INVALID, "tile exceeds the kernel's thread limit");
-    if ((size_t)fast_smem_entries(p.n, lines) * 2 * (size_t)e->prec > 200 * 1024)
-      return fail(GBFFT_ERR_INVALID, "tile exceeds the shared-memory limit");
-    e->tile_L[kind] = lines;
-    return GBFFT_OK;
-  }
-  if (two_plans(p.n)) {
-    const int tpl_m = p.n / mixed_r0(p.n);
-    if (lines * tpl_m > 256) return fail(GBFFT_ERR_INVALID, "tile exceeds the kernel's thread limit");
-    if ((size_t)fast_smem_entries(p.n, lines) * 2 * (size_t)e->prec > 200 * 1024)
-      return fail(GBFFT_ERR_INVALID, "tile exceeds the shared-memory limit");
-    e->tile_L[kind] = lines;
-    return GBFFT_OK;
-  }
-  const bool fast = fast_length(p.n);
-  const bool contiguous = (kind == GBFFT_PASS_C2C_X) ||
-                          ((kind == GBFFT_PASS_R2C || kind == GBFFT_PASS_C2R) &&
-                           e->format == GBFFT_PHYSICAL_IN_X);
-  const int fe = p.fast_e;
-  int tpl = fast ? p.n / fe : p.tpl;
-  const int maxt = fast ? fast_max_threads(fe, e->prec) : kMaxThreads;
-  if (!fast && !contiguous)
-    while (lines * tpl > kMaxThreads && tpl > 32) tpl /= 2;
-  if (lines * tpl > maxt) return fail(GBFFT_ERR_INVALID, "tile exceeds the kernel's thread limit");
-  const size_t smem = fast ? (size_t)fast_smem_entries(p.n, lines) * 2 * (size_t)e->prec
-                            : pass_smem_bytes(e->prec, p.n, lines);
-  if (smem > 200 * 1024) return fail(GBFFT_ERR_INVALID, "tile exceeds the shared-memory limit");
-  e->tile_L[kind] = lines;
+  const char* why = nullptr;
+  if (!tile_allowed(p, e->prec, axis == 0, lines, &why)) return fail(GBFFT_ERR_INVALID, why);
+  // a tile that only another kernel of the length holds: the built-in one
+  e->tile_L[kind] = tile_runs(p, e->prec, lines) ? lines : 0;
   return GBFFT_OK;
 }
 
@@ -2288,7 +2287,7 @@ int gbfft_exec_r2r(gbfft_dtt_t d, void* d_in, void* d_out, int isign, void* stre
     if (ax.plan.d_twf) {
       // compile-time 16-point plan: M / 16 threads a line; contiguous
       // 128-thread CTAs, strided up to 16 neighbouring lines
-      const int tplf = ax.M / 16, maxt = fast_max_threads(16, d->prec);
+      const int tplf = ax.M / 16, maxt = fast_max_threads(16);
       int Lf = contiguous ? (tplf >= 128 ? 1 : 128 / tplf) : 16;
       while (Lf > 1 && Lf * tplf > maxt) --Lf;
       while (Lf > 1 && (size_t)fast_smem_entries(ax.M, Lf) * 2 * d->prec > 100 * 1024) --Lf;

@@ -187,7 +187,7 @@ struct GenPlan {
 // row segments on strided axes) one.  32 points a thread: up to 512
 // threads, at most 128 registers.
 template <typename T, int KIND, bool CONTIG, int N, int E>
-__global__ void __launch_bounds__(fast_max_threads(E, sizeof(T)), 1)
+__global__ void __launch_bounds__(fast_max_threads(E), 1)
     fast_pass_kernel(const __grid_constant__ PassArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Cx<T>* Sm = reinterpret_cast<Cx<T>*>(smem_raw);

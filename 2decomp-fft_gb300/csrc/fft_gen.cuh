@@ -24,7 +24,7 @@ template <> struct PlanOf<384> { using type = fast::GenPlan<384, 24, 8, 8, 6>; }
 template <> struct PlanOf<400> { using type = fast::GenPlan<400, 20, 20, 20>; };
 
 template <typename T, int KIND, bool CONTIG, int N>
-__global__ void __launch_bounds__(gen_max_threads(PlanOf<N>::type::E, sizeof(T)), 1)
+__global__ void __launch_bounds__(gen_max_threads(PlanOf<N>::type::E), 1)
     gen_pass_kernel(const __grid_constant__ PassArgs a) {
   using P = typename PlanOf<N>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(gen_max_threads(PlanOf<N>::type::E, sizeof(T))
 template <typename T, int KIND, bool CONTIG, int N>
 cudaError_t launch_n(const PassArgs& a, cudaStream_t stream) {
   using P = typename PlanOf<N>::type;
-  if (a.tpl != P::TPL || a.L < 1 || a.L * P::TPL > gen_max_threads(P::E, (int)sizeof(T)))
+  if (a.tpl != P::TPL || a.L < 1 || a.L * P::TPL > gen_max_threads(P::E))
     return cudaErrorInvalidValue;
   const size_t smem = (size_t)fast_smem_entries(N, a.L) * sizeof(Cx<T>);
   auto kern = gen_pass_kernel<T, KIND, CONTIG, N>;

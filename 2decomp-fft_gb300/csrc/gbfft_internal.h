@@ -262,11 +262,10 @@ __host__ __device__ constexpr int fast_radix(int n, int e, int s) {
                  : (s < ilog2c(n) / ilog2c(e) ? e : (1 << (ilog2c(n) % ilog2c(e))));
 }
 // Thread limits of the power-of-two kernel, launched with one CTA per SM
-// guaranteed: 16 points a thread at most 64 registers (1024 threads, FP32),
+// guaranteed: 16 points a thread at most 64 registers (1024 threads),
 // 32 points a thread at most 128 (512 threads).  Smaller tiles of the same
 // kernel still run several CTAs per SM.
-constexpr int kFastMaxThreadsF32 = 1024;
-constexpr int kFastMaxThreadsF64 = 256;
+__host__ __device__ constexpr int fast_max_threads(int e) { return e == 32 ? 512 : 1024; }
 // Lengths with a compile-time two-stage plan (fft_mixed.cuh): n = R0 * R1,
 // R0 <= R1 <= 32, the most balanced such split, R1 at most 3 R0 (only R0 of
 // the R1 threads work in the second stage), of the primes up to 13 (a larger
@@ -311,10 +310,8 @@ __host__ __device__ constexpr int gen_radix(int n, int s) {
        : n == 400 ? (s < 2 ? 20 : 0) : 0;
 }
 // thread limit: E <= 16 at most 64 registers (1024 threads, FP32), more
-// points at most 128 (512 threads); FP64 256 threads
-__host__ __device__ constexpr int gen_max_threads(int e, int prec_bytes) {
-  return prec_bytes == 8 ? 256 : (e <= 16 ? 1024 : 512);
-}
+// points at most 128 (512 threads)
+__host__ __device__ constexpr int gen_max_threads(int e) { return e <= 16 ? 1024 : 512; }
 cudaError_t launch_gen_f32(int kind, bool contiguous, const PassArgs& a, cudaStream_t s);
 // Split-precision tensor-core passes (fft_split.cuh): FP32 lines of 256,
 // 512, 1024 points, 256-thread CTAs of split_lines_per_cta lines.
@@ -327,10 +324,6 @@ cudaError_t launch_split_f32(int kind, bool contiguous, const PassArgs& a, cudaS
 // at 4096 with radix-8 stages; 0.25 to 0.6 at 64 to 2048 points).
 __host__ __device__ constexpr bool fx_length(int n) { return (n >= 2 && n <= 2048) || n == 4096; }
 
-// Thread limit of the power-of-two kernel for E points a thread.
-__host__ __device__ constexpr int fast_max_threads(int e, int prec_bytes) {
-  return e == 32 ? (prec_bytes == 4 ? 512 : 256) : (prec_bytes == 4 ? kFastMaxThreadsF32 : kFastMaxThreadsF64);
-}
 // Shared-memory entries of one power-of-two tile of L lines: the exchange
 // buffer, or for c2r the staged half spectra (n/2+1 per real line).
 __host__ __device__ constexpr long long fast_smem_entries(int n, int L) {

@@ -264,7 +264,9 @@ int gbfft_engine_set_profiling(gbfft_engine_t engine, int enable);
 
 /* Tile shape of one pass kind (GBFFT_PASS_*): lines per CTA.  0 restores the
  * built-in choice.  Used by the autotuner; rejected when the CTA would exceed
- * the kernel's thread or shared-memory limit. */
+ * the thread or shared-memory limit of the axis length's kernels.  A tile
+ * within these that the kernel the axis runs cannot hold restores the
+ * built-in choice too: gbfft_engine_get_tuning reports the tile in use. */
 int gbfft_engine_set_tile(gbfft_engine_t engine, int kind, int lines_per_cta);
 
 /* Cluster launch of one pass kind (GBFFT_PASS_*) on its power-of-two
