@@ -81,6 +81,40 @@ def measure(eng, x, s, y, steps=6, warm=2):
     return {k: v[1] / v[0] for k, v in prof.items()}, step
 
 
+BALANCED = {243: 9, 270: 30, 360: 30, 384: 24, 400: 20}  # points of the balanced plans
+
+
+def plan_choices(prec, n):
+    """Points a thread to try on an axis of n points ([None]: one plan).  In
+    double precision lines of these lengths run in fixed point, with one plan
+    each, whatever set_plan keeps."""
+    if prec == 8:
+        return [None]
+    if n in (512, 1024):
+        return [16, 32]
+    if n in BALANCED:
+        return [BALANCED[n], 2]
+    if n in (16, 32, 64, 128):
+        return [16, 8, 4]  # short lines: more threads on small grids
+    return [16, 8] if n == 256 else [None]
+
+
+def launch_choices(prec, kind, n, points):
+    """Launch forms to try: clusters exist for the compile-time power-of-two
+    kernels, which are single precision's."""
+    return [(0, 0)] if prec == 8 or kind == "xy_fused" or not points or n & (n - 1) else LAUNCHES
+
+
+def take_tile(eng, kind, lines):
+    """Sets a tile; whether the pass runs it (a refused one, or one that the
+    kernel in use replaces by the built-in tile, is not worth timing)."""
+    try:
+        eng.set_tile(kind, lines)
+    except gbfft.GbfftError:
+        return False
+    return eng.tuning()["tiles"][kind] == lines
+
+
 def tune_shape(prec, fmt, nx, ny, nz, log=print):
     import torch
     rdt = torch.float32 if prec == 4 else torch.float64
@@ -88,19 +122,7 @@ def tune_shape(prec, fmt, nx, ny, nz, log=print):
     x = torch.randn((nz, ny, nx), dtype=rdt, device="cuda")
     s = eng.empty_spectral()
     y = eng.empty_physical()
-    opts = {}
-    balanced = {243: 9, 270: 30, 360: 30, 384: 24, 400: 20}  # points of the balanced plans
-    for axis, n in ((0, nx), (1, ny), (2, nz)):
-        if n in (512, 1024):
-            opts[axis] = [16, 32]
-        elif n in balanced:
-            opts[axis] = [balanced[n], 2]
-        elif n in (16, 32, 64, 128):
-            opts[axis] = [16, 8, 4]  # short lines: more threads on small grids
-        elif n == 256:
-            opts[axis] = [16, 8]
-        else:
-            opts[axis] = [None]
+    opts = {axis: plan_choices(prec, n) for axis, n in ((0, nx), (1, ny), (2, nz))}
     eng.set_fusion(False)
 
     def apply(ex, ey, ez, layout, tma):
@@ -135,14 +157,10 @@ def tune_shape(prec, fmt, nx, ny, nz, log=print):
         bt, bl, bc = t0, 0, (0, 0)
         axis = {"c2c_x": 0, "c2c_y": 1, "c2c_z": 2}.get(kind, 0 if fmt == 1 else 2)
         n = (nx, ny, nz)[axis]
-        # cluster launches exist for the compile-time power-of-two kernels
-        forms = [(0, 0)] if (kind == "xy_fused" or not pts[axis] or n & (n - 1)) else LAUNCHES
-        for clus in forms:
+        for clus in launch_choices(prec, kind, n, pts[axis]):
             eng.set_cluster(kind, *clus)
             for L in [0] + TILES:
-                try:
-                    eng.set_tile(kind, L)
-                except gbfft.GbfftError:
+                if not take_tile(eng, kind, L):
                     continue
                 t = measure(eng, x, s, y, steps=4, warm=1)[0].get(kind, t0)
                 # a choice other than the built-in one must win by 1 %
