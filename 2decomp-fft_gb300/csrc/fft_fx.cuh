@@ -363,8 +363,10 @@ __device__ __forceinline__ void dft(I2* v) {
 // ---- between doubles and a line's integers ---------------------------------
 // m: the largest magnitude's high word of a line; em = m >> 20 its biased
 // exponent.  A finite line whose exponent lies in [kMinExp, kMaxExp] runs in
-// integers: its results then neither overflow nor leave the normal range.
-constexpr int kMinExp = 200, kMaxExp = 1990;
+// integers: its results then neither overflow nor leave the normal range (the
+// unit of a result lies at most 64 powers of two below the line's largest
+// value, and a sum of 8192 moduli 14 above it).
+constexpr int kMinExp = 80, kMaxExp = 1990;
 
 __device__ __forceinline__ int abs_hi(double v) { return __double2hiint(v) & 0x7fffffff; }
 __device__ __forceinline__ int max_hi(double2 v) { return max(fx::abs_hi(v.x), fx::abs_hi(v.y)); }

@@ -135,3 +135,22 @@ def test_direct_sums_keep_fp64_accuracy(n, axis):
     got, ref = real_passes(a, axis)[1]
     for i in range(9):
         assert rel(got[i], ref[i]) <= FP64_PEAK[n], i
+
+
+@pytest.mark.parametrize("real", [False, True])
+@pytest.mark.parametrize("n", KERNELS)
+def test_small_fields_scale_exactly(n, real):
+    """Down to 2^-930 a line is transformed as its multiple by a power of two."""
+    rng = np.random.default_rng(n)
+    a = rng.standard_normal((6, n)) + (0 if real else 1j * rng.standard_normal((6, n)))
+    out = []
+    for k in (0, -930):
+        e = engine(n, 6, 0, real)
+        x = to_device(a * 2.0 ** k, 0, real)
+        y = e.empty_spectral() if real else torch.empty_like(x)
+        e.r2c(x, y) if real else e.c2c(x, y, -1)
+        if real:
+            e.c2r(y, x)
+            out.append(x * 2.0 ** -k)
+        out.append(y * 2.0 ** -k)
+    assert all(torch.equal(u, v) for u, v in zip(out[:len(out) // 2], out[len(out) // 2:]))
