@@ -196,7 +196,10 @@ def _ptr(t):
 def _stream(stream):
     if stream is None:
         import torch
-        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+        # the raw handle without a Stream object (0.3 us, by the public call
+        # 2.9), where this torch has that entry
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        return raw(torch.cuda.current_device()) if raw else torch.cuda.current_stream().cuda_stream
     if isinstance(stream, int):
         return stream
     return stream.cuda_stream
