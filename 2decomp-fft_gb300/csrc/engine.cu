@@ -371,8 +371,9 @@ struct Splitter {
   }
 };
 bool fx_special(int r) { return radix_cost(true, r) > 0 || r == 16; }  // 16: compile-time plans
-// Fill a plan's stages from its radices.
-void set_stages(FxPlan& p, const std::vector<int>& rad, bool fixed) {
+// Fill a plan's stages from its radices.  quarters: of the general fixed-point
+// kernel, whose stages divide by four after a radix of 8 or more.
+void set_stages(FxPlan& p, const std::vector<int>& rad, bool fixed, bool quarters = false) {
   std::memset(&p, 0, sizeof p);
   p.nst = (int)rad.size();
   int ns = 1, shift = 0;
@@ -381,7 +382,8 @@ void set_stages(FxPlan& p, const std::vector<int>& rad, bool fixed) {
     p.radix[s] = r;
     p.ns[s] = ns;
     p.magic[s] = ns > 1 ? (unsigned)(((1ull << 32) + ns - 1) / ns) : 0;
-    if (fixed) shift += !fx_special(r) ? 2 : ns > 1 ? 1 : 0;  // a direct sum takes quarters
+    // a direct sum takes quarters, of its stage's inputs or the line's
+    if (fixed) shift += !fx_special(r) ? 2 : s == 0 ? 0 : quarters && rad[s - 1] >= 8 ? 2 : 1;
     ns *= r;
     int lg = 0;
     while ((1 << lg) < ns) ++lg;
@@ -446,7 +448,7 @@ FxPlan fx_plan(int n, int rmax, bool near) {
   }
   Splitter sp{true, true, rmax, {}, {}};
   sp.go(n, 1 << 30, 0);
-  set_stages(p, sp.out, true);
+  set_stages(p, sp.out, true, true);
   const int lo = (n + kFxPoints - 1) / kFxPoints;
   p.tpl = best_threads(p, n, true, lo, std::min(kFxMaxThreads, std::max(lo, (n + rmax - 1) / rmax * 5 / 4)));
   return p;

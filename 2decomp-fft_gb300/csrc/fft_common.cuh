@@ -1,6 +1,6 @@
 // Complex helpers, radix butterflies and the per-line addressing shared by
-// the axis-pass kernels (fft_axis.cu: runtime plans; fft_fast.cu:
-// compile-time power-of-two plans).
+// the axis-pass kernels (fft_axis.cu: runtime plans; fft_fast.cuh, fft_gen.cuh,
+// fft_mixed.cuh: compile-time plans; fft_fx*: fixed point).
 #pragma once
 
 #include <type_traits>

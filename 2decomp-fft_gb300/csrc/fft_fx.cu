@@ -34,10 +34,12 @@ using fx::W4;
 
 constexpr int kE = kFxPoints;
 
-// dc: what joins every output of the line, or null
+// down: the powers of two that a stage's twiddles divide by, 1, or 2 after a
+// radix of 8 or more (1 throughout left c2r of 2023 = 17 17 7 points 1.1 times
+// the FP64 kernels' error).  dc: what joins every output of the line, or null.
 template <int R, class Ctx>
 __device__ __forceinline__ void fx_stage(const Ctx& c, const I2* A, I2* B, const W4* __restrict__ tw, int Ns,
-                                         unsigned magic, const I2* dc) {
+                                         unsigned magic, int down, const I2* dc) {
   const int nb = c.N / R;
 #pragma unroll 1
   for (int b = c.t; b < nb; b += c.tpl) {
@@ -48,9 +50,9 @@ __device__ __forceinline__ void fx_stage(const Ctx& c, const I2* A, I2* B, const
     if (Ns > 1) {
       k = b - (int)__umulhi((unsigned)b, magic) * Ns;
       const W4* w = tw + (Ns - 1) + k;
-      v[0] = fx::mk(fx::scale_down(v[0].x), fx::scale_down(v[0].y));
+      v[0] = fx::mk(fx::scale_down(v[0].x, down), fx::scale_down(v[0].y, down));
 #pragma unroll
-      for (int r = 1; r < R; ++r) v[r] = fx::mul_tw(v[r], fx::ldw(w + (r - 1) * Ns), r);
+      for (int r = 1; r < R; ++r) v[r] = fx::mul_tw(v[r], fx::ldw(w + (r - 1) * Ns), r, down);
     }
     if (dc) v[0] = fx::add(v[0], *dc);
     const int base = (b - k) * R + k;
@@ -99,20 +101,21 @@ __device__ __forceinline__ const I2* fx_stages(const Ctx& c, const FxPlan& p, I2
   for (int s = 0; s < p.nst; ++s) {
     const int R = p.radix[s], Ns = p.ns[s];
     const unsigned mg = p.magic[s];
+    const int down = s > 0 ? p.shift[s] - p.shift[s - 1] : 0;
     const I2* const add = s == p.nst - 1 ? dc : nullptr;
     switch (R) {
-      case 2: fx_stage<2>(c, A, B, tw, Ns, mg, add); break;
-      case 3: fx_stage<3>(c, A, B, tw, Ns, mg, add); break;
-      case 4: fx_stage<4>(c, A, B, tw, Ns, mg, add); break;
-      case 5: fx_stage<5>(c, A, B, tw, Ns, mg, add); break;
-      case 6: fx_stage<6>(c, A, B, tw, Ns, mg, add); break;
-      case 7: fx_stage<7>(c, A, B, tw, Ns, mg, add); break;
-      case 8: fx_stage<8>(c, A, B, tw, Ns, mg, add); break;
-      case 9: fx_stage<9>(c, A, B, tw, Ns, mg, add); break;
-      case 10: fx_stage<10>(c, A, B, tw, Ns, mg, add); break;
-      case 11: fx_stage<11>(c, A, B, tw, Ns, mg, add); break;
-      case 13: fx_stage<13>(c, A, B, tw, Ns, mg, add); break;
-      case 17: fx_stage<17>(c, A, B, tw, Ns, mg, add); break;
+      case 2: fx_stage<2>(c, A, B, tw, Ns, mg, down, add); break;
+      case 3: fx_stage<3>(c, A, B, tw, Ns, mg, down, add); break;
+      case 4: fx_stage<4>(c, A, B, tw, Ns, mg, down, add); break;
+      case 5: fx_stage<5>(c, A, B, tw, Ns, mg, down, add); break;
+      case 6: fx_stage<6>(c, A, B, tw, Ns, mg, down, add); break;
+      case 7: fx_stage<7>(c, A, B, tw, Ns, mg, down, add); break;
+      case 8: fx_stage<8>(c, A, B, tw, Ns, mg, down, add); break;
+      case 9: fx_stage<9>(c, A, B, tw, Ns, mg, down, add); break;
+      case 10: fx_stage<10>(c, A, B, tw, Ns, mg, down, add); break;
+      case 11: fx_stage<11>(c, A, B, tw, Ns, mg, down, add); break;
+      case 13: fx_stage<13>(c, A, B, tw, Ns, mg, down, add); break;
+      case 17: fx_stage<17>(c, A, B, tw, Ns, mg, down, add); break;
       default: fx_stage_generic(c, A, B, reinterpret_cast<const W4*>(p.root), R, Ns, add); break;
     }
     __syncthreads();

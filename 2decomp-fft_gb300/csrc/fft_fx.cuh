@@ -189,6 +189,18 @@ template <int SH = 1>
 __device__ __forceinline__ ll scale_down(ll v) {
   return (v + (SH - 1) + ((v >> SH) & 1)) >> SH;
 }
+// The same two for a scale known at run time (1 or 2).
+__device__ __forceinline__ I2 mul_tw(I2 a, W4 w, int r, int sh) {
+  const int xh = hi(a.x), xl = lo(a.x), yh = hi(a.y), yl = lo(a.y);
+  const int xd = xh << (2 - sh), yd = yh << (2 - sh);
+  const int odd = (0x6996 >> (r & 15)) & 1;
+  const ll ur = (kHalf >> (2 - sh)) - odd, ui = (kHalf >> (2 - sh)) - 1 + odd;
+  const int nh = -w.yh, nl = -w.yl;
+  const ll mr = madw(yl, nh, madw(yh, nl, madw(xl, w.xh, madw(xh, w.xl, ur))));
+  const ll mi = madw(yl, w.xh, madw(yh, w.xl, madw(xl, w.yh, madw(xh, w.yl, ui))));
+  return mk(madw(yd, nh, madw(xd, w.xh, mr >> (30 + sh))), madw(yd, w.xh, madw(xd, w.yh, mi >> (30 + sh))));
+}
+__device__ __forceinline__ ll scale_down(ll v, int sh) { return (v + (sh - 1) + ((v >> sh) & 1)) >> sh; }
 
 // ---- butterflies (forward, natural order in and out) -----------------------
 __device__ __forceinline__ void dft4v(I2& a0, I2& a1, I2& a2, I2& a3) {

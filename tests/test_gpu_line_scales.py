@@ -154,3 +154,15 @@ def test_small_fields_scale_exactly(n, real):
             out.append(x * 2.0 ** -k)
         out.append(y * 2.0 ** -k)
     assert all(torch.equal(u, v) for u, v in zip(out[:len(out) // 2], out[len(out) // 2:]))
+
+
+# rel-L2 of the FP64 kernels, c2r of the spectrum of noise
+FP64_NOISE = {7 * 11 * 13: 2.3e-16, 7 * 17 * 17: 2.8e-16}
+
+
+@pytest.mark.parametrize("axis", [0, 1])
+@pytest.mark.parametrize("n", FP64_NOISE)
+def test_large_radices_keep_fp64_accuracy(n, axis):
+    rng = np.random.default_rng(n)
+    got, ref = real_passes(rng.standard_normal((9, n)), axis)[1]
+    assert rel(got, ref) <= FP64_NOISE[n]
