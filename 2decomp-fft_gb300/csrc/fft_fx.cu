@@ -11,15 +11,16 @@
 //      largest high word goes to shared memory;
 //   2. the line's sum of moduli, in units of 2^-20 of that, follows; the two
 //      give the scale at which no stage's output leaves the word;
-//   3. the points become integers in shared buffer 0 (c2r: the Hermitian
-//      combination of the two half spectra);
+//   3. the points become integers in shared buffer 0, a mean taken off (c2r:
+//      the Hermitian combination of the two half spectra but for their bins 0);
 //   4. Stockham stages ping-pong between the two buffers, twiddles from a
 //      stage-major Q62 table;
 //   5. the result goes back to doubles (r2c: the two half spectra apart),
 //      rounded once, to nearest.
 // A CTA that meets a NaN, an infinity or a line outside the exponents of
-// fx::kMinExp..kMaxExp runs its lines in FP64 instead (fx::fallback), with the
-// result those had before.
+// fx::kMinExp..kMaxExp runs its lines in FP64 instead (fx::fallback), on the
+// general kernel's stages: 256^3 r2c + c2r 3.5 ms, in fixed point 0.5 (64^3: 154
+// and 28 us).
 #include "fft_fx.cuh"
 #include "fft_r2r.cuh"
 

@@ -5,19 +5,33 @@
 // and multiplications by constants of modulus one, and no value of a line's
 // transform exceeds the sum of the moduli of its inputs, so a line can be
 // transformed in integers that share one power-of-two scale, chosen from
-// that sum: 64 bits for numbers that hold 53, of which at most a few go to
-// headroom.  The scale is the line's own (never a neighbour's; of two real
-// lines that share a complex one, each its own), so a small line next to a
-// large one keeps all its digits.
+// that sum: 64 bits for numbers that hold 53.  The scale is the line's own
+// (never a neighbour's; of two real lines that share a complex one, each its
+// own), so a small line next to a large one keeps all its digits.
+//
+// Headroom: of 62 bits, those by which the largest of a stage's sums can exceed
+// the line's largest value once the twiddles' divisions are taken off: at most
+// the maximum over the stages of lg(points summed) - (halvings so far), 3 to 7
+// for the compile-time plans of up to 2048 points, 8 at 4096, 9 for the worst
+// supported length (1912 = 8 x 239; direct sums).
+//
+// What this keeps: against the line's norm the error is 0.1 to 0.9 of the FP64
+// kernels', whatever the values (figures at fx_length).  A part of a line far
+// below its largest value has an error of 2^-53 to 2^-59 of that value.  In
+// FP64 it can have less, if the large part cancels exactly there, which takes
+// numbers of few digits.  The two common cases are handled: a mean (PassScale,
+// take_means) and c2r's bin 0.  Other patterns that cancel exactly (+c -c +c
+// -c, say) leave the small rest of such a line the error above, as FP64 does
+// for numbers of full length.
 //
 // Formats: a value is a signed 64-bit integer v, |v| < 2^62.  Table twiddles
-// are Q62 (w 2^62) and multiplying by one divides by 2, in the compile-time
-// plans after a stage of radix 8 or more by 4, which is cheaper (a value grows
-// by sqrt(R) in a stage of radix R on noise and by nothing on a line with one
-// large point; dividing by more than the growth loses bits); constants of the
-// butterflies are Q64 and keep the scale.  Every product is rounded to
-// nearest at 2^-64 of its factors' range; the low 32 x 32 product (below
-// half a unit) is left out.
+// are Q62 (w 2^62) and multiplying by one divides by 2, after a stage of radix
+// 8 or more by 4 (compile-time plans and the general kernel; the radices of
+// fft_rt.cuh are small), which is cheaper (a value grows by sqrt(R) in a stage
+// of radix R on noise and by nothing on a line with one large point; dividing
+// by more than the growth loses bits); constants of the butterflies are Q64
+// and keep the scale.  Every product is rounded to nearest at 2^-64 of its
+// factors' range; the low 32 x 32 product (below half a unit) is left out.
 #pragma once
 
 #include "fft_common.cuh"

@@ -22,8 +22,8 @@ using namespace dev;
 // FP32 on the CUDA cores.  The table twiddles are a high and a low part: on a
 // line with a few large modes the rounding errors of a table add up in the
 // modes' bins.  (Over 70 random boxes the rel-L2 against 64 bits is 0.96 of
-// the general kernel's on average, 0.83 to 1.08 on single ones; with rounded
-// twiddles 0.98.)
+// the general kernel's on average, 0.83 to 1.08 on single ones, where the order
+// of the roundings differs; with rounded twiddles 0.98.)
 struct F32 {
   using T = float;
   using C = float2;

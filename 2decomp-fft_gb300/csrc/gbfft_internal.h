@@ -101,9 +101,13 @@ __host__ __device__ constexpr size_t fxc_smem_bytes(int n, int L) {
 // of 256 threads an SM) but for 1024, 2048 and 4096 points, and the threads a line
 // are those that leave the fewest idle over the stages.  `group` splits the
 // instantiations over translation units.
-// The list holds the powers of two and the smooth lengths that grids are
-// commonly given; the others take the runtime plans (fft_rt.cuh).  r2c / c2r x
-// passes of 24 M points, us, here and on the runtime plan:
+// The list is a choice, not a rule: the powers of two, and of the smooth
+// lengths those of the grids that this library is tested and measured on and
+// round ones like them.  The other 7-smooth lengths (112, 140, 168, 224, 252, 280,
+// 336, 448, 504, 672, 840, 896 and 60 odd more up to 1024) would gain as much as
+// these did over the runtime plans (fft_rt.cuh), 1.1 to 1.3 times, for 5 MB of
+// library each.  r2c / c2r x passes of 24 M points, us, here and on the runtime
+// plan, as measured when the list was made:
 //   72  118 / 117   144 / 158      450  205 / 208   238 / 254
 //   144 146 / 148   188 / 209      540  192 / 196   218 / 236
 //   225 176 / 174   203 / 222      720  189 / 187   225 / 233
@@ -320,8 +324,11 @@ int split_lines_per_cta(int n, bool contiguous);
 cudaError_t launch_split_f32(int kind, bool contiguous, const PassArgs& a, cudaStream_t s);
 // Lengths whose FP64 lines run in fixed point: up to 2048 points, and 4096,
 // whose plan divides by enough on the way.  On longer lines the headroom
-// costs more bits than a double's rounding (rel-L2 0.9 of the FP64 kernels'
-// at 4096 with radix-8 stages; 0.25 to 0.6 at 64 to 2048 points).
+// costs more bits than a double's rounding.  rel-L2 against 64 bits over the
+// FP64 kernels', 126 lengths, lines of noise, of one modulus, of modes and of 1
+// to 256 peaks: c2c and r2c 0.1 to 0.7, c2r 0.15 to 0.92; 4096 points up to 0.9
+// but c2r of a few modes, 1.15 (2.5e-16: the first stage's bound is the sum of
+// the whole line).
 __host__ __device__ constexpr bool fx_length(int n) { return (n >= 2 && n <= 2048) || n == 4096; }
 
 // Shared-memory entries of one power-of-two tile of L lines: the exchange
@@ -348,7 +355,7 @@ __host__ __device__ constexpr size_t rt_entries(int n, int L) { return ((size_t)
 // fallback needs two for a single line), and the lines' scale words
 __host__ __device__ constexpr size_t rt_smem_bytes(int prec_bytes, int n, int L, int nst) {
   return (nst > 2 || (prec_bytes == 8 && L == 1) ? 2 : 1) * rt_entries(n, L) * (size_t)(2 * prec_bytes) + 32 +
-         (size_t)L * kFxWordBytes;
+         (prec_bytes == 8 ? (size_t)L * kFxWordBytes : 0);
 }
 cudaError_t launch_rt_f32(int kind, bool contiguous, const PassArgs& a, cudaStream_t s);
 cudaError_t launch_rt_f64(int kind, bool contiguous, const PassArgs& a, cudaStream_t s);
