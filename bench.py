@@ -605,7 +605,8 @@ def run_gb300(args):
     if dom:
         d = passes[dom]
         traffic = read_traffic(args.workload + ("" if args.form == "plain" else ":" + args.form), dom)
-        roof = {"bound": "hbm", "kernel": "axis pass %s" % dom, "achieved": round(d["gbs"], 1),
+        axis = {"c2c_x": nx, "c2c_y": ny, "c2c_z": nz}.get(dom, nx if fmt == 1 else nz)
+        roof = {"bound": roof_bound(prec, axis), "kernel": "axis pass %s" % dom, "achieved": round(d["gbs"], 1),
                 "peak": peak, "unit": "GB/s", "frac": round(d["gbs"] / peak, 4),
                 "traffic": traffic,
                 "traffic_source": ("committed profile (profiles/dram_traffic.txt: ncu dram bytes of reduced grids "
@@ -930,6 +931,12 @@ def measure_fp64_tflops(dev, n=4096):
     return 2.0 * n ** 3 / best / 1e12
 
 
+def roof_bound(prec, n):
+    """What bounds a pass over n-point lines, beside the HBM fraction that the
+    roofline entry gives: FP64 lines of one tile run in 64-bit fixed point."""
+    return "integer pipe" if prec == 8 and (n <= 2048 or n == 4096) else "hbm"
+
+
 def read_traffic(workload, kernel):
     """DRAM bytes per launch of `kernel` from the committed ncu summary
     (profiles/dram_traffic.txt: `workload kernel bytes_per_launch`)."""
@@ -1053,7 +1060,7 @@ def run_dtt(args):
                 nx, ny, nz, "fp32" if prec == 4 else "fp64"), "name": args.workload, "nx": nx, "ny": ny,
                 "nz": nz, "kinds": list(kinds), "l2": "inputs larger than L2" if npts * (prec) > 130e6
                 else "inputs smaller than L2 (no flush)", "parallelism": "replicas (one grid per GPU)"},
-            "roofline": {"bound": "hbm", "kernel": "all six r2r axis passes of the step",
+            "roofline": {"bound": roof_bound(prec, max(nx, ny, nz)), "kernel": "all six r2r axis passes of the step",
                          "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                          "frac": round(achieved / peak, 4), "traffic": None,
                          "peak_source": "measured (MEASURED_PEAKS.json hbm_gbs)"},
