@@ -210,10 +210,10 @@ __global__ void __launch_bounds__(kMaxThreads) dtt_pass_kernel(const __grid_cons
 // Power-of-two extension length: the extension is transformed by the
 // compile-time 16-point plan (fft_fast.cuh), reading it from and leaving its
 // transform in one padded shared buffer.
-template <typename T, bool CONTIG, int M>
+template <bool CONTIG, int M>
 __global__ void __launch_bounds__(fast_max_threads(16), 1)
     dtt_fast_kernel(const __grid_constant__ DttArgs a) {
-  using C = Cx<T>;
+  using C = float2;
   using P = fast::P2Plan<M, 16>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* Sm = reinterpret_cast<C*>(smem_raw);
@@ -232,11 +232,11 @@ __global__ void __launch_bounds__(fast_max_threads(16), 1)
   }
   const bool valid = u < a.nlines;
   const long long base = CONTIG ? u * a.sl : u + v * a.sl;
-  const T* src = reinterpret_cast<const T*>(a.src);
-  T* dst = reinterpret_cast<T*>(a.dst);
+  const float* src = reinterpret_cast<const float*>(a.src);
+  float* dst = reinterpret_cast<float*>(a.dst);
   const int n = a.n, kind = a.kind;
   const C* w4 = reinterpret_cast<const C*>(a.w4);
-  LineCtx<T, K_C2C, CONTIG> c;
+  LineCtx<float, K_C2C, CONTIG> c;
   c.tw = reinterpret_cast<const C*>(a.twf);
   c.N = M;
   c.L = a.L;
@@ -244,14 +244,14 @@ __global__ void __launch_bounds__(fast_max_threads(16), 1)
   c.tpl = P::TPL;
   c.line = line;
   c.inverse = false;
-  auto X = [&](int j) -> T { return valid ? src[base + (long long)(a.off + j) * a.sn] : T(0); };
+  auto X = [&](int j) -> float { return valid ? src[base + (long long)(a.off + j) * a.sn] : float(0); };
 #pragma unroll 1
   for (int m = t; m < M; m += P::TPL) Sm[c.sidx(m)] = extension<C>(kind, m, n, M, X, w4);
   __syncthreads();
   C x[16];
-  fast::run_plan<P, 0, LineCtx<T, K_C2C, CONTIG>, C, true, true>(c, Sm, x);
+  fast::run_plan<P, 0, LineCtx<float, K_C2C, CONTIG>, C, true, true>(c, Sm, x);
   if (!valid) return;
-  const C c0 = cmk<C>(T(a.c0x), T(a.c0y));
+  const C c0 = cmk<C>(float(a.c0x), float(a.c0y));
 #pragma unroll 1
   for (int k = t; k < n; k += P::TPL)
     dst[base + (long long)(a.off + k) * a.sn] = output<C>(kind, k, n, [&](int i) { return Sm[c.sidx(i)]; }, w4, c0);
@@ -267,9 +267,9 @@ __global__ void __launch_bounds__(fast_max_threads(16), 1)
 // buffer.  R1 threads a line: stage 0 radix R0 (butterfly t, points t + r R1),
 // stage 1 radix R1 (threads t < R0, points t + r R0, twiddles from the
 // stage-major table a.twf), in place.
-template <typename T, bool CONTIG, int M>
+template <bool CONTIG, int M>
 __global__ void __launch_bounds__(256) dtt_mixed_kernel(const __grid_constant__ DttArgs a) {
-  using C = Cx<T>;
+  using C = float2;
   constexpr int R0 = mixed_r0(M), R1 = M / R0;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* Sm = reinterpret_cast<C*>(smem_raw);
@@ -288,18 +288,18 @@ __global__ void __launch_bounds__(256) dtt_mixed_kernel(const __grid_constant__ 
   }
   const bool valid = u < a.nlines;
   const long long base = CONTIG ? u * a.sl : u + v * a.sl;
-  const T* src = reinterpret_cast<const T*>(a.src);
-  T* dst = reinterpret_cast<T*>(a.dst);
+  const float* src = reinterpret_cast<const float*>(a.src);
+  float* dst = reinterpret_cast<float*>(a.dst);
   const int n = a.n, kind = a.kind;
   const C* w4 = reinterpret_cast<const C*>(a.w4);
   const C* tw = reinterpret_cast<const C*>(a.twf);
-  LineCtx<T, K_C2C, CONTIG> c;
+  LineCtx<float, K_C2C, CONTIG> c;
   c.N = M;
   c.L = a.L;
   c.t = t;
   c.tpl = R1;
   c.line = line;
-  auto X = [&](int j) -> T { return valid ? src[base + (long long)(a.off + j) * a.sn] : T(0); };
+  auto X = [&](int j) -> float { return valid ? src[base + (long long)(a.off + j) * a.sn] : float(0); };
 #pragma unroll 1
   for (int m = t; m < M; m += R1) Sm[c.sidx(m)] = extension<C>(kind, m, n, M, X, w4);
   __syncthreads();
@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(256) dtt_mixed_kernel(const __grid_constant__ 
   }
   __syncthreads();
   if (!valid) return;
-  const C c0 = cmk<C>(T(a.c0x), T(a.c0y));
+  const C c0 = cmk<C>(float(a.c0x), float(a.c0y));
 #pragma unroll 1
   for (int k = t; k < n; k += R1)
     dst[base + (long long)(a.off + k) * a.sn] = output<C>(kind, k, n, [&](int i) { return Sm[c.sidx(i)]; }, w4, c0);
@@ -335,12 +335,12 @@ __global__ void __launch_bounds__(256) dtt_mixed_kernel(const __grid_constant__ 
   }
 }
 
-template <typename T, bool CONTIG, int M>
+template <bool CONTIG, int M>
 cudaError_t launch_mixed_m(const DttArgs& a, cudaStream_t stream) {
   constexpr int TPL = M / mixed_r0(M);
   if (a.tpl != TPL || a.L * TPL > 256) return cudaErrorInvalidValue;
-  const size_t smem = (size_t)fast_smem_entries(M, a.L) * sizeof(Cx<T>);
-  auto kern = dtt_mixed_kernel<T, CONTIG, M>;
+  const size_t smem = (size_t)fast_smem_entries(M, a.L) * sizeof(float2);
+  auto kern = dtt_mixed_kernel<CONTIG, M>;
   if (smem > 48 * 1024) {
     cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
@@ -352,21 +352,21 @@ cudaError_t launch_mixed_m(const DttArgs& a, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
-template <typename T, bool CONTIG>
+template <bool CONTIG>
 cudaError_t launch_mixed(const DttArgs& a, cudaStream_t s) {
   switch (a.M) {
-    case 126: return launch_mixed_m<T, CONTIG, 126>(a, s);
-    case 510: return launch_mixed_m<T, CONTIG, 510>(a, s);
+    case 126: return launch_mixed_m<CONTIG, 126>(a, s);
+    case 510: return launch_mixed_m<CONTIG, 510>(a, s);
     default: return cudaErrorNotSupported;
   }
 }
 
-template <typename T, bool CONTIG, int M>
+template <bool CONTIG, int M>
 cudaError_t launch_fast_m(const DttArgs& a, cudaStream_t stream) {
   constexpr int TPL = M / 16;
   if (a.tpl != TPL || a.L * TPL > fast_max_threads(16)) return cudaErrorInvalidValue;
-  const size_t smem = (size_t)fast_smem_entries(M, a.L) * sizeof(Cx<T>);
-  auto kern = dtt_fast_kernel<T, CONTIG, M>;
+  const size_t smem = (size_t)fast_smem_entries(M, a.L) * sizeof(float2);
+  auto kern = dtt_fast_kernel<CONTIG, M>;
   if (smem > 48 * 1024) {
     cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
@@ -378,16 +378,16 @@ cudaError_t launch_fast_m(const DttArgs& a, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
-template <typename T, bool CONTIG>
+template <bool CONTIG>
 cudaError_t launch_fast(const DttArgs& a, cudaStream_t s) {
   switch (a.M) {
-    case 32: return launch_fast_m<T, CONTIG, 32>(a, s);
-    case 64: return launch_fast_m<T, CONTIG, 64>(a, s);
-    case 128: return launch_fast_m<T, CONTIG, 128>(a, s);
-    case 256: return launch_fast_m<T, CONTIG, 256>(a, s);
-    case 512: return launch_fast_m<T, CONTIG, 512>(a, s);
-    case 1024: return launch_fast_m<T, CONTIG, 1024>(a, s);
-    case 2048: return launch_fast_m<T, CONTIG, 2048>(a, s);
+    case 32: return launch_fast_m<CONTIG, 32>(a, s);
+    case 64: return launch_fast_m<CONTIG, 64>(a, s);
+    case 128: return launch_fast_m<CONTIG, 128>(a, s);
+    case 256: return launch_fast_m<CONTIG, 256>(a, s);
+    case 512: return launch_fast_m<CONTIG, 512>(a, s);
+    case 1024: return launch_fast_m<CONTIG, 1024>(a, s);
+    case 2048: return launch_fast_m<CONTIG, 2048>(a, s);
     default: return cudaErrorNotSupported;
   }
 }
@@ -425,9 +425,9 @@ cudaError_t launch_dtt_one(int prec_bytes, bool contiguous, const DttArgs& a, cu
     // compile-time plans: FP32 only (FP64 runs in fixed point or on the runtime plan)
     if (prec_bytes != 4) return cudaErrorInvalidValue;
     if (dtt_mixed_length(a.M))
-      return contiguous ? launch_mixed<float, true>(a, stream) : launch_mixed<float, false>(a, stream);
+      return contiguous ? launch_mixed<true>(a, stream) : launch_mixed<false>(a, stream);
     if (!dtt_fast_length(a.M)) return cudaErrorInvalidValue;
-    return contiguous ? launch_fast<float, true>(a, stream) : launch_fast<float, false>(a, stream);
+    return contiguous ? launch_fast<true>(a, stream) : launch_fast<false>(a, stream);
   }
   if (a.L * a.tpl > kMaxThreads) return cudaErrorInvalidValue;
   if (prec_bytes == 4) return contiguous ? launch_t<float, true>(a, stream) : launch_t<float, false>(a, stream);

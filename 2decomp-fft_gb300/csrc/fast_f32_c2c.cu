@@ -6,7 +6,7 @@ namespace gbfft {
 
 cudaError_t launch_fast_f32_c2c(int kind, bool contiguous, const PassArgs& a, cudaStream_t s) {
   (void)kind;
-  return contiguous ? fast::launch_pow2<float, K_C2C, true>(a, s) : fast::launch_pow2<float, K_C2C, false>(a, s);
+  return contiguous ? fast::launch_pow2<K_C2C, true>(a, s) : fast::launch_pow2<K_C2C, false>(a, s);
 }
 
 }  // namespace gbfft

@@ -186,17 +186,17 @@ struct GenPlan {
 // 1024-thread one (16 lines of 1024 points, 32 of 512: 128- and 256-byte
 // row segments on strided axes) one.  32 points a thread: up to 512
 // threads, at most 128 registers.
-template <typename T, int KIND, bool CONTIG, int N, int E>
+template <int KIND, bool CONTIG, int N, int E>
 __global__ void __launch_bounds__(fast_max_threads(E), 1)
     fast_pass_kernel(const __grid_constant__ PassArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  Cx<T>* Sm = reinterpret_cast<Cx<T>*>(smem_raw);
+  float2* Sm = reinterpret_cast<float2*>(smem_raw);
   chained_entry();
   // launched in clusters: start together, so that neighbouring CTAs' loads
   // of the same rows are in the DRAM queues at the same time
   if (a.csync) cooperative_groups::this_cluster().sync();
   // unpredicated padding-line loads
-  LineCtx<T, KIND, CONTIG, false, false> c;
+  LineCtx<float, KIND, CONTIG, false, false> c;
   c.init(a);
   // the block is (TPL, L) or (L, TPL): the compiler may fold the per-point
   // conditions of the c2r gather and the r2c split that depend on t.
@@ -204,15 +204,15 @@ __global__ void __launch_bounds__(fast_max_threads(E), 1)
   // lines, slower on strided 512-point lines (128 registers instead of 112,
   // z pass 0.76 -> 0.86 ms on 1024 x 1024 x 512) and 256-point ones.
   if constexpr (CONTIG || N == 1024) __builtin_assume(c.t >= 0 && c.t < N / E);
-  Cx<T> v[E];
+  float2 v[E];
   run_stages<N, E, 0>(c, Sm, v);
   if constexpr (KIND == K_R2C) c.template store_r2c_pairs_ct<N, N / E>(Sm);
 }
 
-template <typename T, int KIND, bool CONTIG, int N, int E>
+template <int KIND, bool CONTIG, int N, int E>
 cudaError_t launch_ne(const PassArgs& a, cudaStream_t stream) {
-  const size_t smem = (size_t)fast_smem_entries(N, a.L) * sizeof(Cx<T>);
-  auto kern = fast_pass_kernel<T, KIND, CONTIG, N, E>;
+  const size_t smem = (size_t)fast_smem_entries(N, a.L) * sizeof(float2);
+  auto kern = fast_pass_kernel<KIND, CONTIG, N, E>;
   if (smem > 48 * 1024) {
     cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
@@ -248,33 +248,33 @@ cudaError_t launch_ne(const PassArgs& a, cudaStream_t stream) {
 // Lines of 512 and 1024 points have two plans: 32 points a thread (two
 // stages; the strided default; a contiguous line is then one warp) or 16
 // (three stages; the contiguous default); a.tpl says which.
-template <typename T, int KIND, bool CONTIG, int N>
+template <int KIND, bool CONTIG, int N>
 cudaError_t launch_n(const PassArgs& a, cudaStream_t stream) {
   if constexpr (N == 512 || N == 1024) {
-    if (a.tpl == N / 16) return launch_ne<T, KIND, CONTIG, N, 16>(a, stream);
-    return launch_ne<T, KIND, CONTIG, N, 32>(a, stream);
+    if (a.tpl == N / 16) return launch_ne<KIND, CONTIG, N, 16>(a, stream);
+    return launch_ne<KIND, CONTIG, N, 32>(a, stream);
   } else {
     // short lines: 4 or 8 points a thread when the engine chose them
     if constexpr (N <= 128)
-      if (a.tpl == N / 4) return launch_ne<T, KIND, CONTIG, N, 4>(a, stream);
+      if (a.tpl == N / 4) return launch_ne<KIND, CONTIG, N, 4>(a, stream);
     if constexpr (N <= 256)
-      if (a.tpl == N / 8) return launch_ne<T, KIND, CONTIG, N, 8>(a, stream);
-    return launch_ne<T, KIND, CONTIG, N, fast_points(N, CONTIG)>(a, stream);
+      if (a.tpl == N / 8) return launch_ne<KIND, CONTIG, N, 8>(a, stream);
+    return launch_ne<KIND, CONTIG, N, fast_points(N, CONTIG)>(a, stream);
   }
 }
 
-template <typename T, int KIND, bool CONTIG>
+template <int KIND, bool CONTIG>
 cudaError_t launch_pow2(const PassArgs& a, cudaStream_t stream) {
   switch (a.n) {
-    case 16: return launch_n<T, KIND, CONTIG, 16>(a, stream);
-    case 32: return launch_n<T, KIND, CONTIG, 32>(a, stream);
-    case 64: return launch_n<T, KIND, CONTIG, 64>(a, stream);
-    case 128: return launch_n<T, KIND, CONTIG, 128>(a, stream);
-    case 256: return launch_n<T, KIND, CONTIG, 256>(a, stream);
-    case 512: return launch_n<T, KIND, CONTIG, 512>(a, stream);
-    case 1024: return launch_n<T, KIND, CONTIG, 1024>(a, stream);
-    case 2048: return launch_n<T, KIND, CONTIG, 2048>(a, stream);
-    case 4096: return launch_n<T, KIND, CONTIG, 4096>(a, stream);
+    case 16: return launch_n<KIND, CONTIG, 16>(a, stream);
+    case 32: return launch_n<KIND, CONTIG, 32>(a, stream);
+    case 64: return launch_n<KIND, CONTIG, 64>(a, stream);
+    case 128: return launch_n<KIND, CONTIG, 128>(a, stream);
+    case 256: return launch_n<KIND, CONTIG, 256>(a, stream);
+    case 512: return launch_n<KIND, CONTIG, 512>(a, stream);
+    case 1024: return launch_n<KIND, CONTIG, 1024>(a, stream);
+    case 2048: return launch_n<KIND, CONTIG, 2048>(a, stream);
+    case 4096: return launch_n<KIND, CONTIG, 4096>(a, stream);
     default: return cudaErrorNotSupported;
   }
 }

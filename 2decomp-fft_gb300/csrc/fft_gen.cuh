@@ -23,27 +23,27 @@ template <> struct PlanOf<360> { using type = fast::GenPlan<360, 30, 10, 6, 6>; 
 template <> struct PlanOf<384> { using type = fast::GenPlan<384, 24, 8, 8, 6>; };
 template <> struct PlanOf<400> { using type = fast::GenPlan<400, 20, 20, 20>; };
 
-template <typename T, int KIND, bool CONTIG, int N>
+template <int KIND, bool CONTIG, int N>
 __global__ void __launch_bounds__(gen_max_threads(PlanOf<N>::type::E), 1)
     gen_pass_kernel(const __grid_constant__ PassArgs a) {
   using P = typename PlanOf<N>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  Cx<T>* Sm = reinterpret_cast<Cx<T>*>(smem_raw);
+  float2* Sm = reinterpret_cast<float2*>(smem_raw);
   chained_entry();
-  LineCtx<T, KIND, CONTIG> c;
+  LineCtx<float, KIND, CONTIG> c;
   c.init(a);
-  Cx<T> v[P::E];
+  float2 v[P::E];
   fast::run_plan<P, 0>(c, Sm, v);
   if constexpr (KIND == K_R2C) c.store_r2c_pairs(Sm);
 }
 
-template <typename T, int KIND, bool CONTIG, int N>
+template <int KIND, bool CONTIG, int N>
 cudaError_t launch_n(const PassArgs& a, cudaStream_t stream) {
   using P = typename PlanOf<N>::type;
   if (a.tpl != P::TPL || a.L < 1 || a.L * P::TPL > gen_max_threads(P::E))
     return cudaErrorInvalidValue;
-  const size_t smem = (size_t)fast_smem_entries(N, a.L) * sizeof(Cx<T>);
-  auto kern = gen_pass_kernel<T, KIND, CONTIG, N>;
+  const size_t smem = (size_t)fast_smem_entries(N, a.L) * sizeof(float2);
+  auto kern = gen_pass_kernel<KIND, CONTIG, N>;
   if (smem > 48 * 1024) {
     cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
@@ -55,23 +55,22 @@ cudaError_t launch_n(const PassArgs& a, cudaStream_t stream) {
   return err != cudaSuccess ? err : cudaGetLastError();
 }
 
-template <typename T, int KIND, bool CONTIG>
+template <int KIND, bool CONTIG>
 cudaError_t launch_k(const PassArgs& a, cudaStream_t s) {
   switch (a.n) {
-    case 243: return launch_n<T, KIND, CONTIG, 243>(a, s);
-    case 270: return launch_n<T, KIND, CONTIG, 270>(a, s);
-    case 360: return launch_n<T, KIND, CONTIG, 360>(a, s);
-    case 384: return launch_n<T, KIND, CONTIG, 384>(a, s);
-    case 400: return launch_n<T, KIND, CONTIG, 400>(a, s);
+    case 243: return launch_n<KIND, CONTIG, 243>(a, s);
+    case 270: return launch_n<KIND, CONTIG, 270>(a, s);
+    case 360: return launch_n<KIND, CONTIG, 360>(a, s);
+    case 384: return launch_n<KIND, CONTIG, 384>(a, s);
+    case 400: return launch_n<KIND, CONTIG, 400>(a, s);
     default: return cudaErrorNotSupported;
   }
 }
 
-template <typename T>
-cudaError_t launch(int kind, bool contiguous, const PassArgs& a, cudaStream_t s) {
-  if (kind == K_C2C) return contiguous ? launch_k<T, K_C2C, true>(a, s) : launch_k<T, K_C2C, false>(a, s);
-  if (kind == K_R2C) return contiguous ? launch_k<T, K_R2C, true>(a, s) : launch_k<T, K_R2C, false>(a, s);
-  return contiguous ? launch_k<T, K_C2R, true>(a, s) : launch_k<T, K_C2R, false>(a, s);
+inline cudaError_t launch(int kind, bool contiguous, const PassArgs& a, cudaStream_t s) {
+  if (kind == K_C2C) return contiguous ? launch_k<K_C2C, true>(a, s) : launch_k<K_C2C, false>(a, s);
+  if (kind == K_R2C) return contiguous ? launch_k<K_R2C, true>(a, s) : launch_k<K_R2C, false>(a, s);
+  return contiguous ? launch_k<K_C2R, true>(a, s) : launch_k<K_C2R, false>(a, s);
 }
 
 }  // namespace gen

@@ -3,6 +3,6 @@
 
 namespace gbfft {
 cudaError_t launch_gen_f32(int kind, bool contiguous, const PassArgs& a, cudaStream_t s) {
-  return gen::launch<float>(kind, contiguous, a, s);
+  return gen::launch(kind, contiguous, a, s);
 }
 }  // namespace gbfft
